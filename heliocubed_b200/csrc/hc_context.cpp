@@ -542,25 +542,28 @@ void roeFrame(const double* A, int dir, double* out) {
   const double normalMag = std::sqrt(normal2), tangentMag = std::sqrt(tangent2);
   const double invN = 1.0 / normalMag, invT = 1.0 / tangentMag;
   for (int i = 0; i < 3; ++i) { f0[i] *= invN; f1[i] *= invT; }
+  double F[3][3], adj[3][3];
   for (int i = 0; i < 3; ++i) {
     const int j = (i + 1) % 3, k = (i + 2) % 3;
-    out[i] = f0[i];
-    out[3 + i] = f1[i];
-    out[6 + i] = f0[j] * f1[k] - f0[k] * f1[j];
+    F[0][i] = f0[i];
+    F[1][i] = f1[i];
+    F[2][i] = f0[j] * f1[k] - f0[k] * f1[j];
   }
-  out[9] = normalMag;
-  double adj[3][3];
   for (int dd = 0; dd < 3; ++dd) {
     const int s1 = (dd + 1) % 3, s2 = (dd + 2) % 3;
     for (int i = 0; i < 3; ++i) {
       const int j = (i + 1) % 3, k = (i + 2) % 3;
       adj[dd][i] = A[3 * j + s1] * A[3 * k + s2] - A[3 * k + s1] * A[3 * j + s2];
-      out[10 + 3 * dd + i] = adj[dd][i];
     }
   }
-  const double det = A[0] * adj[0][0] + A[3] * adj[0][1] + A[6] * adj[0][2];
-  out[19] = 1.0 / det;
-  out[20] = 1.0 / (det * det);
+  const double det = A[0] * adj[0][0] + A[3] * adj[0][1] + A[6] * adj[0][2], invDet = 1.0 / det;
+  const double back = normalMag * (1.0 / (det * det));
+  for (int r = 0; r < 3; ++r)
+    for (int s = 0; s < 3; ++s) {
+      out[3 * r + s] = F[r][0] * A[s] + F[r][1] * A[3 + s] + F[r][2] * A[6 + s];
+      out[9 + 3 * r + s] = back * (adj[r][0] * F[s][0] + adj[r][1] * F[s][1] + adj[r][2] * F[s][2]);
+    }
+  out[18] = normalMag * invDet;
 }
 
 // Fourth-order metric tables over angular indices [-ext, na+ext] (ghost

@@ -185,11 +185,12 @@ constexpr int kO4Rad = 10;   // radial margin of the O4 radial table
 // Face metrics of direction d at angular (j,k): <det A A> (9), <det A> (1),
 // <adjA row d> (3), pointwise basis at the face centre (9; d = 0: cell centre).
 constexpr int kO4FaceRec = 22;
-// Frame of the factored Roe dissipation at a face of direction d (angular
-// (j,k)), from the face-centre basis A (d = 0: cell centre): unit normal f0,
-// unit tangent f1, f2 = f0 x f1 (9), |cofactor row d of A| (1), adj A (9),
-// 1 / det A, 1 / det A^2 (2); padded to 24 (16-byte aligned pairs).
-constexpr int kO4RoeRec = 24;
+// Products of the factored Roe dissipation at a face of direction d (angular
+// (j,k)), from the face-centre basis A (d = 0: cell centre) and the frame F
+// with rows f0 (unit normal), f1 (unit tangent), f2 = f0 x f1: F A (9),
+// |n| adj A F^T / det A^2 (9), |n| / det A (1), |n| the length of cofactor
+// row d of A; padded to 20 (16-byte aligned pairs).
+constexpr int kO4RoeRec = 20;
 
 struct O4Geo {
   int nr, na, ext;        // tables cover angular indices [-ext, na+ext]

@@ -323,71 +323,61 @@ __device__ __forceinline__ bool usablePrimitive(const double w[8]) {
 }
 
 // mappedRoe8WaveDissipation + factoredRoe8WaveDissipation (src/MHD_Roe8Wave.H:634-740)
-// with the face's frame from the Roe frame table R (kO4RoeRec): the states
-// are rotated into the frame, the 8-wave dissipation (Rusanov where the fan
-// check fails) is taken there, rotated back, scaled by the face area and
-// mapped through adj A / det A.  The frame is read again after the solver
-// (roeLoad2 is not merged with the first read), so it does not occupy
-// registers while the solver runs.
+// with the face's products from the Roe frame table R (kO4RoeRec): one 3 x 3
+// matrix takes native vectors into the face frame (F A), the 8-wave
+// dissipation (Rusanov where the fan check fails) is taken there, and one
+// matrix takes it back (|n| adj A F^T / det A^2); the angular products are
+// in the table, so a vector costs nine operations each way.  The second
+// matrix is read after the solver (roeLoad2 is not merged with the first
+// read), so it does not occupy registers while the solver runs.
 __device__ __forceinline__ double2 roeLoad2(const double* p) {
   double2 v;
   asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
   return v;
 }
 
-__device__ __forceinline__ void factoredRoe(double out[8], const double* wl, const double* wr, const double* A,
+__device__ __forceinline__ void factoredRoe(double out[8], const double* wl, const double* wr,
                                             const double* __restrict__ R, double radialArea, double gamma,
                                             double invGm1, double entropy) {
   double loc[2][8];
   {
-    double f[9];
+    double f[10];
 #pragma unroll
-    for (int q = 0; q < 9; ++q) f[q] = R[q];
+    for (int q = 0; q < 5; ++q) {
+      const double2 v = roeLoad2(R + 2 * q);
+      f[2 * q] = v.x;
+      f[2 * q + 1] = v.y;
+    }
 #pragma unroll
     for (int side = 0; side < 2; ++side) {
       const double* w = side == 0 ? wl : wr;
       loc[side][0] = fmax(w[0], kRHO00);
       loc[side][4] = fmax(w[4], 0.0);
-      double vC[3], bC[3];
-#pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        vC[i] = A[3 * i] * w[1] + A[3 * i + 1] * w[2] + A[3 * i + 2] * w[3];
-        bC[i] = A[3 * i] * w[5] + A[3 * i + 1] * w[6] + A[3 * i + 2] * w[7];
-      }
 #pragma unroll
       for (int r = 0; r < 3; ++r) {
-        loc[side][1 + r] = f[3 * r] * vC[0] + f[3 * r + 1] * vC[1] + f[3 * r + 2] * vC[2];
-        loc[side][5 + r] = f[3 * r] * bC[0] + f[3 * r + 1] * bC[1] + f[3 * r + 2] * bC[2];
+        loc[side][1 + r] = dot3(f[3 * r], w[1], f[3 * r + 1], w[2], f[3 * r + 2], w[3]);
+        loc[side][5 + r] = dot3(f[3 * r], w[5], f[3 * r + 1], w[6], f[3 * r + 2], w[7]);
       }
     }
   }
   double diss[8];
   if (!roe8Body<true>(diss, loc[0], loc[1], gamma, entropy, invGm1))
     rusanovDissipation(diss, loc[0], loc[1], gamma, invGm1);
-  double g[22];
+  double g[12];
 #pragma unroll
-  for (int q = 0; q < 11; ++q) {
-    const double2 v = roeLoad2(R + 2 * q);
+  for (int q = 0; q < 6; ++q) {
+    const double2 v = roeLoad2(R + 8 + 2 * q);
     g[2 * q] = v.x;
     g[2 * q + 1] = v.y;
   }
-  const double area = radialArea * g[9];
-  double mapped[8];
-  mapped[0] = area * diss[0];
-  mapped[4] = area * diss[4];
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    mapped[1 + i] = area * g[i] * diss[1] + area * g[3 + i] * diss[2] + area * g[6 + i] * diss[3];
-    mapped[5 + i] = area * g[i] * diss[5] + area * g[3 + i] * diss[6] + area * g[6 + i] * diss[7];
-  }
-  const double* adj = g + 10;
-  const double invDet = g[19], invDet2 = g[20];
-  out[0] = mapped[0] * invDet;
-  out[4] = mapped[4] * invDet;
+  // g[1 .. 9] the matrix back, g[10] = |n| / det A
+  const Rn area = radialArea;
+  out[0] = area * (Rn(g[10]) * diss[0]);
+  out[4] = area * (Rn(g[10]) * diss[4]);
 #pragma unroll
   for (int dd = 0; dd < 3; ++dd) {
-    out[1 + dd] = (adj[3 * dd] * mapped[1] + adj[3 * dd + 1] * mapped[2] + adj[3 * dd + 2] * mapped[3]) * invDet2;
-    out[5 + dd] = (adj[3 * dd] * mapped[5] + adj[3 * dd + 1] * mapped[6] + adj[3 * dd + 2] * mapped[7]) * invDet2;
+    out[1 + dd] = area * dot3(g[1 + 3 * dd], diss[1], g[2 + 3 * dd], diss[2], g[3 + 3 * dd], diss[3]);
+    out[5 + dd] = area * dot3(g[1 + 3 * dd], diss[5], g[2 + 3 * dd], diss[6], g[3 + 3 * dd], diss[7]);
   }
 }
 
@@ -670,8 +660,8 @@ __global__ void __launch_bounds__(128, MB) o4RoePointKernel(const Ctx* __restric
     double l[8], r[8], o[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) { l[q] = base[(F_WL + q) * NF]; r[q] = base[(F_WR + q) * NF]; }
-    factoredRoe(o, l, r, faceBasis<D>(c, b, j, k), roeRec(a.G, a.block0 + b, D, j, k), radialPoint(a.G, d, i),
-                a.G.gamma, a.G.invGm1, a.G.entropy);
+    factoredRoe(o, l, r, roeRec(a.G, a.block0 + b, D, j, k), radialPoint(a.G, d, i), a.G.gamma, a.G.invGm1,
+                a.G.entropy);
 #pragma unroll
     for (int q = 0; q < 8; ++q) base[(F_QD + q) * NF] = o[q];
   });
