@@ -69,12 +69,10 @@ OPERATOR_BYTES_PER_CELL_STAGE = 128  # read 8 FP64 primitives, write 8 FP64 rhs
 
 def operator_launches(args) -> int:
     """Kernels of one fourth-order operator evaluation (hc_level_rhs)."""
-    roe, powell = int(args.riemann == 2), 1
-    # detector + point values (3); per direction reconstruction, Roe point
-    # dissipation, fused face chain and the Powell face chain (3); the radial
-    # face averages of the TMA-staged radial chain (1); Powell coefficients,
-    # averages and application (3)
-    return 3 + 3 * (2 + roe + 3 * powell) + 1 + 3 * powell
+    # detector + point values (3); reconstruction, Riemann problem, face
+    # averages and final flux of all directions (4); Powell averages, face
+    # fluxes and divergence (3); the cell pass (1)
+    return 3 + 4 + 3 + 1
 
 
 def launches_per_step(args) -> int:

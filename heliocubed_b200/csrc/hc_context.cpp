@@ -560,8 +560,9 @@ void roeFrame(const double* A, int dir, double* out) {
   const double back = normalMag * (1.0 / (det * det));
   for (int r = 0; r < 3; ++r)
     for (int s = 0; s < 3; ++s) {
-      out[3 * r + s] = F[r][0] * A[s] + F[r][1] * A[3 + s] + F[r][2] * A[6 + s];
-      out[9 + 3 * r + s] = back * (adj[r][0] * F[s][0] + adj[r][1] * F[s][1] + adj[r][2] * F[s][2]);
+      const int ns = (dir + s) % 3, nr = (dir + r) % 3;  // native direction at place s, r
+      out[3 * r + s] = F[r][0] * A[ns] + F[r][1] * A[3 + ns] + F[r][2] * A[6 + ns];
+      out[9 + 3 * r + s] = back * (adj[nr][0] * F[s][0] + adj[nr][1] * F[s][1] + adj[nr][2] * F[s][2]);
     }
   out[18] = normalMag * invDet;
 }
@@ -575,7 +576,8 @@ int buildO4Geometry(hc_ctx* c) {
   const int n = na + 2 * ext + 1;
   const double h = 1.0 / na;
   Gauss G;
-  std::vector<double> face((size_t)6 * 3 * n * n * kO4FaceRec), cell((size_t)6 * n * n * 9);
+  constexpr int kRec = 22;  // <det A A> (9), <det A>, normal (3), point basis (9)
+  std::vector<double> face((size_t)6 * 3 * n * n * kRec), cell((size_t)6 * n * n * 9);
   for (int b = 0; b < 6; ++b)
     for (int k = -ext; k <= na + ext; ++k)
       for (int j = -ext; j <= na + ext; ++j) {
@@ -585,7 +587,7 @@ int buildO4Geometry(hc_ctx* c) {
         for (int r = 0; r < 3; ++r)
           for (int q = 0; q < 3; ++q) cb[3 * r + q] = A[r][q];
         for (int d = 0; d < 3; ++d) {
-          double* e = &face[((((size_t)b * 3 + d) * n + (k + ext)) * n + (j + ext)) * kO4FaceRec];
+          double* e = &face[((((size_t)b * 3 + d) * n + (k + ext)) * n + (j + ext)) * kRec];
           double dA[3][3] = {{0}}, det = 0, nn[3] = {0, 0, 0};
           if (d == 0) {
             for (int p = 0; p < 8; ++p)
@@ -636,8 +638,31 @@ int buildO4Geometry(hc_ctx* c) {
       for (int k = 0; k < n; ++k)
         for (int j = 0; j < n; ++j) {
           const size_t at = (((size_t)b * 3 + d) * n + k) * n + j;
-          const double* A = d == 0 ? &cell[((size_t)b * n + k) * n * 9 + (size_t)j * 9] : &face[at * kO4FaceRec + 13];
+          const double* A = d == 0 ? &cell[((size_t)b * n + k) * n * 9 + (size_t)j * 9] : &face[at * kRec + 13];
           roeFrame(A, d, &roe[at * kO4RoeRec]);
+        }
+  // The device records: halves and angular differences / 48 (the table's
+  // outermost positions, which no kernel reads, get none).
+  std::vector<double> face0((size_t)6 * n * n * kO4FaceRec0, 0.0), face12((size_t)6 * 2 * n * n * kO4FaceRec12, 0.0);
+  for (int b = 0; b < 6; ++b)
+    for (int d = 0; d < 3; ++d)
+      for (int k = 0; k < n; ++k)
+        for (int j = 0; j < n; ++j) {
+          const double* e = &face[((((size_t)b * 3 + d) * n + k) * n + j) * kRec];
+          double* out = d == 0 ? &face0[(((size_t)b * n + k) * n + j) * kO4FaceRec0]
+                               : &face12[((((size_t)b * 2 + d - 1) * n + k) * n + j) * kO4FaceRec12];
+          auto at = [d](const double* rec, int q) {  // entry q of the device record's thirteen
+            return 0.5 * (q < 9 ? rec[3 * (q / 3) + (d + q % 3) % 3] : rec[q]);
+          };
+          for (int q = 0; q < 13; ++q) out[q] = at(e, q);
+          for (int t = 1, slot = 13; t <= 2; ++t) {
+            if (t == d) continue;
+            const long step = (t == 1 ? 1L : (long)n) * kRec;
+            const int x = t == 1 ? j : k;
+            if (x > 0 && x < n - 1)
+              for (int q = 0; q < 13; ++q) out[slot + q] = (at(e + step, q) - at(e - step, q)) / 48.0;
+            slot += 13;
+          }
         }
   std::vector<double4> radial(nr + 2 * kO4Rad + 1);
   for (int i = -kO4Rad; i <= nr + kO4Rad; ++i) {
@@ -647,7 +672,8 @@ int buildO4Geometry(hc_ctx* c) {
   cudaError_t err = cudaSuccess;
   O4Geo& g = c->o4;
   g.nr = nr; g.na = na; g.ext = ext;
-  g.face = upload(face, c->owned, err);
+  g.face0 = upload(face0, c->owned, err);
+  g.face12 = upload(face12, c->owned, err);
   g.cell = upload(cell, c->owned, err);
   g.frames = upload(roe, c->owned, err);
   g.radial = upload(radial, c->owned, err);
@@ -656,13 +682,12 @@ int buildO4Geometry(hc_ctx* c) {
   g.roe = P.riemann_solver == 2; g.powell = P.divergence_cleaning == 1; g.fallback = P.berta_fallback_type;
   // the CME insertion window's Rusanov flag (0 until a schedule sets it)
   {
-    cudaError_t ferr = cudaMalloc(&c->rusanovFlag, 2 * sizeof(int));
-    if (ferr == cudaSuccess) ferr = cudaMemset(c->rusanovFlag, 0, 2 * sizeof(int));
+    cudaError_t ferr = cudaMalloc(&c->rusanovFlag, sizeof(int));
+    if (ferr == cudaSuccess) ferr = cudaMemset(c->rusanovFlag, 0, sizeof(int));
     if (ferr != cudaSuccess) return cudaFail(ferr, "O4 flag");
     c->owned.push_back(c->rusanovFlag);
   }
   g.rusanov = c->rusanovFlag;
-  g.status = c->rusanovFlag + 1;
   if (err != cudaSuccess) return cudaFail(err, "O4 geometry upload");
   return HC_OK;
 }
@@ -967,7 +992,7 @@ O4Batch* cachedBatch(hc_ctx* c, const O4Args& a, int* rc) {
   put(a.vlo, sizeof a.vlo); put(a.vhi, sizeof a.vhi); put(&a.U, sizeof a.U); put(a.ur.lo, sizeof a.ur.lo);
   put(a.ur.n, sizeof a.ur.n); put(&a.uStride, sizeof a.uStride); put(&a.scale, sizeof a.scale);
   put(&a.rhs, sizeof a.rhs); put(&a.rhsStride, sizeof a.rhsStride); put(a.flux, sizeof a.flux);
-  put(&a.WA, sizeof a.WA); put(&a.face, sizeof a.face); put(&a.face2, sizeof a.face2); put(&a.kp, sizeof a.kp);
+  put(&a.WA, sizeof a.WA); put(a.face, sizeof a.face); put(&a.ka, sizeof a.ka);
   put(&a.rr, sizeof a.rr);
   for (auto& e : c->o4cache)
     if (e.first == key) return e.second;
@@ -1538,7 +1563,7 @@ std::string o4Key(const hc_ctx* c) {
 // Fourth order: the state's stage preparation into the level workspace, then
 // the level operator timed for each register-cap variant of one tuned kernel
 // at a time, the others held at the best found so far (coordinate descent
-// over reconstruction, Roe point dissipation, final flux).
+// over the reconstruction, Riemann problem and final flux).
 int autotuneO4(hc_ctx* c, const double* ju, cudaStream_t s, int* tilesOut, double* msOut) {
   int rc = ensureO4Buffers(c);
   if (rc != HC_OK) return rc;
@@ -1546,10 +1571,6 @@ int autotuneO4(hc_ctx* c, const double* ju, cudaStream_t s, int* tilesOut, doubl
   rc = checkLaunch(launchO4Prepare(io, s), "autotune O4 prepare");
   int best[kO4TunedKernels] = {0, 0, 0};
   for (int q = 0; q < kO4TunedKernels && rc == HC_OK; ++q) {
-    if (q == 1 && c->P.riemann_solver != 2) {  // no Roe point kernel with Rusanov
-      for (int v = 0; v < kO4Variants && msOut; ++v) msOut[q * kO4Variants + v] = 0.0;
-      continue;
-    }
     double bestMs = 1e300;
     for (int v = 0; v < kO4Variants && rc == HC_OK; ++v) {
       int var[kO4TunedKernels] = {best[0], best[1], best[2]};

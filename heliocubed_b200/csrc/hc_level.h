@@ -182,27 +182,31 @@ constexpr int kO4Ghost = 5;  // NGHOST: Jameson detector + WENOZ + transverse pr
 constexpr int kO4Ang = 8;    // angular margin of the O4 metric tables
 constexpr int kO4Rad = 10;   // radial margin of the O4 radial table
 
-// Face metrics of direction d at angular (j,k): <det A A> (9), <det A> (1),
-// <adjA row d> (3), pointwise basis at the face centre (9; d = 0: cell centre).
-constexpr int kO4FaceRec = 22;
+// Face metrics of direction d at angular (j,k): half of <det A A> (9,
+// row-major, columns in (normal, next, next but one) direction order), of
+// <det A> (1) and of the normal <adjA row d> (3); then their differences
+// (upper - lower neighbour) / 48 along the angular transverse directions: j,
+// then k for d = 0 (padded to 40), the one angular transverse direction for
+// d = 1, 2 (26).
+constexpr int kO4FaceRec0 = 40, kO4FaceRec12 = 26;
 // Products of the factored Roe dissipation at a face of direction d (angular
 // (j,k)), from the face-centre basis A (d = 0: cell centre) and the frame F
 // with rows f0 (unit normal), f1 (unit tangent), f2 = f0 x f1: F A (9),
 // |n| adj A F^T / det A^2 (9), |n| / det A (1), |n| the length of cofactor
-// row d of A; padded to 20 (16-byte aligned pairs).
+// row d of A; native indices in (normal, next, next but one) direction order;
+// padded to 20 (16-byte aligned pairs).
 constexpr int kO4RoeRec = 20;
 
 struct O4Geo {
   int nr, na, ext;        // tables cover angular indices [-ext, na+ext]
-  const double* face;     // [6][3][na+2ext+1 (k)][na+2ext+1 (j)][22]
+  const double* face0;    // [6][na+2ext+1 (k)][na+2ext+1 (j)][kO4FaceRec0], direction 0
+  const double* face12;   // [6][2][na+2ext+1 (k)][na+2ext+1 (j)][kO4FaceRec12], directions 1, 2
   const double* cell;     // [6][na+2ext+1][na+2ext+1][9] cell-centre basis
   const double* frames;   // [6][3][na+2ext+1 (k)][na+2ext+1 (j)][kO4RoeRec] Roe frames
   const double4* radial;  // [nr+2*kO4Rad+1], index i+kO4Rad: {rlow^2, areaT, Dr0, dVolr}
   double gamma, invGm1, entropy, eta_d, dx[3];
   int roe, powell, fallback;
   const int* rusanov;     // device flag (may be null): nonzero runs a Roe context with Rusanov dissipation
-  int* status;            // device word (may be null): set to 1 when a kernel's bounded wait for a
-                          // shared-memory tile gave up (that tile's rhs is then NaN)
 };
 
 // A box region: low corner, extents, cell count.
@@ -231,10 +235,9 @@ struct O4Args {
   double* WP;   // [nbox][8][G]
   double* th;   // [nbox][G]
   double* thr;  // [nbox][G] raw detector flag
-  double* face; // [nbox][kO4FaceArrays][F]: face arrays of directions 0 and 2
-  double* face2; // [nbox][kO4FaceArrays][F]: face arrays of direction 1 (its pass overlaps its neighbours')
-  double* mj;   // [nbox][V+1]
-  double* kp;   // [nbox][8][V+2]
+  double* face[3];  // [nbox][kO4FaceArrays][F]: face arrays of each direction
+  double* mj;       // [nbox][V+1]
+  double* ka;       // [nbox][7][V+1]
   // The seam-flux register of the box's own level when the box runs in one
   // launch with other levels' boxes (an ensemble): null takes the launch's
   // RegArgs; else the face flux times (stage weight) * seamCfl / *seamInvMax
@@ -247,7 +250,11 @@ struct O4Args {
   // valid box itself.
   Reg rr;
 };
-constexpr int kO4FaceArrays = 8 * 4 + 5 + 9;  // WL, WR, FS, QD/DP (8 each) + thF, PS, BP, Bflux, Bprod + averages (8 + 1)
+// Flux sums (7, the normal field's vanishes) and pressure sum, whose place the
+// final fluxes (8) take; point dissipation (8); left and right states (16),
+// the left ones' place taken by the area products of the averages (7 + 1);
+// flag, centred normal field, speed bound, Powell flux.
+constexpr int kO4FaceArrays = 36;
 
 size_t o4ScratchDoubles(int nbox, const int vlo[3], const int vhi[3], int ghost);
 // Carve the operator scratch of a.nbox boxes with the valid box a.vlo..vhi
@@ -267,11 +274,11 @@ struct RegArgs {
 
 // A batch of boxes of any sizes for the operator kernels: per box and
 // direction a kernel context in device memory; every kernel of the operator
-// is one launch over the whole batch (one CTA row per box).  Each entry of
+// is one launch over the whole batch.  Each entry of
 // `boxes` describes one box (nbox 1) with its own input, output and scratch.
 struct O4Batch;
-// Register-cap variants of the operator's three heaviest kernels
-// (reconstruction, Roe point dissipation, final flux), chosen by the
+// Register-cap variants of the operator's three face kernels
+// (reconstruction, Riemann problem, final flux), chosen by the
 // autotuner; results do not depend on them.
 constexpr int kO4TunedKernels = 3, kO4Variants = 3;
 void o4BatchSetVariants(O4Batch* b, const int v[kO4TunedKernels]);

@@ -3,20 +3,19 @@
 // src/BoxOp_RoeCubedSphere.H:29-145 and the Powell terms of
 // src/BoxOp_DivBcleaning.H:35-172.  FP64.
 //
-// Kernels per evaluation: the detector and point values on the ghosted box
-// G (cell arrays); per direction d the reconstruction on the face box
-// F = G.extrude(d).grow(-3) and the Roe point dissipation (face arrays in
-// the face scratch), then one fused face-chain kernel that takes tiles of
-// the final faces through the flux average, mapped flux, radial products,
-// final flux and divergence with its intermediates in shared memory; the
-// Powell terms on a side stream.  Every intermediate covers the box the
-// reference computes it on.
-#include <cuda.h>
+// Kernels per evaluation, each one launch over every box and (for the face
+// kernels) all three directions of a batch:
+//   o4PrimAvgKernel, o4ThetaRawKernel, o4PointKernel: detector and point values
+//   o4FaceReconKernel: both states of every face
+//   o4FaceRiemannKernel: point flux sums and dissipation
+//   o4FaceAvgKernel: face averages and their radial-area products
+//   o4FaceFinalKernel: mapped final flux of every face
+//   o4CellKernel: flux divergence and Powell source into rhs
+// and on a side stream o4PowellAvgKernel, o4PowellFluxKernel, o4PowellDivKernel.
+// Every intermediate covers the box the reference computes it on.
 #include <cuda_runtime.h>
-#include <math_constants.h>
 
 #include <algorithm>
-#include <cstdint>
 #include <vector>
 
 #include "hc_device.cuh"
@@ -53,59 +52,67 @@ __device__ __forceinline__ long roff(const Reg& r, int i, int j, int k) {
   return (long)((i - r.lo[0]) + r.n[0] * ((j - r.lo[1]) + r.n[1] * (k - r.lo[2])));
 }
 
-// Offsets of the face arrays inside a box's face scratch (units of F.N).
-enum FaceArr { F_WL = 0, F_WR = 8, F_FS = 16, F_QD = 24, F_THF = 32, F_PS = 33, F_BP = 34, F_BFLUX = 35,
-               F_BPROD = 36, F_FA0 = 37, F_PA0 = 45 };  // F_FA0, F_PA0: direction 0's averages (TMA path)
+// Offsets of the face arrays inside a direction's face scratch (units of
+// F.N).  Vector components of the flux sums, dissipations and averages are
+// kept along (normal, next, next but one) native direction; the flux sum of
+// the normal field vanishes and has no array.  The final fluxes (Cartesian
+// components) take the place of the flux sums and pressures, and the area
+// products that of the left states, which nothing reads any more by then.
+enum FaceArr { F_FS = 0, F_PS = 7, F_FX = 0, F_QD = 8, F_L = 16, F_R = 24, F_X = 16, F_T3 = 23, F_THF = 32, F_BP = 33,
+               F_SPD = 34, F_BF = 35 };
+static_assert(F_BF + 1 == kO4FaceArrays, "face arrays");
+// F_FS array of component c in (rho, m_n, m_1, m_2, E, B_n, B_1, B_2) order (c != 5), also of F_X.
+__host__ __device__ constexpr int fluxSlot(int c) { return c < 5 ? c : c - 1; }
 
 struct Ctx {
   O4Args a;
   int d;
-  Box3 V, G, GR, GD, F, F1, F2, V0, V1, V2;
-  Reg gr, fr, v1r, v2r, vr;
+  Box3 V, G, GR, GD, F, F1, V0, V1;
+  Reg gr, fr, v1r, vr;
 };
 
 // Regions the operator's kernels loop over (host and device agree through
-// this one table): the work lists of a batch are built from it.
-enum RegionId { RG_G = 0, RG_GR, RG_F, RG_PB, RG_F1, RG_V0, RG_V, RG_PF, RG_PP, RG_V1, RG_V2, RG_COUNT };
+// this one table): the work lists of a batch are built from it.  The face
+// regions are walked for all three directions by one launch.
+enum RegionId { RG_G = 0, RG_GR, RG_V, RG_V1, RG_F, RG_PB, RG_V0, RG_PF, RG_COUNT };
+__host__ __device__ constexpr bool faceRegion(int id) { return id >= RG_F; }
 __host__ __device__ inline Box3 regionOf(const Ctx& c, int id) {
   switch (id) {
     case RG_G: return c.G;
     case RG_GR: return c.GR;
+    case RG_V: return c.V;
+    case RG_V1: return c.V1;
     case RG_F: return c.F;
     case RG_PB: return c.V0.growTrans(c.d, 1);
-    case RG_F1: return c.F1;
     case RG_V0: return c.V0;
-    case RG_V: return c.V;
-    case RG_PF: return c.V1.extrude(c.d).growTrans(c.d, 1);
-    case RG_PP: return c.V1.extrude(c.d);
-    case RG_V1: return c.V1;
-    default: return c.V2;
+    default: return c.V1.extrude(c.d).growTrans(c.d, 1);
   }
 }
+// Points a CTA takes per pass: the face averages give up one thread at each
+// end, whose averages only serve their neighbours.
+constexpr int kAvgPoints = 126;
+__host__ __device__ constexpr int passPoints(int id) { return id == RG_PB ? kAvgPoints : 128; }
 
-// One CTA's work: flat points begin, begin + stride, ... below end (each
-// thread adds its index) of one region of box `box`.
+// One CTA's work: flat points begin .. end - 1 of one region of box `box`,
+// direction `dir`.
 struct WorkChunk {
-  int box, stride;
+  int box, dir;
   long begin, end;
 };
-// Points per CTA (128 threads) of a work list: its total points over about
-// 148 x 32 CTAs, rounded up to whole passes of the CTA and held within
-// [128, 1024], so one launch has as many CTAs whatever the box sizes.
-inline long chunkPoints(long total) {
-  const long target = (total + 148L * 32 - 1) / (148L * 32);
-  const long c = ((target + 127) / 128) * 128;
-  return c < 128 ? 128 : c > 1024 ? 1024 : c;
+// Points per CTA of a work list: its total points over about 148 x 16 CTAs,
+// rounded up to whole passes of the CTA and held within 1 to 16 passes, so
+// one launch has as many CTAs whatever the box sizes.
+inline long chunkPoints(long total, long pass) {
+  const long target = (total + 148L * 16 - 1) / (148L * 16);
+  const long passes = (target + pass - 1) / pass;
+  return pass * (passes < 1 ? 1 : passes > 16 ? 16 : passes);
 }
 
 // The box the face arrays of every direction are laid out on: the face
-// boxes G.extrude(d).grow(-3) together, its radial extent rounded up to an
-// even count so that a radial row of doubles spans a multiple of 16 bytes
-// (the strides a TMA tensor map accepts).
+// boxes G.extrude(d).grow(-3) together.
 Box3 faceBox(const Box3& G) {
   Box3 FB = G.grow(-3);
   for (int q = 0; q < 3; ++q) FB.hi[q] += 1;
-  if (FB.n(0) & 1) FB.hi[0] += 1;
   return FB;
 }
 
@@ -113,36 +120,34 @@ Ctx makeCtx(const O4Args& a, int d) {
   Ctx c;
   c.a = a;
   c.d = d;
-  // direction 1 keeps its face arrays apart, so its pass can run beside the
-  // passes of directions 0 and 2
-  if (d == 1) c.a.face = a.face2;
   for (int q = 0; q < 3; ++q) { c.V.lo[q] = a.vlo[q]; c.V.hi[q] = a.vhi[q]; }
   c.G = c.V.grow(a.ghost);
   c.GR = c.G.grow(-1);
   c.GD = c.G.grow(-2);
   c.F = c.G.extrude(d).grow(-3);
   c.F1 = c.F.growTrans(d, -1);
-  c.F2 = c.F1.growTrans(d, -1);
   c.V0 = c.V.extrude(d);
   c.V1 = c.V.grow(1);
-  c.V2 = c.V.grow(2);
   c.gr = regOf(c.G);
   // face scratch is laid out on the largest face box over the directions
   c.fr = regOf(faceBox(c.G));
   c.v1r = regOf(c.V1);
-  c.v2r = regOf(c.V2);
   c.vr = a.rr.N ? a.rr : regOf(c.V);
   return c;
 }
 
 // ---- geometry access -------------------------------------------------------
+// Position of angular (j, k) of a panel in the metric tables.
+__device__ __forceinline__ long angular(const O4Geo& g, long plane, int j, int k) {
+  const int n = g.na + 2 * g.ext + 1;
+  return (plane * n + (k + g.ext)) * n + (j + g.ext);
+}
 __device__ __forceinline__ const double* faceRec(const O4Geo& g, int block, int d, int j, int k) {
-  const long n = g.na + 2 * g.ext + 1;
-  return g.face + ((((long)block * 3 + d) * n + (k + g.ext)) * n + (j + g.ext)) * kO4FaceRec;
+  return d == 0 ? g.face0 + angular(g, block, j, k) * kO4FaceRec0
+                : g.face12 + angular(g, block * 2 + (d - 1), j, k) * kO4FaceRec12;
 }
 __device__ __forceinline__ const double* roeRec(const O4Geo& g, int block, int d, int j, int k) {
-  const long n = g.na + 2 * g.ext + 1;
-  return g.frames + ((((long)block * 3 + d) * n + (k + g.ext)) * n + (j + g.ext)) * kO4RoeRec;
+  return g.frames + angular(g, block * 3 + d, j, k) * kO4RoeRec;
 }
 __device__ __forceinline__ const double* cellBasis(const O4Geo& g, int block, int j, int k) {
   const long n = g.na + 2 * g.ext + 1;
@@ -182,35 +187,6 @@ __device__ __forceinline__ void sphToPrim(const double u[8], const double* A, do
   ke *= w[0];
   w[4] = (w[4] - ke - me) * (gamma - 1.0);
   if (w[4] < 0.0) w[4] = 0.0;
-}
-
-// EnergyW (src/BoxOp_Utilities.H:447-520)
-__device__ __forceinline__ void energyW(const double w[8], const double* A, double& ke, double& me, double& vb) {
-  ke = 0.; me = 0.; vb = 0.;
-#pragma unroll
-  for (int d0 = 0; d0 < 3; ++d0) {
-    const double vc = A[3 * d0] * w[1] + A[3 * d0 + 1] * w[2] + A[3 * d0 + 2] * w[3];
-    const double bc = A[3 * d0] * w[5] + A[3 * d0 + 1] * w[6] + A[3 * d0 + 2] * w[7];
-    ke += vc * vc;
-    me += bc * bc * kInv8Pi;
-    vb += vc * bc;
-  }
-  ke *= w[0] * .5;
-}
-
-// f_primflux (src/BoxOp_EulerCubedSphere.H:195-225)
-__device__ __forceinline__ void primFlux(double f[8], const double w[8], double ke, double me, double vb, double gamma, int c) {
-  const int c1 = (c + 1) % 3, c2 = (c + 2) % 3;
-  const double velnorm = w[c + 1], veltan1 = w[c1 + 1], veltan2 = w[c2 + 1];
-  const double bnorm = w[c + 5], btan1 = w[c1 + 5], btan2 = w[c2 + 5];
-  f[0] = w[0] * velnorm;
-  f[c + 1] = f[0] * velnorm - bnorm * bnorm * kInv4Pi;
-  f[c1 + 1] = f[0] * veltan1 - bnorm * btan1 * kInv4Pi;
-  f[c2 + 1] = f[0] * veltan2 - bnorm * btan2 * kInv4Pi;
-  f[4] = (2.0 * me + ke + w[4] * gamma / (gamma - 1.0)) * velnorm - bnorm * vb * kInv4Pi;
-  f[5] = velnorm * w[5] - w[1] * bnorm;
-  f[6] = velnorm * w[6] - w[2] * bnorm;
-  f[7] = velnorm * w[7] - w[3] * bnorm;
 }
 
 // bertaNormalizeWenoStencil (:747-773)
@@ -331,63 +307,13 @@ __device__ __forceinline__ bool usablePrimitive(const double w[8]) {
   return ok && w[0] >= kRHO00 && w[4] >= 0.0;
 }
 
-// mappedRoe8WaveDissipation + factoredRoe8WaveDissipation (src/MHD_Roe8Wave.H:634-740)
-// with the face's products from the Roe frame table R (kO4RoeRec): one 3 x 3
-// matrix takes native vectors into the face frame (F A), the 8-wave
-// dissipation (Rusanov where the fan check fails) is taken there, and one
-// matrix takes it back (|n| adj A F^T / det A^2); the angular products are
-// in the table, so a vector costs nine operations each way.  The second
-// matrix is read after the solver (roeLoad2 is not merged with the first
-// read), so it does not occupy registers while the solver runs.
+// Pairs of a face's record in the frame table.  The second half is read
+// after the solver (volatile: not merged with an earlier read), so it does
+// not occupy registers while the solver runs.
 __device__ __forceinline__ double2 roeLoad2(const double* p) {
   double2 v;
   asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
   return v;
-}
-
-__device__ __forceinline__ void factoredRoe(double out[8], const double* wl, const double* wr,
-                                            const double* __restrict__ R, double radialArea, double gamma,
-                                            double invGm1, double entropy) {
-  double loc[2][8];
-  {
-    double f[10];
-#pragma unroll
-    for (int q = 0; q < 5; ++q) {
-      const double2 v = roeLoad2(R + 2 * q);
-      f[2 * q] = v.x;
-      f[2 * q + 1] = v.y;
-    }
-#pragma unroll
-    for (int side = 0; side < 2; ++side) {
-      const double* w = side == 0 ? wl : wr;
-      loc[side][0] = fmax(w[0], kRHO00);
-      loc[side][4] = fmax(w[4], 0.0);
-#pragma unroll
-      for (int r = 0; r < 3; ++r) {
-        loc[side][1 + r] = dot3(f[3 * r], w[1], f[3 * r + 1], w[2], f[3 * r + 2], w[3]);
-        loc[side][5 + r] = dot3(f[3 * r], w[5], f[3 * r + 1], w[6], f[3 * r + 2], w[7]);
-      }
-    }
-  }
-  double diss[8];
-  if (!roe8Body<true>(diss, loc[0], loc[1], gamma, entropy, invGm1))
-    rusanovDissipation(diss, loc[0], loc[1], gamma, invGm1);
-  double g[12];
-#pragma unroll
-  for (int q = 0; q < 6; ++q) {
-    const double2 v = roeLoad2(R + 8 + 2 * q);
-    g[2 * q] = v.x;
-    g[2 * q + 1] = v.y;
-  }
-  // g[1 .. 9] the matrix back, g[10] = |n| / det A
-  const Rn area = radialArea;
-  out[0] = area * (Rn(g[10]) * diss[0]);
-  out[4] = area * (Rn(g[10]) * diss[4]);
-#pragma unroll
-  for (int dd = 0; dd < 3; ++dd) {
-    out[1 + dd] = area * dot3(g[1 + 3 * dd], diss[1], g[2 + 3 * dd], diss[2], g[3 + 3 * dd], diss[3]);
-    out[5 + dd] = area * dot3(g[1 + 3 * dd], diss[5], g[2 + 3 * dd], diss[6], g[3 + 3 * dd], diss[7]);
-  }
 }
 
 // ---- stencils on scratch arrays --------------------------------------------
@@ -398,50 +324,54 @@ struct View {
 };
 
 
-__device__ __forceinline__ double lapFace(const View& f, int c, int d, int i, int j, int k) {
-  const int t1 = d == 0 ? 1 : 0, t2 = d == 2 ? 1 : 2;
-  int a[3] = {i, j, k}, b[3] = {i, j, k}, e[3] = {i, j, k}, g[3] = {i, j, k};
-  a[t1] -= 1; b[t1] += 1; e[t2] -= 1; g[t2] += 1;
-  return (f(c, a[0], a[1], a[2]) + f(c, b[0], b[1], b[2])) + (f(c, e[0], e[1], e[2]) + f(c, g[0], g[1], g[2])) -
-         4.0 * f(c, i, j, k);
-}
-
-__device__ __forceinline__ double cdiff(const View& f, int c, int t, int i, int j, int k) {
-  int a[3] = {i, j, k}, b[3] = {i, j, k};
-  a[t] += 1; b[t] -= 1;
-  return 0.5 * f(c, a[0], a[1], a[2]) - 0.5 * f(c, b[0], b[1], b[2]);
-}
-
 __device__ __forceinline__ double lapCell(const View& f, int c, int i, int j, int k) {
   return (f(c, i - 1, j, k) + f(c, i + 1, j, k)) + (f(c, i, j - 1, k) + f(c, i, j + 1, k)) +
          (f(c, i, j, k - 1) + f(c, i, j, k + 1)) - 6.0 * f(c, i, j, k);
 }
 
-__device__ __forceinline__ double faceProd(double f4, double g4, double df0, double dg0, double df1, double dg1) {
-  double value = 0.0;
-  value += df0 * dg0 * (1.0 / 12.0);
-  value += df1 * dg1 * (1.0 / 12.0);
-  value += f4 * g4 * 1.0;
-  return value;
+// Order in which a work list's flat points cover a region (radial index
+// fastest): a CTA's contiguous points then march along the direction its
+// stencil reaches, and the rows that its next pass needs are in L1.
+//   WALK_J  j, then k
+//   WALK_K  k, then j
+//   WALK_JK k over strips of kStrip rows of j, strip by strip (both)
+enum Walk { WALK_J = 0, WALK_K, WALK_JK };
+constexpr int kStrip = 8;
+
+// Point t of region b: regions hold fewer than 2^31 points (o4BatchCreate
+// rejects larger boxes), so the index split runs in 32-bit unsigned
+// arithmetic.
+__device__ __forceinline__ void pointOf(const Box3& b, int walk, unsigned t, int& i, int& j, int& k) {
+  const unsigned n0 = (unsigned)b.n(0), n1 = (unsigned)b.n(1), n2 = (unsigned)b.n(2);
+  unsigned q = t / n0;
+  i = b.lo[0] + (int)(t - q * n0);
+  unsigned row, col;
+  if (walk == WALK_JK) {
+    const unsigned strip = q / (kStrip * n2), first = strip * kStrip;
+    const unsigned rows = n1 - first < (unsigned)kStrip ? n1 - first : (unsigned)kStrip;
+    q -= first * n2;
+    col = q / rows;
+    row = first + (q - col * rows);
+  } else if (walk == WALK_K) {
+    row = q / n2;
+    col = q - row * n2;
+  } else {
+    col = q / n1;
+    row = q - col * n1;
+  }
+  j = b.lo[1] + (int)row;
+  k = b.lo[2] + (int)col;
 }
 
-
-// Thread -> (i, j, k) over the chunk's points of region b (flat index,
-// radial fastest) of the chunk's box; the end is clamped to the region.
-// Regions hold fewer than 2^31 points (o4BatchCreate rejects larger boxes),
-// so the index split runs in 32-bit unsigned arithmetic: two hardware-sized
-// divisions per point instead of three 64-bit ones.
+// Thread -> (i, j, k) over the chunk's points of region b of the chunk's box.
 template <class F>
-__device__ __forceinline__ void forRegion(const Box3& b, const WorkChunk& w, F f) {
-  const unsigned n0 = (unsigned)b.n(0), n1 = (unsigned)b.n(1);
-  const unsigned n = n0 * n1 * (unsigned)b.n(2);
+__device__ __forceinline__ void forRegion(const Box3& b, int walk, const WorkChunk& w, F f) {
+  const unsigned n = (unsigned)b.n(0) * (unsigned)b.n(1) * (unsigned)b.n(2);
   const unsigned end = w.end < (long)n ? (unsigned)w.end : n;
-  for (unsigned t = (unsigned)w.begin + threadIdx.x; t < end; t += (unsigned)w.stride) {
-    const unsigned q = t / n0, kk = q / n1;
-    const int i = b.lo[0] + (int)(t - q * n0);
-    const int j = b.lo[1] + (int)(q - kk * n1);
-    const int k = b.lo[2] + (int)kk;
-    f(0, i, j, k);
+  for (unsigned t = (unsigned)w.begin + threadIdx.x; t < end; t += 128u) {
+    int i, j, k;
+    pointOf(b, walk, t, i, j, k);
+    f(i, j, k);
   }
 }
 
@@ -455,19 +385,15 @@ __global__ void o4PrimAvgKernel(const Ctx* __restrict__ tab, const RegArgs rg, c
   const WorkChunk wc = wk[blockIdx.x];
   const Ctx& c = tab[wc.box * 3 + 0];
   const O4Args& a = c.a;
-  forRegion(c.G, wc, [&](int b, int i, int j, int k) {
+  forRegion(c.G, WALK_JK, wc, [&](int i, int j, int k) {
     double u[8], w[8];
-    const double* U = a.U + b * a.uStride + roff(a.ur, i, j, k);
+    const double* U = a.U + roff(a.ur, i, j, k);
 #pragma unroll
     for (int q = 0; q < 8; ++q) u[q] = U[q * a.ur.N];
-    sphToPrim(u, cellBasis(a.G, a.block0 + b, j, k), a.G.gamma, w);
-    double* W = a.WA + (long)b * 8 * c.gr.N + roff(c.gr, i, j, k);
+    sphToPrim(u, cellBasis(a.G, a.block0, j, k), a.G.gamma, w);
+    double* W = a.WA + roff(c.gr, i, j, k);
 #pragma unroll
     for (int q = 0; q < 8; ++q) W[q * c.gr.N] = w[q];
-    // the Powell accumulator -J div B starts at zero on V1
-    if (a.G.powell && i >= c.V1.lo[0] && i <= c.V1.hi[0] && j >= c.V1.lo[1] && j <= c.V1.hi[1] && k >= c.V1.lo[2] &&
-        k <= c.V1.hi[2])
-      a.mj[(long)b * c.v1r.N + roff(c.v1r, i, j, k)] = 0.0;
   });
 }
 
@@ -486,8 +412,8 @@ __global__ void o4ThetaRawKernel(const Ctx* __restrict__ tab, const RegArgs rg, 
   const WorkChunk wc = wk[blockIdx.x];
   const Ctx& c = tab[wc.box * 3 + 0];
   const O4Args& a = c.a;
-  forRegion(c.GR, wc, [&](int b, int i, int j, int k) {
-    const double* W = a.WA + (long)b * 8 * c.gr.N;
+  forRegion(c.GR, WALK_JK, wc, [&](int i, int j, int k) {
+    const double* W = a.WA;
     const long N = c.gr.N, o = roff(c.gr, i, j, k);
     double et[3];
 #pragma unroll
@@ -501,7 +427,7 @@ __global__ void o4ThetaRawKernel(const Ctx* __restrict__ tab, const RegArgs rg, 
       et[d] = dmax(er, dmax(ep, em));
     }
     const double eta = sqrt(et[0] * et[0] + et[1] * et[1] + et[2] * et[2]);
-    a.thr[(long)b * N + o] = eta < a.G.eta_d ? 1.0 : 0.0;
+    a.thr[o] = eta < a.G.eta_d ? 1.0 : 0.0;
   });
 }
 
@@ -511,9 +437,9 @@ __global__ void o4PointKernel(const Ctx* __restrict__ tab, const RegArgs rg, con
   const WorkChunk wc = wk[blockIdx.x];
   const Ctx& c = tab[wc.box * 3 + 0];
   const O4Args& a = c.a;
-  forRegion(c.G, wc, [&](int b, int i, int j, int k) {
+  forRegion(c.G, WALK_JK, wc, [&](int i, int j, int k) {
     const long N = c.gr.N, o = roff(c.gr, i, j, k);
-    const double* R = a.thr + (long)b * N;
+    const double* R = a.thr;
     double t = 0.0;
     const bool inD = i >= c.GD.lo[0] && i <= c.GD.hi[0] && j >= c.GD.lo[1] && j <= c.GD.hi[1] && k >= c.GD.lo[2] &&
                      k <= c.GD.hi[2];
@@ -528,305 +454,581 @@ __global__ void o4PointKernel(const Ctx* __restrict__ tab, const RegArgs rg, con
     }
     const bool inner = i >= c.GR.lo[0] && i <= c.GR.hi[0] && j >= c.GR.lo[1] && j <= c.GR.hi[1] &&
                        k >= c.GR.lo[2] && k <= c.GR.hi[2];
-    View U{a.U + b * a.uStride, a.ur};
+    View U{a.U, a.ur};
     double u[8], w[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) u[q] = (inner && t > 0.5) ? U(q, i, j, k) - lapCell(U, q, i, j, k) * (1.0 / 24.0) : U(q, i, j, k);
-    sphToPrim(u, cellBasis(a.G, a.block0 + b, j, k), a.G.gamma, w);
-    double* W = a.WP + (long)b * 8 * N + o;
+    sphToPrim(u, cellBasis(a.G, a.block0, j, k), a.G.gamma, w);
+    double* W = a.WP + o;
 #pragma unroll
     for (int q = 0; q < 8; ++q) W[q * N] = w[q];
     // stored last: a store ahead of the state loads would hold them back
     // until the dilation's loads return
-    a.th[(long)b * N + o] = t;
+    a.th[o] = t;
   });
 }
 
-__device__ __forceinline__ double* faceArr(const Ctx& c, int b, int arr) {
-  return c.a.face + ((long)b * kO4FaceArrays + arr) * c.fr.N;
+__device__ __forceinline__ double* faceArr(const Ctx& c, int arr) { return c.a.face[c.d] + arr * c.fr.N; }
+// Asynchronous copy of one double to shared memory.
+__device__ __forceinline__ void copyAsync(double* dst, const double* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
-__device__ __forceinline__ View faceView(const Ctx& c, int b, int arr) { return View{faceArr(c, b, arr), c.fr}; }
-template <int D>
-__device__ __forceinline__ const double* faceBasis(const Ctx& c, int b, int j, int k) {
-  return D == 0 ? cellBasis(c.a.G, c.a.block0 + b, j, k) : faceRec(c.a.G, c.a.block0 + b, D, j, k) + 13;
+// Strides of the two directions transverse to d in an array laid out on r,
+// lower direction first.
+__device__ __forceinline__ int2 transverse(const Reg& r, int d) {
+  return make_int2(d == 0 ? r.n[0] : 1, d == 2 ? r.n[0] : r.n[0] * r.n[1]);
+}
+__device__ __forceinline__ int stride(const Reg& r, int d) { return d == 0 ? 1 : d == 1 ? r.n[0] : r.n[0] * r.n[1]; }
+
+// Component array of place q of the (rho, m_n, m_1, m_2, E, B_n, B_1, B_2)
+// order along direction d.
+__device__ __forceinline__ int place(int q, int d) {
+  const int first = q > 4 ? 5 : 1;
+  if (q == 0 || q == 4) return q;
+  const int e = d + q - first;
+  return first + (e > 2 ? e - 3 : e);
 }
 
-// 4. reconstruction (WENOZ / WENO3 / PLM with clamps), Roe repair, energies,
-// point flux sum, total-pressure sum, centred normal B, Rusanov jump (F).
-template <int D, int MB>
+// 4a. Reconstruction (WENOZ / WENO3 / PLM) of the eight components on both
+// sides of every face of F, and the face's flag; the Riemann kernel clamps.
+//
+// One thread per face, one launch for the three directions.  The kernel
+// holds two components at a time: with the Riemann solver in the same kernel
+// it took 128 registers, and 16 warps an SM are too few for the latency of
+// the FP64 chains (64 x 32^2 x 6, three directions: 325 us against NN + NN).
+// Pairs of components in a loop: all eight unrolled overflow the
+// instruction cache.
+template <int MB>
 __global__ void __launch_bounds__(128, MB) o4FaceReconKernel(const Ctx* __restrict__ tab, const RegArgs rg, const WorkChunk* __restrict__ wk) {
   const WorkChunk wc = wk[blockIdx.x];
-  const Ctx& c = tab[wc.box * 3 + D];
+  const int d = wc.dir;
+  const Ctx& c = tab[wc.box * 3 + d];
   const O4Args& a = c.a;
-  constexpr int d = D;
+  const long NG = c.gr.N, NF = c.fr.N;
+  const int st = stride(c.gr, d);
   const double dx2 = a.G.dx[d] * a.G.dx[d];
-  forRegion(c.F, wc, [&](int b, int i, int j, int k) {
-    const long NG = c.gr.N, NF = c.fr.N;
-    const double* th = a.th + (long)b * NG;
-    const double* WP = a.WP + (long)b * 8 * NG;
-    const double* WA = a.WA + (long)b * 8 * NG;
-    long cell[6];
+  forRegion(c.F, d == 2 ? WALK_K : WALK_J, wc, [&](int i, int j, int k) {
+    const long o = roff(c.gr, i, j, k);
+    const double* W = a.WP + o;
+    double v[6], nx[6];
 #pragma unroll
-    for (int s = -3; s <= 2; ++s) {
-      int q[3] = {i, j, k};
-      q[d] += s;
-      cell[s + 3] = roff(c.gr, q[0], q[1], q[2]);
-    }
-    const long fo = roff(c.fr, i, j, k);
-    double thF = dmin(th[cell[2]], th[cell[3]]);
-    double value = th[cell[0]];
-    value = dmin(value, th[cell[1]]);
-    value = dmin(value, th[cell[2]]);
-    value = dmin(value, th[cell[3]]);
-    value = dmin(value, th[cell[4]]);
-    const double thR = dmin(value, th[cell[5]]);
-    const bool smooth = thR > 0.5;
-    // one copy of the reconstruction code for the eight components (a rolled
-    // loop; the states go through this thread's shared-memory column)
-    __shared__ double sLR[16][128];
-    // the next component's six cells are loaded while this one is
-    // reconstructed (all six cells lie in G for every face of F)
-    double nx[6];
+    for (int m = 0; m < 6; ++m) nx[m] = __ldg(W + (m - 3) * st);
+    double th[6];
 #pragma unroll
-    for (int s = 0; s < 6; ++s) nx[s] = WP[cell[s]];
-#pragma unroll 1
-    for (int q = 0; q < 8; ++q) {
-      const double cur[6] = {nx[0], nx[1], nx[2], nx[3], nx[4], nx[5]};
-      if (q < 7) {
-        const double* Wn = WP + (q + 1) * NG;
-#pragma unroll
-        for (int s = 0; s < 6; ++s) nx[s] = Wn[cell[s]];
-      }
-      double L, R;
+    for (int m = 0; m < 6; ++m) th[m] = __ldg(a.th + o + (m - 3) * st);
+    const double thF = dmin(th[2], th[3]);
+    const bool smooth = dmin(dmin(th[0], th[1]), dmin(thF, dmin(th[4], th[5]))) > 0.5;
+    double* out = faceArr(c, F_L) + roff(c.fr, i, j, k);
+    out[(F_THF - F_L) * NF] = thF;
+    auto states = [&](const double (&x)[6]) {
+      double l, r;
       if (smooth) {
-        wenozFace(cur, L, R);
+        wenozFace(x, l, r);
       } else {
-        const double st[4] = {cur[1], cur[2], cur[3], cur[4]};
-        if (a.G.fallback == 0) weno3Face(st, dx2, L, R);
-        else plmFallbackFace(st, L, R);
+        const double y[4] = {x[1], x[2], x[3], x[4]};
+        if (a.G.fallback == 0) weno3Face(y, dx2, l, r);
+        else plmFallbackFace(y, l, r);
       }
-      if (q == 0) { L = dmax(L, kRHO00); R = dmax(R, kRHO00); }
-      if (q == 4) { L = dmax(L, 1.0e-12); R = dmax(R, 1.0e-12); }
-      sLR[q][threadIdx.x] = L;
-      sLR[8 + q][threadIdx.x] = R;
+      out[0] = l;
+      out[(F_R - F_L) * NF] = r;
+      out += NF;
+    };
+    // the next component's cells are loaded while one is reconstructed
+#pragma unroll 1
+    for (int q = 0; q < 8; q += 2) {
+      W += NG;
+#pragma unroll
+      for (int m = 0; m < 6; ++m) v[m] = __ldg(W + (m - 3) * st);
+      states(nx);
+      if (q < 6) {
+        W += NG;
+#pragma unroll
+        for (int m = 0; m < 6; ++m) nx[m] = __ldg(W + (m - 3) * st);
+      }
+      states(v);
     }
+  });
+}
+
+// 4b. Riemann problem of every face of F: Roe repair, point flux sum,
+// total-pressure sum, centred normal B, and the point dissipation: factored
+// Roe (src/BoxOp_RoeCubedSphere.H:73-98, mappedRoe8WaveDissipation +
+// factoredRoe8WaveDissipation, src/MHD_Roe8Wave.H:634-740) on the final
+// faces plus one transverse ring, or the Rusanov jump and the face's speed
+// bound (src/BoxOp_BertaCubedSphereImplem.H:1665-1720).
+//
+// The next pass's states are copied to shared memory while this pass is
+// solved (cp.async, each thread its own column, no barrier), its frame record
+// prefetched.
+//
+// One 3 x 3 matrix (F A of the frame table) turns both states into the face
+// frame, where the energies, fluxes and the Roe solver use them; one matrix
+// (|n| adj A F^T / det A^2) takes the dissipation back.
+template <bool ROE, int MB>
+__global__ void __launch_bounds__(128, MB) o4FaceRiemannKernel(const Ctx* __restrict__ tab, const RegArgs rg, const WorkChunk* __restrict__ wk) {
+  const WorkChunk wc = wk[blockIdx.x];
+  const int d = wc.dir;
+  const Ctx& c = tab[wc.box * 3 + d];
+  const O4Args& a = c.a;
+  const bool roe = ROE && roeNow(a.G);
+  const long NF = c.fr.N;
+  const int blk = a.block0;
+  // states of this pass and the next, a column per thread
+  __shared__ double sh[2][16][128];
+  const Box3 F = c.F;
+  auto fetch = [&](unsigned t, int slot) {
+    int i, j, k;
+    pointOf(F, WALK_J, t, i, j, k);
+    const double* src = faceArr(c, F_L) + roff(c.fr, i, j, k);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      copyAsync(&sh[slot][q][threadIdx.x], src + place(q, d) * NF);
+      copyAsync(&sh[slot][8 + q][threadIdx.x], src + (F_R - F_L + place(q, d)) * NF);
+    }
+    const double* R = roeRec(a.G, blk, d, j, k);
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(R));
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(R + 16));
+  };
+  const unsigned end = (unsigned)wc.end;
+  int slot = 0;
+  if ((unsigned)wc.begin + threadIdx.x < end) fetch((unsigned)wc.begin + threadIdx.x, 0);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  for (unsigned t = (unsigned)wc.begin + threadIdx.x; t < end; t += 128u, slot ^= 1) {
+    if (t + 128u < end) fetch(t + 128u, slot ^ 1);
+    asm volatile("cp.async.commit_group;\n cp.async.wait_group 1;" ::: "memory");
+    int i, j, k;
+    pointOf(F, WALK_J, t, i, j, k);
+    double* const base = faceArr(c, 0) + roff(c.fr, i, j, k);
     double l[8], r[8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) { l[q] = sLR[q][threadIdx.x]; r[q] = sLR[8 + q][threadIdx.x]; }
-    // Roe repair: only faces whose reconstructed states are unusable read
-    // the adjacent cells' average primitives (most faces never do)
-    if (roeNow(a.G) && !(usablePrimitive(l) && usablePrimitive(r))) {
+    for (int q = 0; q < 8; ++q) { l[q] = sh[slot][q][threadIdx.x]; r[q] = sh[slot][8 + q][threadIdx.x]; }
+    l[0] = dmax(l[0], kRHO00); r[0] = dmax(r[0], kRHO00);
+    l[4] = dmax(l[4], 1.0e-12); r[4] = dmax(r[4], 1.0e-12);
+    const Rn area = radialPoint(a.G, d, i);
+    // only faces whose reconstructed states are unusable read the adjacent
+    // cells' average primitives (most faces never do)
+    if (roe && !(usablePrimitive(l) && usablePrimitive(r))) {
+      const long o = roff(c.gr, i, j, k);
+      const int st = stride(c.gr, d);
       double cl[8], cr[8];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) { cl[q] = WA[q * NG + cell[2]]; cr[q] = WA[q * NG + cell[3]]; }
+      for (int q = 0; q < 8; ++q) {
+        const double* W = a.WA + place(q, d) * c.gr.N + o;
+        cl[q] = W[-st];
+        cr[q] = W[0];
+      }
       if (usablePrimitive(cl) && usablePrimitive(cr)) {
 #pragma unroll
         for (int q = 0; q < 8; ++q) { l[q] = cl[q]; r[q] = cr[q]; }
-        thF = 0.0;
+        base[F_THF * NF] = 0.0;
       }
     }
-    double* base = a.face + (long)b * kO4FaceArrays * NF + fo;
+    const double* R = roeRec(a.G, blk, d, j, k);
+    double f[10];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) { base[(F_WL + q) * NF] = l[q]; base[(F_WR + q) * NF] = r[q]; }
-    base[F_THF * NF] = thF;
-    const double* A = faceBasis<D>(c, b, j, k);
-    double kl, ml, vl, kr, mr, vr, fl[8], fr[8];
-    energyW(l, A, kl, ml, vl);
-    energyW(r, A, kr, mr, vr);
-    primFlux(fl, l, kl, ml, vl, a.G.gamma, d);
-    primFlux(fr, r, kr, mr, vr, a.G.gamma, d);
+    for (int q = 0; q < 5; ++q) {
+      const double2 v = roeLoad2(R + 2 * q);
+      f[2 * q] = v.x;
+      f[2 * q + 1] = v.y;
+    }
+    double loc[2][8];
+    Rn fs[7], ps = 0.0, energy[2];
+    const double enthalpy = a.G.gamma * a.G.invGm1;
 #pragma unroll
-    for (int q = 0; q < 8; ++q) base[(F_FS + q) * NF] = fl[q] + fr[q];
-    base[F_PS * NF] = (l[4] + ml) + (r[4] + mr);
-    base[F_BP * NF] = (l[5 + d] + r[5 + d]) * 0.5;
-    if (!roeNow(a.G)) {
-      const double rad = radialPoint(a.G, d, i);
-      const double g = a.G.gamma;
-      base[(F_QD + 0) * NF] = rad * r[0] - rad * l[0];
+    for (int side = 0; side < 2; ++side) {
+      const double* w = side == 0 ? l : r;
+      double* q = loc[side];
+      q[0] = w[0];
+      q[4] = w[4];
 #pragma unroll
       for (int e = 0; e < 3; ++e) {
-        base[(F_QD + 1 + e) * NF] = rad * r[0] * r[1 + e] - rad * l[0] * l[1 + e];
-        base[(F_QD + 5 + e) * NF] = rad * r[5 + e] - rad * l[5 + e];
+        q[1 + e] = dot3(f[3 * e], w[1], f[3 * e + 1], w[2], f[3 * e + 2], w[3]);
+        q[5 + e] = dot3(f[3 * e], w[5], f[3 * e + 1], w[6], f[3 * e + 2], w[7]);
       }
-      base[(F_QD + 4) * NF] = rad * (kr + mr + r[4] / (g - 1.0)) - rad * (kl + ml + l[4] / (g - 1.0));
+      // energies (EnergyW, src/BoxOp_Utilities.H:447-520) and f_primflux
+      // (src/BoxOp_EulerCubedSphere.H:195-225)
+      const Rn ke = 0.5 * Rn(w[0]) * dot3(q[1], q[1], q[2], q[2], q[3], q[3]);
+      const Rn me = kInv8Pi * dot3(q[5], q[5], q[6], q[6], q[7], q[7]);
+      const Rn vb = dot3(q[1], q[5], q[2], q[6], q[3], q[7]);
+      const Rn mass = Rn(w[0]) * w[1], bn = -kInv4Pi * Rn(w[5]);
+      Rn g[7];
+      g[0] = mass;
+#pragma unroll
+      for (int e = 0; e < 3; ++e) g[1 + e] = mad(bn, w[5 + e], mass * w[1 + e]);
+      g[4] = mad(bn, vb, (mad(2.0, me, ke) + enthalpy * Rn(w[4])) * w[1]);
+#pragma unroll
+      for (int e = 1; e < 3; ++e) g[4 + e] = mad(w[1], w[5 + e], -(Rn(w[1 + e]) * w[5]));
+#pragma unroll
+      for (int q7 = 0; q7 < 7; ++q7) fs[q7] = side == 0 ? g[q7] : fs[q7] + g[q7];
+      ps = side == 0 ? me + w[4] : ps + (me + w[4]);
+      energy[side] = mad(w[4], a.G.invGm1, ke + me);
     }
-  });
-}
-
-// 4b. pointwise factored Roe dissipation on the final faces + one transverse
-// ring (src/BoxOp_RoeCubedSphere.H:73-98).
-template <int D, int MB>
-__global__ void __launch_bounds__(128, MB) o4RoePointKernel(const Ctx* __restrict__ tab, const RegArgs rg, const WorkChunk* __restrict__ wk) {
-  const WorkChunk wc = wk[blockIdx.x];
-  const Ctx& c = tab[wc.box * 3 + D];
-  const O4Args& a = c.a;
-  if (!roeNow(a.G)) return;  // the Rusanov window: the reconstruction wrote the Rusanov jump
-  constexpr int d = D;
-  const Box3 PB = c.V0.growTrans(d, 1);
-  forRegion(PB, wc, [&](int b, int i, int j, int k) {
-    const long NF = c.fr.N;
-    double* base = a.face + (long)b * kO4FaceArrays * NF + roff(c.fr, i, j, k);
-    double l[8], r[8], o[8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) { l[q] = base[(F_WL + q) * NF]; r[q] = base[(F_WR + q) * NF]; }
-    factoredRoe(o, l, r, roeRec(a.G, a.block0 + b, D, j, k), radialPoint(a.G, d, i), a.G.gamma, a.G.invGm1,
-                a.G.entropy);
+    for (int q = 0; q < 7; ++q) base[(F_FS + q) * NF] = fs[q];
+    base[F_PS * NF] = ps;
+    base[F_BP * NF] = 0.5 * (Rn(l[5]) + r[5]);
+    const Box3 PB = regionOf(c, RG_PB);
+    if (i < PB.lo[0] || i > PB.hi[0] || j < PB.lo[1] || j > PB.hi[1] || k < PB.lo[2] || k > PB.hi[2]) continue;
+    if (roe) {
 #pragma unroll
-    for (int q = 0; q < 8; ++q) base[(F_QD + q) * NF] = o[q];
-  });
-}
-
-// 10. Powell face flux (DivBPowell1, src/BoxOp_DivBcleaning.H:35-74).
-template <int D>
-__global__ void o4PowellFluxKernel(const Ctx* __restrict__ tab, const RegArgs rg, const WorkChunk* __restrict__ wk) {
-  const WorkChunk wc = wk[blockIdx.x];
-  const Ctx& c = tab[wc.box * 3 + D];
-  const O4Args& a = c.a;
-  constexpr int d = D;
-  const int t1 = d == 0 ? 1 : 0, t2 = d == 2 ? 1 : 2;
-  const int tr[2] = {t1, t2};
-  const Box3 BF = c.V1.extrude(d).growTrans(d, 1);
-  forRegion(BF, wc, [&](int b, int i, int j, int k) {
-    const long NF = c.fr.N, fo = roff(c.fr, i, j, k);
-    double* base = a.face + (long)b * kO4FaceArrays * NF;
-    const int blk = a.block0 + b;
-    const double det = faceRec(a.G, blk, d, j, k)[9];
-    double out;
-    if (base[F_THF * NF + fo] <= 0.5) {
-      out = det * base[F_BP * NF + fo];
+      for (int side = 0; side < 2; ++side) {
+        loc[side][0] = fmax(loc[side][0], kRHO00);
+        loc[side][4] = fmax(loc[side][4], 0.0);
+      }
+      double diss[8];
+      if (!roe8Body<true>(diss, loc[0], loc[1], a.G.gamma, a.G.entropy, a.G.invGm1))
+        rusanovDissipation(diss, loc[0], loc[1], a.G.gamma, a.G.invGm1);
+      double g[12];  // g[1 .. 9] the matrix back, g[10] = |n| / det A
+#pragma unroll
+      for (int q = 0; q < 6; ++q) {
+        const double2 v = roeLoad2(R + 8 + 2 * q);
+        g[2 * q] = v.x;
+        g[2 * q + 1] = v.y;
+      }
+      base[F_QD * NF] = area * (Rn(g[10]) * diss[0]);
+      base[(F_QD + 4) * NF] = area * (Rn(g[10]) * diss[4]);
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        base[(F_QD + 1 + e) * NF] = area * dot3(g[1 + 3 * e], diss[1], g[2 + 3 * e], diss[2], g[3 + 3 * e], diss[3]);
+        base[(F_QD + 5 + e) * NF] = area * dot3(g[1 + 3 * e], diss[5], g[2 + 3 * e], diss[6], g[3 + 3 * e], diss[7]);
+      }
     } else {
-      View U{a.U + b * a.uStride, a.ur};
-      auto bface = [&](int ii, int jj, int kk) {
-        int m2[3] = {ii, jj, kk}, m1[3] = {ii, jj, kk}, p1[3] = {ii, jj, kk};
-        m2[d] -= 2; m1[d] -= 1; p1[d] += 1;
-        return (7.0 / 12.0) * (U(5 + d, m1[0], m1[1], m1[2]) + U(5 + d, ii, jj, kk)) -
-               (1.0 / 12.0) * (U(5 + d, m2[0], m2[1], m2[2]) + U(5 + d, p1[0], p1[1], p1[2]));
-      };
-      double df[2], dg[2];
+      base[F_QD * NF] = area * (Rn(r[0]) - l[0]);
+      base[(F_QD + 4) * NF] = area * (energy[1] - energy[0]);
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int t = tr[q];
-        int pa[3] = {i, j, k}, pb[3] = {i, j, k};
-        pa[t] += 1; pb[t] -= 1;
-        df[q] = 0.5 * faceRec(a.G, blk, d, pa[1], pa[2])[9] - 0.5 * faceRec(a.G, blk, d, pb[1], pb[2])[9];
-        dg[q] = 0.5 * bface(pa[0], pa[1], pa[2]) - 0.5 * bface(pb[0], pb[1], pb[2]);
+      for (int e = 0; e < 3; ++e) {
+        base[(F_QD + 1 + e) * NF] = area * mad(r[0], r[1 + e], -(Rn(l[0]) * l[1 + e]));
+        base[(F_QD + 5 + e) * NF] = area * (Rn(r[5 + e]) - l[5 + e]);
       }
-      out = faceProd(det, bface(i, j, k), df[0], dg[0], df[1], dg[1]);
-    }
-    base[F_BFLUX * NF + fo] = out;
-  });
-}
-
-// 11. Powell radial-area product and divergence into -J div B (V+1).
-template <int D>
-__global__ void o4PowellProdKernel(const Ctx* __restrict__ tab, const RegArgs rg, const WorkChunk* __restrict__ wk) {
-  const WorkChunk wc = wk[blockIdx.x];
-  const Ctx& c = tab[wc.box * 3 + D];
-  const O4Args& a = c.a;
-  constexpr int d = D;
-  const int t1 = d == 0 ? 1 : 0, t2 = d == 2 ? 1 : 2;
-  const int tr[2] = {t1, t2};
-  const Box3 BP = c.V1.extrude(d);
-  forRegion(BP, wc, [&](int b, int i, int j, int k) {
-    const long NF = c.fr.N, fo = roff(c.fr, i, j, k);
-    double* base = a.face + (long)b * kO4FaceArrays * NF;
-    const View BF = faceView(c, b, F_BFLUX);
-    double df[2], dg[2];
+      // fast speed of the mean state, from the field along the radial basis
+      // vector; the mean normal velocity; |A_d|
+      double bm[3];
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int t = tr[q];
-      df[q] = cdiff(BF, 0, t, i, j, k);
-      dg[q] = t == 0 ? 0.5 * adjDr(a.G, d, i + 1) - 0.5 * adjDr(a.G, d, i - 1) : 0.0;
+      for (int e = 0; e < 3; ++e) bm[e] = 0.5 * (Rn(loc[0][5 + e]) + loc[1][5 + e]);
+      double ar[3];  // the matrix' radial column: place (3 - d) % 3 of the (d, d1, d2) order
+#pragma unroll
+      for (int e = 0; e < 3; ++e) ar[e] = d == 0 ? f[3 * e] : d == 1 ? f[3 * e + 2] : f[3 * e + 1];
+      const Rn bn = dot3(ar[0], bm[0], ar[1], bm[1], ar[2], bm[2]), b2 = dot3(bm[0], bm[0], bm[1], bm[1], bm[2], bm[2]);
+      const double rho = dmax(0.5 * (Rn(l[0]) + r[0]), kRHO00);
+      const double p = dmax(0.5 * (Rn(l[4]) + r[4]), 0.0);
+      const Rn rs = rsqrtN(rho), ce2 = a.G.gamma * Rn(p) * (rs * rs);
+      const Rn aa = mad(kInv4Pi * b2, rs * rs, ce2);
+      const Rn bb = Rn(fabs(bn.v)) * sqrtN(ce2) * rs * 0.56418958354775628694807945156077;  // 1 / sqrt(pi)
+      const Rn af = 0.5 * (Rn(sqrtN(aa + bb)) + sqrtN(aa - bb));
+      base[F_SPD * NF] = mad(af, sqrt(dot3(f[0], f[0], f[3], f[3], f[6], f[6]).v), fabs(0.5 * (Rn(l[1]) + r[1])));
     }
-    base[F_BPROD * NF + fo] = faceProd(BF(0, i, j, k), adjDr(a.G, d, i), df[0], dg[0], df[1], dg[1]);
-  });
+  }
 }
 
-template <int D>
-__global__ void o4PowellDivKernel(const Ctx* __restrict__ tab, const RegArgs rg, const WorkChunk* __restrict__ wk) {
+// 5. Theta-aware point-to-average of the flux sum and the total pressure, and
+// (7) their products with the radial areas: with the areas s(i) varying
+// radially only, X = s <F> + (1/12) D_r s D_r <F> on the final faces plus one
+// transverse ring (D_r s = 0 for d = 0, whose transverse directions are
+// angular).  The reference maps first and multiplies by the area after;
+// the metric factors of the mapping do not vary radially, so the two
+// commute, and the mapping then takes flux and dissipation together.
+//
+// One thread per face.  The radial neighbours' averages are the
+// neighbouring threads' (shared memory; the first and last thread of the
+// CTA only serve as neighbours).  HBM-bound: nine arrays read with four
+// neighbours each through L1, eight written.
+__global__ void __launch_bounds__(128, 8) o4FaceAvgKernel(const Ctx* __restrict__ tab, const RegArgs rg, const WorkChunk* __restrict__ wk) {
+  __shared__ double sh[8][128];
   const WorkChunk wc = wk[blockIdx.x];
-  const Ctx& c = tab[wc.box * 3 + D];
+  const int d = wc.dir, tid = threadIdx.x;
+  const Ctx& c = tab[wc.box * 3 + d];
+  const O4Geo& G = c.a.G;
+  const Box3 PB = regionOf(c, RG_PB);
+  const long NF = c.fr.N;
+  const int2 tr = transverse(c.fr, d);
+  const int n = PB.n(0) * PB.n(1) * PB.n(2);
+  for (long at = wc.begin; at < wc.end; at += kAvgPoints) {
+    const int t = (int)at + tid - 1;
+    const bool in = t >= 0 && t < n;
+    Rn fa[8];
+    int i = 0;
+    double* base = nullptr;
+    if (in) {
+      int j, k;
+      pointOf(PB, d == 0 ? WALK_JK : d == 1 ? WALK_K : WALK_J, (unsigned)t, i, j, k);
+      base = faceArr(c, 0) + roff(c.fr, i, j, k);
+      const double w = base[F_THF * NF] > 0.5 ? 1.0 / 24.0 : 0.0;
+      // the pressure sum follows the seven flux sums
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const double* F = base + (F_FS + e) * NF;
+        const Rn pt = __ldg(F);
+        const Rn lap = mad(-4.0, pt, (Rn(__ldg(F - tr.x)) + __ldg(F + tr.x)) + (Rn(__ldg(F - tr.y)) + __ldg(F + tr.y)));
+        fa[e] = w != 0.0 ? mad(lap, w, pt) : pt;
+      }
+    }
+    if (d != 0) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) sh[e][tid] = fa[e];
+      __syncthreads();
+    }
+    // outputs: the CTA's inner threads, below the chunk's end, radially on final faces
+    if (in && tid >= 1 && tid <= kAvgPoints && t < wc.end && i >= c.V0.lo[0] && i <= c.V0.hi[0]) {
+      const Rn s = adjDr(G, d, i);
+      if (d != 0) {
+        const Rn ds = (Rn(adjDr(G, d, i + 1)) - adjDr(G, d, i - 1)) * (1.0 / 48.0);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) fa[e] = mad(Rn(sh[e][tid + 1]) - sh[e][tid - 1], ds, s * fa[e]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) fa[e] = s * fa[e];
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) base[(F_X + e) * NF] = fa[e];
+    }
+    if (d != 0) __syncthreads();
+  }
+}
+
+// 6, 8. Final flux of every face: mapped flux with its transverse products,
+// pressure force, averaged dissipation.  Flux and dissipation are mapped by
+// the same metric averages M = <det A A>, so their difference is mapped
+// once: F = (1/2) [M Z + sum_t (1/12) D_t M D_t Y] with Z = X - sigma <Q>,
+// D_t Y = D_t X - D_t Q (Roe, sigma = 1; Q the point dissipation) or D_t X
+// (Rusanov, sigma the speed bound).  D_t M vanishes radially, so directions
+// 1 and 2 have one transverse product and direction 0 two.  The record
+// holds the halved M, det and normal and their angular differences / 48.
+//
+// One thread per face, no walk and no barrier: about 90 loads (five taps of
+// 15 arrays, the record) through L1.  The walk over face slabs staged by TMA
+// that this replaces ran at 10-20 % of the warp slots between its barriers
+// (66-80 KB of shared memory and 128 registers a CTA).
+template <int D0, class Load>
+__device__ __forceinline__ void finalFlux(const double* __restrict__ M, Load load, const double* __restrict__ T3, long ta, long tb, Rn fx[8]) {
+  // components in two vector groups and the two scalars
+  {
+    Rn z, ya, yb;
+    load(0, z, ya, yb);
+    fx[0] = mad(M[9], z, Rn(M[22]) * ya);
+    if (D0) fx[0] = mad(M[35], yb, fx[0]);
+    load(4, z, ya, yb);
+    fx[4] = mad(M[9], z, Rn(M[22]) * ya);
+    if (D0) fx[4] = mad(M[35], yb, fx[4]);
+  }
+#pragma unroll
+  for (int grp = 0; grp < 2; ++grp) {
+    const int b = grp == 0 ? 1 : 5;
+    Rn out[3];
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+      Rn z, ya, yb;
+      load(b + e, z, ya, yb);
+#pragma unroll
+      for (int row = 0; row < 3; ++row) {
+        const Rn first = e == 0 ? Rn(M[3 * row]) * z : mad(M[3 * row + e], z, out[row]);
+        out[row] = mad(M[13 + 3 * row + e], ya, first);
+        if (D0) out[row] = mad(M[26 + 3 * row + e], yb, out[row]);
+      }
+    }
+#pragma unroll
+    for (int row = 0; row < 3; ++row) fx[b + row] = out[row];
+  }
+  const Rn p = __ldg(T3), pa = Rn(__ldg(T3 + ta)) - __ldg(T3 - ta);
+  const Rn pb = D0 ? Rn(__ldg(T3 + tb)) - __ldg(T3 - tb) : Rn(0.0);
+#pragma unroll
+  for (int row = 0; row < 3; ++row) {
+    fx[1 + row] = fx[1 + row] + mad(M[10 + row], p, Rn(M[23 + row]) * pa);
+    if (D0) fx[1 + row] = mad(M[36 + row], pb, fx[1 + row]);
+  }
+}
+
+template <int MB>
+__global__ void __launch_bounds__(128, MB) o4FaceFinalKernel(const Ctx* __restrict__ tab, const RegArgs rg, const WorkChunk* __restrict__ wk) {
+  const WorkChunk wc = wk[blockIdx.x];
+  const int d = wc.dir;
+  const Ctx& c = tab[wc.box * 3 + d];
   const O4Args& a = c.a;
-  constexpr int d = D;
-  const double coef = -1.0 / a.G.dx[d];
-  forRegion(c.V1, wc, [&](int b, int i, int j, int k) {
-    const View BP = faceView(c, b, F_BPROD);
-    int p[3] = {i, j, k};
-    p[d] += 1;
-    a.mj[(long)b * c.v1r.N + roff(c.v1r, i, j, k)] += coef * (BP(0, p[0], p[1], p[2]) - BP(0, i, j, k));
+  const bool roe = roeNow(a.G);
+  const long NF = c.fr.N;
+  const int2 tr = transverse(c.fr, d);
+  forRegion(c.V0, d == 0 ? WALK_JK : d == 1 ? WALK_K : WALK_J, wc, [&](int i, int j, int k) {
+    double* const base = faceArr(c, 0) + roff(c.fr, i, j, k);
+    const double* M = faceRec(a.G, a.block0, d, j, k);
+    const bool sm = base[F_THF * NF] > 0.5;
+    const double sigma = roe ? 1.0 : base[F_SPD * NF];
+    // first angular transverse direction: j for d = 0, the only one otherwise
+    const int ta = d == 0 ? tr.x : tr.y, tb = tr.y;
+    auto load = [&](int q, Rn& z, Rn& ya, Rn& yb) {
+      const double* Q = base + (F_QD + q) * NF;
+      const Rn pt = __ldg(Q), a1 = __ldg(Q - tr.x), b1 = __ldg(Q + tr.x), a2 = __ldg(Q - tr.y), b2 = __ldg(Q + tr.y);
+      const Rn avg = sm ? mad(mad(-4.0, pt, (a1 + b1) + (a2 + b2)), 1.0 / 24.0, pt) : pt;
+      const Rn q1 = b1 - a1, q2 = b2 - a2;
+      z = -(sigma * avg);
+      ya = 0.0;
+      yb = 0.0;
+      if (q != 5) {  // the normal field has no flux
+        const double* X = base + (F_X + fluxSlot(q)) * NF;
+        z = z + __ldg(X);
+        ya = Rn(__ldg(X + ta)) - __ldg(X - ta);
+        if (d == 0) yb = Rn(__ldg(X + tb)) - __ldg(X - tb);
+      }
+      if (roe) {
+        ya = ya - (d == 0 ? q1 : q2);
+        if (d == 0) yb = yb - q2;
+      }
+    };
+    Rn fx[8];
+    if (d == 0) finalFlux<1>(M, load, base + F_T3 * NF, ta, tb, fx);
+    else finalFlux<0>(M, load, base + F_T3 * NF, ta, tb, fx);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) base[(F_FX + q) * NF] = fx[q];
+    // the caller's flux and the seam register
+    if (a.flux[d]) {
+      const Reg r0 = regOf(c.V0);
+      double* out = a.flux[d] + roff(r0, i, j, k);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) out[q * r0.N] = fx[q];
+    }
+    double* const reg = a.seamReg ? a.seamReg : rg.reg;
+    if (reg && d > 0) {
+      const int f = d == 1 ? j : k;
+      if (f == 0 || f == a.G.na) {
+        const long nrna = (long)a.G.na * a.G.nr;
+        const int side = f == 0 ? 0 : 1, s = d == 1 ? k : j;
+        const double w = a.seamReg ? rg.w * (a.seamCfl / *a.seamInvMax) : rg.wDev ? rg.w * (rg.cfl / *rg.wDev) : rg.w;
+        double* S = reg + (((long)a.block0 * 2 + (d - 1)) * 2 + side) * 8 * nrna + (long)s * a.G.nr + i;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) S[q * nrna] = mad(w, fx[q], S[q * nrna]);
+      }
+    }
   });
 }
 
-// 12. DivBPowell2 with point primitives (src/BoxOp_DivBcleaning.H:80-172).
-__global__ void o4PowellCoefKernel(const Ctx* __restrict__ tab, const RegArgs rg, const WorkChunk* __restrict__ wk) {
+// 9, 12b. Flux divergence of the three directions and the Powell source
+// (DivBPowell2's cell products) into rhs, one pass over the cells.
+__global__ void __launch_bounds__(128) o4CellKernel(const Ctx* __restrict__ tab, const RegArgs rg, const WorkChunk* __restrict__ wk) {
   const WorkChunk wc = wk[blockIdx.x];
   const Ctx& c = tab[wc.box * 3 + 0];
   const O4Args& a = c.a;
-  forRegion(c.V2, wc, [&](int b, int i, int j, int k) {
-    const long NG = c.gr.N, o = roff(c.gr, i, j, k);
-    const double* WP = a.WP + (long)b * 8 * NG;
-    const double* A = cellBasis(a.G, a.block0 + b, j, k);
-    double vel[3], mag[3];
+  const long NF = c.fr.N;
+  forRegion(c.V, WALK_JK, wc, [&](int i, int j, int k) {
+    double* R = a.rhs + roff(c.vr, i, j, k);
+    const long fo = roff(c.fr, i, j, k);
+    Rn kv[8];
 #pragma unroll
-    for (int e = 0; e < 3; ++e) {
-      vel[e] = A[3 * e] * WP[1 * NG + o] + A[3 * e + 1] * WP[2 * NG + o] + A[3 * e + 2] * WP[3 * NG + o];
-      mag[e] = A[3 * e] * WP[5 * NG + o] + A[3 * e + 1] * WP[6 * NG + o] + A[3 * e + 2] * WP[7 * NG + o];
-    }
-    double* K = a.kp + (long)b * 16 * c.v2r.N + roff(c.v2r, i, j, k);
-    const long N = c.v2r.N;
-    K[0] = 0;
-    double e4 = 0;
+    for (int q = 0; q < 8; ++q) kv[q] = R[q * c.vr.N];
 #pragma unroll
-    for (int e = 0; e < 3; ++e) {
-      K[(1 + e) * N] = mag[e] / (4.0 * kPi);
-      K[(5 + e) * N] = vel[e];
-      e4 += vel[e] * mag[e] / (4.0 * kPi);
+    for (int d = 0; d < 3; ++d) {
+      const Rn coef = -a.scale / a.G.dx[d];
+      const int st = stride(c.fr, d);
+      const double* F = a.face[d] + F_FX * NF + fo;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) kv[q] = mad(coef, Rn(__ldg(F + q * NF + st)) - __ldg(F + q * NF), kv[q]);
     }
-    K[4 * N] = e4;
+    if (a.G.powell) {
+      const long o = roff(c.v1r, i, j, k), N = c.v1r.N;
+      const double* MJ = a.mj + o;
+      const Rn m0 = MJ[0];
+      Rn dm[3];
+#pragma unroll
+      for (int t = 0; t < 3; ++t) dm[t] = (Rn(MJ[stride(c.v1r, t)]) - MJ[-stride(c.v1r, t)]) * (1.0 / 48.0);
+#pragma unroll
+      for (int q = 1; q < 8; ++q) {
+        const double* K = a.ka + (q - 1) * N + o;
+        Rn value = m0 * K[0];
+#pragma unroll
+        for (int t = 0; t < 3; ++t) value = mad(dm[t], Rn(__ldg(K + stride(c.v1r, t))) - __ldg(K - stride(c.v1r, t)), value);
+        kv[q] = kv[q] + value;
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) R[q * c.vr.N] = kv[q];
   });
 }
 
+// 10. Powell face flux (DivBPowell1, src/BoxOp_DivBcleaning.H:35-74): <det A>
+// times the fourth-order face average of the normal field with its angular
+// product (<det A> does not vary radially), or the reconstruction's centred
+// field where the face is not smooth.
+__global__ void o4PowellFluxKernel(const Ctx* __restrict__ tab, const RegArgs rg, const WorkChunk* __restrict__ wk) {
+  const WorkChunk wc = wk[blockIdx.x];
+  const int d = wc.dir;
+  const Ctx& c = tab[wc.box * 3 + d];
+  const O4Args& a = c.a;
+  forRegion(regionOf(c, RG_PF), WALK_J, wc, [&](int i, int j, int k) {
+    const long NF = c.fr.N;
+    double* base = faceArr(c, 0) + roff(c.fr, i, j, k);
+    const double* M = faceRec(a.G, a.block0, d, j, k);
+    Rn out;
+    if (base[F_THF * NF] <= 0.5) {
+      out = M[9] * Rn(base[F_BP * NF]);
+    } else {
+      const double* U = a.U + (5 + d) * a.ur.N + roff(a.ur, i, j, k);
+      const int st = stride(a.ur, d);
+      auto bface = [&](const double* u) -> Rn {
+        return mad(7.0 / 12.0, Rn(u[-st]) + u[0], (-1.0 / 12.0) * (Rn(u[-2 * st]) + u[st]));
+      };
+      const int2 tr = transverse(a.ur, d);
+      const int ta = d == 0 ? tr.x : tr.y;
+      out = mad(M[22], bface(U + ta) - bface(U - ta), M[9] * bface(U));
+      if (d == 0) out = mad(M[35], bface(U + tr.y) - bface(U - tr.y), out);
+    }
+    base[F_BF * NF] = 2.0 * out;
+  });
+}
+
+// 11. -J div B on V1: radial-area products of the Powell face fluxes and
+// their divergence, the three directions at once.
+__global__ void o4PowellDivKernel(const Ctx* __restrict__ tab, const RegArgs rg, const WorkChunk* __restrict__ wk) {
+  const WorkChunk wc = wk[blockIdx.x];
+  const Ctx& c = tab[wc.box * 3 + 0];
+  const O4Args& a = c.a;
+  forRegion(c.V1, WALK_JK, wc, [&](int i, int j, int k) {
+    const long fo = roff(c.fr, i, j, k);
+    const double* B0 = a.face[0] + F_BF * c.fr.N + fo;
+    Rn mj = (-1.0 / a.G.dx[0]) * mad(B0[1], adjDr(a.G, 0, i + 1), -(Rn(B0[0]) * adjDr(a.G, 0, i)));
+    const Rn s = adjDr(a.G, 1, i), ds = (Rn(adjDr(a.G, 1, i + 1)) - adjDr(a.G, 1, i - 1)) * (1.0 / 48.0);
+#pragma unroll
+    for (int d = 1; d < 3; ++d) {
+      const double* B = a.face[d] + F_BF * c.fr.N + fo;
+      const int st = stride(c.fr, d);
+      const Rn flux = s * (Rn(B[st]) - B[0]), slope = (Rn(B[st + 1]) - B[1]) - (Rn(B[st - 1]) - B[-1]);
+      mj = mad(-1.0 / a.G.dx[d], mad(ds, slope, flux), mj);
+    }
+    a.mj[roff(c.v1r, i, j, k)] = mj;
+  });
+}
+
+// 12a. Averages of DivBPowell2's cell coefficients (src/BoxOp_DivBcleaning.H:
+// 80-172) on V1: K = (0, B, v . B, v) / (4 pi, 4 pi, 1) of the point
+// primitives in the cell basis, <K> = K + lap K / 24, formed from the seven
+// cells' primitives (the density coefficient is zero and has no array).
 __global__ void o4PowellAvgKernel(const Ctx* __restrict__ tab, const RegArgs rg, const WorkChunk* __restrict__ wk) {
   const WorkChunk wc = wk[blockIdx.x];
   const Ctx& c = tab[wc.box * 3 + 0];
   const O4Args& a = c.a;
-  forRegion(c.V1, wc, [&](int b, int i, int j, int k) {
-    const View KP{a.kp + (long)b * 16 * c.v2r.N, c.v2r};
-    double* KA = a.kp + (long)b * 16 * c.v2r.N + 8 * c.v2r.N + roff(c.v2r, i, j, k);
-    // all loads before the first store (KA and KP share one array)
-    double out[8];
+  forRegion(c.V1, WALK_JK, wc, [&](int i, int j, int k) {
+    const long NG = c.gr.N;
+    const double* W = a.WP + roff(c.gr, i, j, k);
+    Rn sum[7], mid[7];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) out[q] = KP(q, i, j, k) + lapCell(KP, q, i, j, k) * (1.0 / 24.0);
+    for (int n = 0; n < 7; ++n) {
+      // the cell itself, then its neighbours in i, j, k
+      const int t = (n - 1) / 2, sgn = (n & 1) ? 1 : -1;
+      const double* w = n == 0 ? W : W + sgn * stride(c.gr, t);
+      const double* A = cellBasis(a.G, a.block0, n > 0 && t == 1 ? j + sgn : j, n > 0 && t == 2 ? k + sgn : k);
+      Rn K[7], vb = 0.0;
 #pragma unroll
-    for (int q = 0; q < 8; ++q) KA[q * c.v2r.N] = out[q];
-  });
-}
-
-__global__ void o4PowellApplyKernel(const Ctx* __restrict__ tab, const RegArgs rg, const WorkChunk* __restrict__ wk) {
-  const WorkChunk wc = wk[blockIdx.x];
-  const Ctx& c = tab[wc.box * 3 + 0];
-  const O4Args& a = c.a;
-  forRegion(c.V, wc, [&](int b, int i, int j, int k) {
-    const View KA{a.kp + (long)b * 16 * c.v2r.N + 8 * c.v2r.N, c.v2r};
-    const View MJ{a.mj + (long)b * c.v1r.N, c.v1r};
-    double* R = a.rhs + b * a.rhsStride + roff(c.vr, i, j, k);
-    // all loads (including the accumulated rhs) before the first store
-    double dmj[3];
+      for (int e = 0; e < 3; ++e) {
+        K[4 + e] = dot3(A[3 * e], w[NG], A[3 * e + 1], w[2 * NG], A[3 * e + 2], w[3 * NG]);
+        K[e] = kInv4Pi * dot3(A[3 * e], w[5 * NG], A[3 * e + 1], w[6 * NG], A[3 * e + 2], w[7 * NG]);
+        vb = mad(K[4 + e], K[e], vb);
+      }
+      K[3] = vb;
 #pragma unroll
-    for (int t = 0; t < 3; ++t) dmj[t] = cdiff(MJ, 0, t, i, j, k);
-    const double mj0 = MJ(0, i, j, k);
-    double add[8], rv[8];
-#pragma unroll
-    for (int q = 1; q < 8; ++q) {
-      double value = 0.0;
-#pragma unroll
-      for (int t = 0; t < 3; ++t) value += dmj[t] * cdiff(KA, q, t, i, j, k) * (1.0 / 12.0);
-      value += mj0 * KA(q, i, j, k) * 1.0;
-      add[q] = value;
-      rv[q] = R[q * c.vr.N];
+      for (int q = 0; q < 7; ++q) {
+        if (n == 0) mid[q] = K[q];
+        else sum[q] = n == 1 ? K[q] : sum[q] + K[q];
+      }
     }
+    double* KA = a.ka + roff(c.v1r, i, j, k);
 #pragma unroll
-    for (int q = 1; q < 8; ++q) R[q * c.vr.N] = rv[q] + add[q];
+    for (int q = 0; q < 7; ++q) KA[q * c.v1r.N] = mad(mad(-6.0, mid[q], sum[q]), 1.0 / 24.0, mid[q]);
   });
 }
 
@@ -841,29 +1043,26 @@ __global__ void o4GravityKernel(const Ctx* __restrict__ tab, const RegArgs rg, c
   const Ctx& c = tab[wc.box * 3 + 0];
   const O4Args& a = c.a;
   const double minusGM = -kGrav * kMsun;
-  forRegion(c.V, wc, [&](int b, int i, int j, int k) {
-    const View U{a.U + b * a.uStride, a.ur};
-    const int blk = a.block0 + b;
+  forRegion(c.V, WALK_JK, wc, [&](int i, int j, int k) {
+    const View U{a.U, a.ur};
+    const int blk = a.block0;
     const double dr0 = radialRow(a.G, i).z;
     const double da = 0.5 * radialRow(a.G, i + 1).z - 0.5 * radialRow(a.G, i - 1).z;
     const int pj[5] = {j, j + 1, j - 1, j, j}, pk[5] = {k, k, k, k + 1, k - 1};
     double rd[5], re[5];
-    const double* M[5];
+    const double* M = faceRec(a.G, blk, 0, j, k);
 #pragma unroll
     for (int q = 0; q < 5; ++q) {
       const double d0 = 0.5 * U(0, i + 1, pj[q], pk[q]) - 0.5 * U(0, i - 1, pj[q], pk[q]);
       const double d1 = 0.5 * U(1, i + 1, pj[q], pk[q]) - 0.5 * U(1, i - 1, pj[q], pk[q]);
       rd[q] = dr0 * U(0, i, pj[q], pk[q]) + da * d0 * (1.0 / 12.0);
       re[q] = dr0 * U(1, i, pj[q], pk[q]) + da * d1 * (1.0 / 12.0);
-      M[q] = faceRec(a.G, blk, 0, pj[q], pk[q]);
     }
+    // the record holds half the averages and their angular differences / 48
     auto faceP = [&](int e, const double* v) {
-      double value = M[0][e] * v[0];
-      value += (0.5 * M[1][e] - 0.5 * M[2][e]) * (0.5 * v[1] - 0.5 * v[2]) * (1.0 / 12.0);
-      value += (0.5 * M[3][e] - 0.5 * M[4][e]) * (0.5 * v[3] - 0.5 * v[4]) * (1.0 / 12.0);
-      return value;
+      return 2.0 * (M[e] * v[0] + M[13 + e] * (v[1] - v[2]) + M[26 + e] * (v[3] - v[4]));
     };
-    double* R = a.rhs + b * a.rhsStride + roff(c.vr, i, j, k);
+    double* R = a.rhs + roff(c.vr, i, j, k);
 #pragma unroll
     for (int d = 0; d < 3; ++d) R[(1 + d) * c.vr.N] += faceP(3 * d, rd) * minusGM;
     R[4 * c.vr.N] += faceP(9, re) * minusGM;
@@ -871,881 +1070,25 @@ __global__ void o4GravityKernel(const Ctx* __restrict__ tab, const RegArgs rg, c
 }
 
 
-// ---- fused face chain ----------------------------------------------------------
-// One CTA (128 threads) takes a tile of the final faces of direction d and
-// runs the whole chain after the reconstruction and the Roe point
-// dissipation on it: the theta-aware point-to-average of the flux sum and of
-// the total pressure (5), the mapped flux with its transverse products (6),
-// the radial-area products (7), the pressure force, the dissipation average
-// and the final flux (8), and the flux divergence into rhs (9).  The
-// intermediates (averaged fluxes, mapped fluxes, radial products) live in
-// shared memory; only the reconstruction's face arrays (FS, PS, thF, QD and,
-// for the Rusanov speed, WL and WR) are read from the face scratch, and the
-// only global writes are rhs, the caller's flux and the seam register.
-//
-// d = 1, 2: the threads cover TI radial x TT angular (t) faces; the CTA
-// walks the normal direction over a segment of cells [c0, c1], one face
-// slab after another, and keeps each face's flux in registers for the
-// divergence of the next cell.  d = 0: the threads cover TI radial cells
-// (TI + 1 faces) x TT rows of j and walk k over [c0, c1], the averages of
-// rows k - 1, k, k + 1 held in a ring of three shared slabs.
-//
-// Every product and sum is formed as in the separate steps of the chain
-// (same operands, same order), so the results do not depend on the tiling.
-struct ChainTile {
-  int box;
-  int i0, a0;  // first radial index; first angular index across the tile (t for d != 0, j for d = 0)
-  int c0, c1;  // walk range of cells (d != 0: along d; d = 0: along k)
-};
-
-template <int D>
-__device__ __forceinline__ void chainPt(int i, int n, int t, int p[3]) {
-  // d != 0: (radial i, normal n, angular t) -> (i, j, k)
-  p[0] = i;
-  p[1] = D == 1 ? n : t;
-  p[2] = D == 1 ? t : n;
-}
-
-// Final flux of one face from its mapped-and-radial flux fs (pressure force
-// added here), the dissipation inputs and the metrics (the final flux of
-// the reference's face pass).  dT3[q]: centred difference of the radial
-// pressure product along transverse q (unused where the separable metrics
-// skip it).
-// The point Roe dissipations a final face averages: component stride and
-// the offsets of the face and its four transverse neighbours (lower and
-// upper along t1, then along t2), in the face scratch or in a shared tile.
-struct QdTaps {
-  const double* p;
-  long stride;
-  long o[5];
-};
-
-__device__ __forceinline__ QdTaps scratchTaps(const Ctx& c, int d, int i, int j, int k) {
-  const View QD = faceView(c, 0, F_QD);
-  const int t1 = d == 0 ? 1 : 0, t2 = d == 2 ? 1 : 2;
-  int m1[3] = {i, j, k}, p1[3] = {i, j, k}, m2[3] = {i, j, k}, p2[3] = {i, j, k};
-  m1[t1] -= 1; p1[t1] += 1; m2[t2] -= 1; p2[t2] += 1;
-  return QdTaps{QD.p, QD.r.N,
-                {roff(QD.r, i, j, k), roff(QD.r, m1[0], m1[1], m1[2]), roff(QD.r, p1[0], p1[1], p1[2]),
-                 roff(QD.r, m2[0], m2[1], m2[2]), roff(QD.r, p2[0], p2[1], p2[2])}};
-}
-
-template <int D>
-__device__ __forceinline__ void chainFinal(const Ctx& c, int i, int j, int k, double fs[8], const double t3,
-                                           const double dT3[2], const QdTaps& tap, double fx[8]) {
-  const O4Args& a = c.a;
-  constexpr int d = D;
-  const int t1 = d == 0 ? 1 : 0, t2 = d == 2 ? 1 : 2;
-  const int tr[2] = {t1, t2};
-  const int blk = a.block0;
-  const long NF = c.fr.N, fo = roff(c.fr, i, j, k);
-  const double* base = a.face;
-  const double* M = faceRec(a.G, blk, d, j, k);
-#pragma unroll
-  for (int row = 0; row < 3; ++row) {
-    double value = 0.0;
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int t = tr[q];
-      if (d != 0 && t == 0) continue;
-      int pa[3] = {i, j, k}, pb[3] = {i, j, k};
-      pa[t] += 1; pb[t] -= 1;
-      const double dn = 0.5 * faceRec(a.G, blk, d, pa[1], pa[2])[10 + row] - 0.5 * faceRec(a.G, blk, d, pb[1], pb[2])[10 + row];
-      value += dn * dT3[q] * (1.0 / 12.0);
-    }
-    value += M[10 + row] * t3 * 1.0;
-    fs[1 + row] += value;
-  }
-  const bool sm = base[F_THF * NF + fo] > 0.5;
-  const View QD = faceView(c, 0, F_QD);
-  double diss[8];
-  if (roeNow(a.G)) {
-    double dM[2][10];
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int t = tr[q];
-      int pa[3] = {i, j, k}, pb[3] = {i, j, k};
-      pa[t] += 1; pb[t] -= 1;
-      const double* Ma = faceRec(a.G, blk, d, pa[1], pa[2]);
-      const double* Mb = faceRec(a.G, blk, d, pb[1], pb[2]);
-#pragma unroll
-      for (int e = 0; e < 10; ++e) dM[q][e] = 0.5 * Ma[e] - 0.5 * Mb[e];
-    }
-    double avg[8], dP0[8], dP1[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const double* Q = tap.p + q * tap.stride;
-      const double pt = Q[tap.o[0]], a1 = Q[tap.o[1]], b1 = Q[tap.o[2]], a2 = Q[tap.o[3]], b2 = Q[tap.o[4]];
-      const double lap = (a1 + b1) + (a2 + b2) - 4.0 * pt;
-      avg[q] = sm ? pt + lap * (1.0 / 24.0) : pt;
-      dP0[q] = 0.5 * b1 - 0.5 * a1;
-      dP1[q] = 0.5 * b2 - 0.5 * a2;
-    }
-    diss[0] = faceProd(M[9], avg[0], dM[0][9], dP0[0], dM[1][9], dP1[0]);
-    diss[4] = faceProd(M[9], avg[4], dM[0][9], dP0[4], dM[1][9], dP1[4]);
-#pragma unroll
-    for (int bb = 0; bb < 2; ++bb) {
-      const int bs = bb == 0 ? 1 : 5;
-#pragma unroll
-      for (int row = 0; row < 3; ++row) {
-        double sum = 0.0;
-#pragma unroll
-        for (int col = 0; col < 3; ++col)
-          sum += faceProd(M[3 * row + col], avg[bs + col], dM[0][3 * row + col], dP0[bs + col], dM[1][3 * row + col],
-                          dP1[bs + col]);
-        diss[bs + row] = sum;
-      }
-    }
-  } else {
-    double qv[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const double pt = QD(q, i, j, k);
-      qv[q] = sm ? pt + lapFace(QD, q, d, i, j, k) * (1.0 / 24.0) : pt;
-    }
-#pragma unroll
-    for (int bb = 0; bb < 2; ++bb) {
-      const int bs = bb == 0 ? 1 : 5;
-#pragma unroll
-      for (int row = 0; row < 3; ++row)
-        diss[bs + row] = M[3 * row] * qv[bs] * 1.0 + M[3 * row + 1] * qv[bs + 1] * 1.0 + M[3 * row + 2] * qv[bs + 2] * 1.0;
-    }
-    diss[0] = M[9] * qv[0];
-    diss[4] = M[9] * qv[4];
-    // face wave-speed bound (:1665-1720)
-    double l[8], r[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) { l[q] = base[(F_WL + q) * NF + fo]; r[q] = base[(F_WR + q) * NF + fo]; }
-    const double* A = faceBasis<D>(c, 0, j, k);
-    double rho = 0.5 * (l[0] + r[0]);
-    const double w_d = 0.5 * (l[1 + d] + r[1 + d]);
-    const double bs3[3] = {0.5 * (l[5] + r[5]), 0.5 * (l[6] + r[6]), 0.5 * (l[7] + r[7])};
-    double p = 0.5 * (l[4] + r[4]);
-    if (p < 0.0) p = 0.0;
-    rho = dmax(rho, kRHO00);
-    double Bn = 0.0, Bm = 0.0;
-#pragma unroll
-    for (int e0 = 0; e0 < 3; ++e0) {
-      const double bC = A[3 * e0] * bs3[0] + A[3 * e0 + 1] * bs3[1] + A[3 * e0 + 2] * bs3[2];
-      Bn += A[3 * e0] * bC;
-      Bm += bC * bC;
-    }
-    Bm = sqrt(Bm);
-    const double g = a.G.gamma;
-    const double ce = sqrt(g * p / rho);
-    const double aa = ce * ce + Bm * Bm / (4.0 * kPi * rho);
-    const double bb2 = fabs(Bn) * ce / sqrt(kPi * rho);
-    const double af = 0.5 * (sqrt(dmax(0.0, aa + bb2)) + sqrt(dmax(0.0, aa - bb2)));
-    const double Am = sqrt(A[d] * A[d] + A[3 + d] * A[3 + d] + A[6 + d] * A[6 + d]);
-    const double speed = fabs(w_d) + af * Am;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) diss[q] *= speed;
-  }
-#pragma unroll
-  for (int q = 0; q < 8; ++q) fx[q] = 0.5 * (fs[q] - diss[q]);
-}
-
-// The caller's flux and the seam register of one final face.
-template <int D>
-__device__ __forceinline__ void chainStore(const Ctx& c, const RegArgs& rg, int i, int j, int k, const double fx[8]) {
-  const O4Args& a = c.a;
-  constexpr int d = D;
-  if (a.flux[d]) {
-    const Reg r0 = regOf(c.V0);
-    double* fo2 = a.flux[d] + roff(r0, i, j, k);
-#pragma unroll
-    for (int q = 0; q < 8; ++q) fo2[q * r0.N] = fx[q];
-  }
-  double* const reg = a.seamReg ? a.seamReg : rg.reg;
-  if (reg && d > 0) {
-    const int f = d == 1 ? j : k;
-    if (f == 0 || f == a.G.na) {
-      const long nrna = (long)a.G.na * a.G.nr;
-      const int side = f == 0 ? 0 : 1, s = d == 1 ? k : j;
-      const double w = a.seamReg ? rg.w * (a.seamCfl / *a.seamInvMax) : rg.wDev ? rg.w * (rg.cfl / *rg.wDev) : rg.w;
-      double* R = reg + (((long)a.block0 * 2 + (d - 1)) * 2 + side) * 8 * nrna + (long)s * a.G.nr + i;
-#pragma unroll
-      for (int q = 0; q < 8; ++q) R[q * nrna] += w * fx[q];
-    }
-  }
-}
-
-// Point-to-average of the flux sum and total pressure at one face (5).
-__device__ __forceinline__ void chainAverage(const Ctx& c, int d, int i, int j, int k, double fa[8], double& pa) {
-  const long NF = c.fr.N, fo = roff(c.fr, i, j, k);
-  const double* base = c.a.face;
-  const bool sm = base[F_THF * NF + fo] > 0.5;
-  const View FS = faceView(c, 0, F_FS);
-  const View PS = faceView(c, 0, F_PS);
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const double pt = FS(q, i, j, k);
-    fa[q] = sm ? pt + lapFace(FS, q, d, i, j, k) * (1.0 / 24.0) : pt;
-  }
-  const double pp = PS(0, i, j, k);
-  pa = sm ? pp + lapFace(PS, 0, d, i, j, k) * (1.0 / 24.0) : pp;
-}
-
-// Directions 1, 2: walk the normal direction.  With TMA, the slab's flux
-// sums, flags and total pressures (tile plus a two-face ring) and its point
-// Roe dissipations (tile plus a one-face ring) are copied into shared
-// memory by the tensor-memory accelerator, the next slab's copies issued as
-// soon as the current slab's are consumed, so they overlap the mapped-flux
-// and final-flux stages; without it (tensor maps unavailable) the same
-// stages read the face scratch through L1.
-// TMA tensor maps per box: directions 1 and 2 (8 arrays, 2 arrays each),
-// then direction 0 (averages: 9 arrays; dissipations: 8).
-constexpr int kChainMaps = 6;
-
-template <int TI>
-struct ChainShape {
-  static constexpr int TT = 128 / TI, NI = TI + 2, NT = TT + 2;  // averages: tile plus a one-face ring
-  static constexpr int NTH = NI * TT;  // threads: one per mapped-flux point (the tile's faces and a radial ring)
-  static constexpr int NX = TI + 4, NY = TT + 4, NXY = NX * NY;  // TMA tiles: tile plus a two-face ring
-  static constexpr int round16(int n) { return (n + 15) / 16 * 16; }
-  static constexpr int oFA = 0, oPA = oFA + round16(8 * NI * NT), oFM = oPA + round16(NI * NT),
-                       oT3 = oFM + round16(8 * NI * TT), oIn = oT3 + round16(TI * NT),
-                       oQD = oIn + round16(10 * NXY), oBar = oQD + round16(8 * NXY);
-  static constexpr int doubles(bool tma) { return tma ? oBar + 2 : oIn; }
-};
-
-__device__ __forceinline__ unsigned smemAddr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbarInit(unsigned long long* bar) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smemAddr(bar)) : "memory");
-}
-
-__device__ __forceinline__ void mbarExpect(unsigned long long* bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smemAddr(bar)), "r"(bytes) : "memory");
-}
-
-// Bounded wait for phase `parity` of an mbarrier: false when it has not
-// completed after kMbarPolls polls (each poll blocks for a short,
-// implementation-defined time), so a copy that never lands cannot hang the
-// GPU.
-constexpr int kMbarPolls = 1 << 22;
-__device__ __forceinline__ bool mbarWait(unsigned long long* bar, unsigned parity) {
-  const unsigned addr = smemAddr(bar);
-  for (int it = 0; it < kMbarPolls; ++it) {
-    unsigned done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(addr), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-
-// One tiled TMA copy of a 4-D box (radial, j, k, array) of the face scratch
-// into shared memory, completing on `bar`.
-__device__ __forceinline__ void tmaLoad(double* dst, const CUtensorMap* map, int x, int y, int z, int w,
-                                        unsigned long long* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
-      "[%6];" ::"r"(smemAddr(dst)),
-      "l"(map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(smemAddr(bar))
-      : "memory");
-}
-
-template <int D, int TI, int MB, bool TMA>
-__global__ void __launch_bounds__(ChainShape<TI>::NTH, MB) o4FaceChainKernel(const Ctx* __restrict__ tab,
-                                                                            const RegArgs rg,
-                                                             const ChainTile* __restrict__ tiles,
-                                                             const CUtensorMap* __restrict__ maps) {
-  static_assert(D == 1 || D == 2, "angular directions");
-  using S = ChainShape<TI>;
-  constexpr int TT = S::TT, NI = S::NI, NT = S::NT, NX = S::NX, NXY = S::NXY;
-  constexpr int tdim = D == 1 ? 2 : 1;
-  extern __shared__ __align__(128) double smem[];
-  double* sFA = smem + S::oFA;  // [8][NI * NT]
-  double* sPA = smem + S::oPA;  // [NI * NT]
-  double* sFM = smem + S::oFM;  // [8][NI * TT]
-  double* sT3 = smem + S::oT3;  // [TI * NT]
-  double* sIn = smem + S::oIn;  // TMA: [FS 8, thF, PS][NY][NX]
-  double* sQD = smem + S::oQD;  // TMA: [8][NY][NX]
-  unsigned long long* bar = reinterpret_cast<unsigned long long*>(smem + S::oBar);
-  const ChainTile tl = tiles[blockIdx.x];
-  const Ctx& c = tab[tl.box * 3 + D];
-  const O4Args& a = c.a;
-  constexpr int NTH = S::NTH;
-  const int tid = threadIdx.x, li = tid % TI, lt = tid / TI;
-  const int i = tl.i0 + li, t = tl.a0 + lt;
-  // threads beyond the tile's TI x TT faces only help with the shared stages
-  const bool mine = tid < TI * TT && i <= c.V.hi[0] && t <= c.V.hi[tdim];
-  // radial products: area at i and its centred difference
-  const double s = adjDr(a.G, D, i), ds = 0.5 * adjDr(a.G, D, i + 1) - 0.5 * adjDr(a.G, D, i - 1);
-  const double coef = -a.scale / a.G.dx[D];
-  const int ilo = c.V.lo[0] - 1, ihi = c.V.hi[0] + 1, tlo = c.V.lo[tdim] - 1, thi = c.V.hi[tdim] + 1;
-  double fxPrev[8];
-#pragma unroll
-  for (int q = 0; q < 8; ++q) fxPrev[q] = 0.0;
-  const int nEnd = tl.c1 + 1;
-  const bool lastSegment = tl.c1 == c.V.hi[D];
-  // TMA tiles: radial from i0 - 2 (an even offset from the face box's low
-  // corner: tiles start at the valid box's low radial index and TI is even),
-  // angular from a0 - 2, one face slab; map 0 copies 8 arrays, map 1 two
-  const CUtensorMap* map8 = TMA ? maps + (long)tl.box * kChainMaps + (D - 1) * 2 : nullptr;
-  const CUtensorMap* map2 = TMA ? map8 + 1 : nullptr;
-  const int tx = tl.i0 - 2 - c.fr.lo[0], ta = tl.a0 - 2 - c.fr.lo[tdim], tnLo = c.fr.lo[D];
-  auto issue = [&](int n, bool inputs) {
-    const int y = D == 1 ? n - tnLo : ta, z = D == 1 ? ta : n - tnLo;
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    if (inputs) {
-      mbarExpect(&bar[0], 10u * NXY * sizeof(double));
-      tmaLoad(sIn, map8, tx, y, z, F_FS, &bar[0]);
-      tmaLoad(sIn + 8 * NXY, map2, tx, y, z, F_THF, &bar[0]);
-    } else {
-      mbarExpect(&bar[1], 8u * NXY * sizeof(double));
-      tmaLoad(sQD, map8, tx, y, z, F_QD, &bar[1]);
-    }
-  };
-  bool failed = false;
-  if (TMA) {
-    if (tid == 0) {
-      mbarInit(&bar[0]);
-      mbarInit(&bar[1]);
-      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-    if (tid == 0) {
-      issue(tl.c0, true);
-      issue(tl.c0, false);
-    }
-  }
-  for (int n = tl.c0; n <= nEnd && !failed; ++n) {
-    const unsigned parity = (unsigned)(n - tl.c0) & 1u;
-    if (TMA) {
-      failed = __syncthreads_or(!mbarWait(&bar[0], parity));
-      if (failed) break;
-    }
-    // (5) averages on radial i0-1 .. i0+TI x angular a0-1 .. a0+TT of face slab n
-    for (int q = tid; q < NI * NT; q += NTH) {
-      const int ii = tl.i0 - 1 + q % NI, tt = tl.a0 - 1 + q / NI;
-      if (ii < ilo || ii > ihi || tt < tlo || tt > thi) continue;
-      double fa[8], pa;
-      if (TMA) {
-        // (ii, tt) in the TMA tile; lapFace's order: radial pair, angular pair
-        const int x = q % NI + 1, y = q / NI + 1, o = y * NX + x;
-        const bool sm = sIn[8 * NXY + o] > 0.5;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const double* F = sIn + e * NXY;
-          const double pt = F[o];
-          fa[e] = sm ? pt + ((F[o - 1] + F[o + 1]) + (F[o - NX] + F[o + NX]) - 4.0 * pt) * (1.0 / 24.0) : pt;
-        }
-        const double* P = sIn + 9 * NXY;
-        const double pp = P[o];
-        pa = sm ? pp + ((P[o - 1] + P[o + 1]) + (P[o - NX] + P[o + NX]) - 4.0 * pp) * (1.0 / 24.0) : pp;
-      } else {
-        int p[3];
-        chainPt<D>(ii, n, tt, p);
-        chainAverage(c, D, p[0], p[1], p[2], fa, pa);
-      }
-#pragma unroll
-      for (int e = 0; e < 8; ++e) sFA[e * NI * NT + q] = fa[e];
-      sPA[q] = pa;
-    }
-    __syncthreads();
-    if (TMA && tid == 0 && n < nEnd) issue(n + 1, true);  // the inputs' tile is free again
-    // (6) mapped flux on radial i0-1 .. i0+TI x angular a0 .. a0+TT-1; the
-    // radial transverse derivative of the angular metrics vanishes (skipped)
-    for (int q = tid; q < NI * TT; q += NTH) {
-      const int ii = tl.i0 - 1 + q % NI, tt = tl.a0 + q / NI;
-      if (ii < ilo || ii > ihi || tt > c.V.hi[tdim]) continue;
-      int p[3];
-      chainPt<D>(ii, n, tt, p);
-      const double* M = faceRec(a.G, a.block0, D, p[1], p[2]);
-      int pa[3] = {p[0], p[1], p[2]}, pb[3] = {p[0], p[1], p[2]};
-      pa[tdim] += 1; pb[tdim] -= 1;
-      const double* Ma = faceRec(a.G, a.block0, D, pa[1], pa[2]);
-      const double* Mb = faceRec(a.G, a.block0, D, pb[1], pb[2]);
-      double dM[10];
-#pragma unroll
-      for (int e = 0; e < 10; ++e) dM[e] = 0.5 * Ma[e] - 0.5 * Mb[e];
-      const int qc = q + NI;  // (ii, tt) in the averages' frame (rows from a0 - 1)
-      const int qu = qc + NI, qd = qc - NI;
-      double fa[8], dF[8];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        fa[e] = sFA[e * NI * NT + qc];
-        dF[e] = 0.5 * sFA[e * NI * NT + qu] - 0.5 * sFA[e * NI * NT + qd];
-      }
-      double out[8];
-#pragma unroll
-      for (int qq = 0; qq < 2; ++qq) {
-        const int e = qq == 0 ? 0 : 4;
-        double term = 0.0;
-        term += dM[9] * dF[e] * (1.0 / 12.0);
-        term += M[9] * fa[e] * 1.0;
-        out[e] = 0.0 + term;
-      }
-#pragma unroll
-      for (int bb = 0; bb < 2; ++bb) {
-        const int bs = bb == 0 ? 1 : 5;
-#pragma unroll
-        for (int row = 0; row < 3; ++row) {
-          double sum = 0.0;
-#pragma unroll
-          for (int col = 0; col < 3; ++col) {
-            double term = 0.0;
-            term += dM[3 * row + col] * dF[bs + col] * (1.0 / 12.0);
-            term += M[3 * row + col] * fa[bs + col] * 1.0;
-            sum += term;
-          }
-          out[bs + row] = sum;
-        }
-      }
-#pragma unroll
-      for (int e = 0; e < 8; ++e) sFM[e * NI * TT + q] = out[e];
-    }
-    // (7) radial product of <p_tot> on radial i0 .. i0+TI-1 x angular a0-1 .. a0+TT
-    for (int q = tid; q < TI * NT; q += NTH) {
-      const int ii = tl.i0 + q % TI, tt = tl.a0 - 1 + q / TI;
-      if (ii > c.V.hi[0] || tt < tlo || tt > thi) continue;
-      const double si = adjDr(a.G, D, ii), dsi = 0.5 * adjDr(a.G, D, ii + 1) - 0.5 * adjDr(a.G, D, ii - 1);
-      const int qc = (q / TI) * NI + (q % TI) + 1;  // (ii, tt) in the averages' frame
-      double value = 0.0;
-      value += (0.5 * sPA[qc + 1] - 0.5 * sPA[qc - 1]) * dsi * (1.0 / 12.0);
-      value += sPA[qc] * si * 1.0;
-      sT3[q] = value;
-    }
-    if (TMA) {
-      failed = __syncthreads_or(!mbarWait(&bar[1], parity));
-      if (failed) break;
-    } else {
-      __syncthreads();
-    }
-    // (7, 8, 9) this thread's face: radial product of the mapped flux, final
-    // flux, divergence of the cell below it
-    if (mine) {
-      int p[3];
-      chainPt<D>(i, n, t, p);
-      const int qm = lt * NI + li + 1;  // (i, t) in the mapped-flux frame
-      double fs[8];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        double value = 0.0;
-        value += (0.5 * sFM[e * NI * TT + qm + 1] - 0.5 * sFM[e * NI * TT + qm - 1]) * ds * (1.0 / 12.0);
-        value += sFM[e * NI * TT + qm] * s * 1.0;
-        fs[e] = value;
-      }
-      const int q3 = (lt + 1) * TI + li;  // (i, t) in the pressure-product frame
-      const double dT3[2] = {0.0, 0.5 * sT3[q3 + TI] - 0.5 * sT3[q3 - TI]};
-      QdTaps tap;
-      if (TMA) {
-        const int o = (lt + 2) * NX + (li + 2);  // (i, t) in the TMA tile
-        tap = QdTaps{sQD, NXY, {o, o - 1, o + 1, o - NX, o + NX}};
-      } else {
-        tap = scratchTaps(c, D, p[0], p[1], p[2]);
-      }
-      double fx[8];
-      chainFinal<D>(c, p[0], p[1], p[2], fs, sT3[q3], dT3, tap, fx);
-      if (n <= tl.c1 || lastSegment) chainStore<D>(c, rg, p[0], p[1], p[2], fx);
-      if (n > tl.c0) {
-        int pc[3];
-        chainPt<D>(i, n - 1, t, pc);
-        double* R = a.rhs + roff(c.vr, pc[0], pc[1], pc[2]);
-        double rv[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) rv[e] = R[e * c.vr.N];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) R[e * c.vr.N] = rv[e] + coef * (fx[e] - fxPrev[e]);
-      }
-#pragma unroll
-      for (int e = 0; e < 8; ++e) fxPrev[e] = fx[e];
-    }
-    __syncthreads();
-    if (TMA && tid == 0 && n < nEnd) issue(n + 1, false);  // the dissipations' tile is free again
-  }
-  if (TMA && failed) {
-    // A copy did not land: report it, wait (bounded) for the copies still in
-    // flight, and make this tile's cells visibly invalid.
-    if (tid == 0) {
-      if (a.G.status) atomicExch(a.G.status, 1);
-      mbarWait(&bar[0], 0u);
-      mbarWait(&bar[1], 0u);
-      mbarWait(&bar[0], 1u);
-      mbarWait(&bar[1], 1u);
-    }
-    __syncthreads();
-    if (mine)
-      for (int n = tl.c0; n <= tl.c1; ++n) {
-        int pc[3];
-        chainPt<D>(i, n, t, pc);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) a.rhs[roff(c.vr, pc[0], pc[1], pc[2]) + e * c.vr.N] = CUDART_NAN;
-      }
-  }
-}
-
-// Direction 0: walk k; shared memory (dynamic): averages of three rows of k
-// [3][8][NS], pressure averages [3][NS], final fluxes [8][(TI + 1) TT].
-template <int TI>
-__host__ __device__ constexpr int chain0Doubles() {
-  return 3 * 9 * (TI + 1) * (128 / TI + 2) + 8 * (TI + 1) * (128 / TI);
-}
-
-// Threads of the direction-0 chain: one per final face of a row of the tile.
-template <int TI>
-__host__ __device__ constexpr int chain0Threads() {
-  return (TI + 1) * (128 / TI);
-}
-
-template <int TI, int MB>
-__global__ void __launch_bounds__(chain0Threads<TI>(), MB) o4FaceChain0Kernel(const Ctx* __restrict__ tab,
-                                                                              const RegArgs rg,
-                                                                              const ChainTile* __restrict__ tiles) {
-  constexpr int TT = 128 / TI, NI = TI + 1, NJ = TT + 2, NS = NI * NJ, NTH = chain0Threads<TI>();
-  extern __shared__ __align__(128) double smem[];
-  double* sFA = smem;              // [3][8][NS]
-  double* sPA = sFA + 3 * 8 * NS;  // [3][NS]
-  double* sFX = sPA + 3 * NS;      // [8][NI * TT]
-  const ChainTile tl = tiles[blockIdx.x];
-  const Ctx& c = tab[tl.box * 3 + 0];
-  const O4Args& a = c.a;
-  const int tid = threadIdx.x;
-  const double coef = -a.scale / a.G.dx[0];
-  const int ihi = c.V.hi[0] + 1, jlo = c.V.lo[1] - 1, jhi = c.V.hi[1] + 1;
-  auto slot = [&](int k) { return (k - tl.c0 + 3) % 3; };
-  auto slab = [&](int k) {
-    double* fa = sFA + slot(k) * 8 * NS;
-    double* pa = sPA + slot(k) * NS;
-    for (int q = tid; q < NS; q += NTH) {
-      const int ii = tl.i0 + q % NI, jj = tl.a0 - 1 + q / NI;
-      if (ii > ihi || jj < jlo || jj > jhi) continue;
-      double f[8], pp;
-      chainAverage(c, 0, ii, jj, k, f, pp);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) fa[e * NS + q] = f[e];
-      pa[q] = pp;
-    }
-  };
-  slab(tl.c0 - 1);
-  slab(tl.c0);
-  for (int k = tl.c0; k <= tl.c1; ++k) {
-    slab(k + 1);
-    __syncthreads();
-    const double* F0 = sFA + slot(k) * 8 * NS;
-    const double* Fm = sFA + slot(k - 1) * 8 * NS;
-    const double* Fp = sFA + slot(k + 1) * 8 * NS;
-    const double* P0 = sPA + slot(k) * NS;
-    const double* Pm = sPA + slot(k - 1) * NS;
-    const double* Pp = sPA + slot(k + 1) * NS;
-    // (6, 7, 8) faces i0 .. i0+TI x rows a0 .. a0+TT-1 of row k
-    for (int q = tid; q < NI * TT; q += NTH) {
-      const int ii = tl.i0 + q % NI, jj = tl.a0 + q / NI;
-      if (ii > ihi || jj > c.V.hi[1]) continue;
-      const int qc = q + NI;  // (ii, jj) in the slab frame
-      const double* M = faceRec(a.G, a.block0, 0, jj, k);
-      const double* Mj1 = faceRec(a.G, a.block0, 0, jj + 1, k);
-      const double* Mj0 = faceRec(a.G, a.block0, 0, jj - 1, k);
-      const double* Mk1 = faceRec(a.G, a.block0, 0, jj, k + 1);
-      const double* Mk0 = faceRec(a.G, a.block0, 0, jj, k - 1);
-      double dM0[10], dM1[10];
-#pragma unroll
-      for (int e = 0; e < 10; ++e) {
-        dM0[e] = 0.5 * Mj1[e] - 0.5 * Mj0[e];
-        dM1[e] = 0.5 * Mk1[e] - 0.5 * Mk0[e];
-      }
-      double fa[8], dF0[8], dF1[8];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        fa[e] = F0[e * NS + qc];
-        dF0[e] = 0.5 * F0[e * NS + qc + NI] - 0.5 * F0[e * NS + qc - NI];
-        dF1[e] = 0.5 * Fp[e * NS + qc] - 0.5 * Fm[e * NS + qc];
-      }
-      double fm[8];
-#pragma unroll
-      for (int qq = 0; qq < 2; ++qq) {
-        const int e = qq == 0 ? 0 : 4;
-        double term = 0.0;
-        term += dM0[9] * dF0[e] * (1.0 / 12.0);
-        term += dM1[9] * dF1[e] * (1.0 / 12.0);
-        term += M[9] * fa[e] * 1.0;
-        fm[e] = 0.0 + term;
-      }
-#pragma unroll
-      for (int bb = 0; bb < 2; ++bb) {
-        const int bs = bb == 0 ? 1 : 5;
-#pragma unroll
-        for (int row = 0; row < 3; ++row) {
-          double sum = 0.0;
-#pragma unroll
-          for (int col = 0; col < 3; ++col) {
-            double term = 0.0;
-            term += dM0[3 * row + col] * dF0[bs + col] * (1.0 / 12.0);
-            term += dM1[3 * row + col] * dF1[bs + col] * (1.0 / 12.0);
-            term += M[3 * row + col] * fa[bs + col] * 1.0;
-            sum += term;
-          }
-          fm[bs + row] = sum;
-        }
-      }
-      // radial products (direction 0: no radial correction)
-      const double si = adjDr(a.G, 0, ii);
-      double fs[8];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        double value = 0.0;
-        value += fm[e] * si * 1.0;
-        fs[e] = value;
-      }
-      auto t3 = [&](double pav) {
-        double value = 0.0;
-        value += pav * si * 1.0;
-        return value;
-      };
-      const double dT3[2] = {0.5 * t3(P0[qc + NI]) - 0.5 * t3(P0[qc - NI]), 0.5 * t3(Pp[qc]) - 0.5 * t3(Pm[qc])};
-      double fx[8];
-      chainFinal<0>(c, ii, jj, k, fs, t3(P0[qc]), dT3, scratchTaps(c, 0, ii, jj, k), fx);
-      chainStore<0>(c, rg, ii, jj, k, fx);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) sFX[e * NI * TT + q] = fx[e];
-    }
-    __syncthreads();
-    // (9) divergence of the row's cells
-    {
-      const int li = tid % TI, lj = tid / TI;
-      const int i = tl.i0 + li, j = tl.a0 + lj;
-      if (tid < TI * TT && i <= c.V.hi[0] && j <= c.V.hi[1]) {
-        const int q = lj * NI + li;
-        double* R = a.rhs + roff(c.vr, i, j, k);
-        double rv[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) rv[e] = R[e * c.vr.N];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) R[e * c.vr.N] = rv[e] + coef * (sFX[e * NI * TT + q + 1] - sFX[e * NI * TT + q]);
-      }
-    }
-  }
-}
-
-
-// Direction 0 with TMA, in two kernels.  First the theta-aware averages of
-// the flux sums and total pressures on the final faces plus a one-face ring
-// in j and k (the region of the Roe point dissipation), one thread per face,
-// into the face scratch (F_FA0, F_PA0); it runs beside the Roe point
-// dissipation.
-__global__ void o4FaceAvg0Kernel(const Ctx* __restrict__ tab, const RegArgs rg, const WorkChunk* __restrict__ wk) {
-  const WorkChunk wc = wk[blockIdx.x];
-  const Ctx& c = tab[wc.box * 3 + 0];
-  const Box3 PB = c.V0.growTrans(0, 1);
-  forRegion(PB, wc, [&](int b, int i, int j, int k) {
-    double fa[8], pa;
-    chainAverage(c, 0, i, j, k, fa, pa);
-    double* base = c.a.face + roff(c.fr, i, j, k);
-    const long NF = c.fr.N;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) base[(F_FA0 + e) * NF] = fa[e];
-    base[F_PA0 * NF] = pa;
-  });
-}
-
-// Then the chain itself: TI radial cells (TI + 1 faces) x TT rows of j per
-// CTA, walking k over [c0, c1]; a ring of three k-slabs of the averages
-// (8 + 1 arrays) and one of the point Roe dissipations (8 arrays), each slab
-// TI + 2 radial x TT + 2 rows, copied by TMA, the slab k + 2 issued as soon
-// as slab k - 1 is consumed.  Everything else as o4FaceChain0Kernel.
-template <int TI>
-struct Chain0Shape {
-  static constexpr int TT = 128 / TI, NI = TI + 1, NTH = NI * TT;
-  static constexpr int NX = TI + 2, NY = TT + 2, NXY = NX * NY;  // TMA slab: faces and one row either side
-  static constexpr int SA = 9 * NXY, SQ = 8 * NXY;                  // doubles per averages / dissipation slab
-  static constexpr int round16(int n) { return (n + 15) / 16 * 16; }
-  // slots start on 128-byte boundaries, as a tensor copy's destination must
-  static constexpr int PA = round16(SA), PQ = round16(SQ);
-  static constexpr int oA = 0, oQ = 3 * PA, oFX = oQ + 3 * PQ, oBar = oFX + round16(8 * NTH);
-  static constexpr int doubles() { return oBar + 6; }
-};
-
-template <int TI, int MB>
-__global__ void __launch_bounds__(Chain0Shape<TI>::NTH, MB)
-    o4FaceChain0TmaKernel(const Ctx* __restrict__ tab, const RegArgs rg, const ChainTile* __restrict__ tiles,
-                          const CUtensorMap* __restrict__ maps) {
-  using S = Chain0Shape<TI>;
-  constexpr int TT = S::TT, NI = S::NI, NX = S::NX, NXY = S::NXY, NTH = S::NTH;
-  extern __shared__ __align__(128) double smem[];
-  double* sA = smem + S::oA;    // [3 slots][9][NY][NX]
-  double* sQ = smem + S::oQ;    // [3 slots][8][NY][NX]
-  double* sFX = smem + S::oFX;  // [8][NTH]
-  unsigned long long* bar = reinterpret_cast<unsigned long long*>(smem + S::oBar);  // [A 3][Q 3]
-  const ChainTile tl = tiles[blockIdx.x];
-  const Ctx& c = tab[tl.box * 3 + 0];
-  const O4Args& a = c.a;
-  const int tid = threadIdx.x;
-  const double coef = -a.scale / a.G.dx[0];
-  const int ihi = c.V.hi[0] + 1;
-  const CUtensorMap* mapA = maps + (long)tl.box * kChainMaps + 4;
-  const CUtensorMap* mapQ = mapA + 1;
-  const int tx = tl.i0 - c.fr.lo[0], ty = tl.a0 - 1 - c.fr.lo[1];
-  // slab k lives in slot (k - c0 + 1) % 3 and is that slot's ((k - c0 + 1) / 3)-th copy
-  auto slot = [&](int k) { return (k - tl.c0 + 1) % 3; };
-  auto use = [&](int k) { return (unsigned)((k - tl.c0 + 1) / 3) & 1u; };
-  const int kLast = tl.c1 + 1;
-  auto issue = [&](int k) {
-    const int sl = slot(k);
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    mbarExpect(&bar[sl], (unsigned)S::SA * sizeof(double));
-    tmaLoad(sA + sl * S::PA, mapA, tx, ty, k - c.fr.lo[2], F_FA0, &bar[sl]);
-    mbarExpect(&bar[3 + sl], (unsigned)S::SQ * sizeof(double));
-    tmaLoad(sQ + sl * S::PQ, mapQ, tx, ty, k - c.fr.lo[2], F_QD, &bar[3 + sl]);
-  };
-  if (tid == 0) {
-    for (int q = 0; q < 6; ++q) mbarInit(&bar[q]);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-  if (tid == 0)
-    for (int k = tl.c0 - 1; k <= tl.c0 + 1; ++k) issue(k);
-  bool failed = false;
-  for (int k = tl.c0; k <= tl.c1 && !failed; ++k) {
-    bool ok = true;
-    if (k == tl.c0) ok = mbarWait(&bar[slot(k - 1)], use(k - 1)) && mbarWait(&bar[3 + slot(k - 1)], use(k - 1)) &&
-                        mbarWait(&bar[slot(k)], use(k)) && mbarWait(&bar[3 + slot(k)], use(k));
-    ok = ok && mbarWait(&bar[slot(k + 1)], use(k + 1)) && mbarWait(&bar[3 + slot(k + 1)], use(k + 1));
-    failed = __syncthreads_or(!ok);
-    if (failed) break;
-    const double* F0 = sA + slot(k) * S::PA;
-    const double* Fm = sA + slot(k - 1) * S::PA;
-    const double* Fp = sA + slot(k + 1) * S::PA;
-    // (6, 7, 8) faces i0 .. i0+TI x rows a0 .. a0+TT-1 of row k: one thread each
-    {
-      const int q = tid, ii = tl.i0 + q % NI, jj = tl.a0 + q / NI;
-      if (ii <= ihi && jj <= c.V.hi[1]) {
-        const int o = (q / NI + 1) * NX + q % NI;  // (ii, jj) in a slab
-        const double* M = faceRec(a.G, a.block0, 0, jj, k);
-        const double* Mj1 = faceRec(a.G, a.block0, 0, jj + 1, k);
-        const double* Mj0 = faceRec(a.G, a.block0, 0, jj - 1, k);
-        const double* Mk1 = faceRec(a.G, a.block0, 0, jj, k + 1);
-        const double* Mk0 = faceRec(a.G, a.block0, 0, jj, k - 1);
-        double dM0[10], dM1[10];
-#pragma unroll
-        for (int e = 0; e < 10; ++e) {
-          dM0[e] = 0.5 * Mj1[e] - 0.5 * Mj0[e];
-          dM1[e] = 0.5 * Mk1[e] - 0.5 * Mk0[e];
-        }
-        double fa[8], dF0[8], dF1[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          fa[e] = F0[e * NXY + o];
-          dF0[e] = 0.5 * F0[e * NXY + o + NX] - 0.5 * F0[e * NXY + o - NX];
-          dF1[e] = 0.5 * Fp[e * NXY + o] - 0.5 * Fm[e * NXY + o];
-        }
-        double fm[8];
-#pragma unroll
-        for (int qq = 0; qq < 2; ++qq) {
-          const int e = qq == 0 ? 0 : 4;
-          double term = 0.0;
-          term += dM0[9] * dF0[e] * (1.0 / 12.0);
-          term += dM1[9] * dF1[e] * (1.0 / 12.0);
-          term += M[9] * fa[e] * 1.0;
-          fm[e] = 0.0 + term;
-        }
-#pragma unroll
-        for (int bb = 0; bb < 2; ++bb) {
-          const int bs = bb == 0 ? 1 : 5;
-#pragma unroll
-          for (int row = 0; row < 3; ++row) {
-            double sum = 0.0;
-#pragma unroll
-            for (int col = 0; col < 3; ++col) {
-              double term = 0.0;
-              term += dM0[3 * row + col] * dF0[bs + col] * (1.0 / 12.0);
-              term += dM1[3 * row + col] * dF1[bs + col] * (1.0 / 12.0);
-              term += M[3 * row + col] * fa[bs + col] * 1.0;
-              sum += term;
-            }
-            fm[bs + row] = sum;
-          }
-        }
-        const double si = adjDr(a.G, 0, ii);
-        double fs[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          double value = 0.0;
-          value += fm[e] * si * 1.0;
-          fs[e] = value;
-        }
-        auto t3 = [&](double pav) {
-          double value = 0.0;
-          value += pav * si * 1.0;
-          return value;
-        };
-        const double* P0 = F0 + 8 * NXY;
-        const double dT3[2] = {0.5 * t3(P0[o + NX]) - 0.5 * t3(P0[o - NX]),
-                               0.5 * t3(Fp[8 * NXY + o]) - 0.5 * t3(Fm[8 * NXY + o])};
-        // the five dissipation taps: the face, rows j -+ 1 of slab k, slabs k -+ 1
-        const long so = (long)slot(k) * S::PQ + o;
-        const QdTaps tap{sQ, NXY, {so, so - NX, so + NX, (long)slot(k - 1) * S::PQ + o, (long)slot(k + 1) * S::PQ + o}};
-        double fx[8];
-        chainFinal<0>(c, ii, jj, k, fs, t3(P0[o]), dT3, tap, fx);
-        chainStore<0>(c, rg, ii, jj, k, fx);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) sFX[e * NTH + q] = fx[e];
-      }
-    }
-    __syncthreads();
-    // slab k - 1 is consumed: its slots take slab k + 2
-    if (tid == 0 && k + 2 <= kLast) issue(k + 2);
-    // (9) divergence of the row's cells
-    {
-      const int li = tid % TI, lj = tid / TI;
-      const int i = tl.i0 + li, j = tl.a0 + lj;
-      if (tid < TI * TT && i <= c.V.hi[0] && j <= c.V.hi[1]) {
-        const int q = lj * NI + li;
-        double* R = a.rhs + roff(c.vr, i, j, k);
-        double rv[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) rv[e] = R[e * c.vr.N];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) R[e * c.vr.N] = rv[e] + coef * (sFX[e * NTH + q + 1] - sFX[e * NTH + q]);
-      }
-    }
-    __syncthreads();
-  }
-  if (failed) {
-    // A copy did not land: report it, wait (bounded) for the copies still in
-    // flight, and make this tile's cells visibly invalid.
-    if (tid == 0) {
-      if (a.G.status) atomicExch(a.G.status, 1);
-      for (int q = 0; q < 6; ++q) {
-        mbarWait(&bar[q], 0u);
-        mbarWait(&bar[q], 1u);
-      }
-    }
-    __syncthreads();
-    const int li = tid % TI, lj = tid / TI;
-    const int i = tl.i0 + li, j = tl.a0 + lj;
-    if (tid < TI * TT && i <= c.V.hi[0] && j <= c.V.hi[1])
-      for (int k = tl.c0; k <= tl.c1; ++k)
-#pragma unroll
-        for (int e = 0; e < 8; ++e) a.rhs[roff(c.vr, i, j, k) + e * c.vr.N] = CUDART_NAN;
-  }
-}
-
 }  // namespace
 
 size_t o4CarveScratch(O4Args& a, double* sp) {
   Box3 V;
   for (int q = 0; q < 3; ++q) { V.lo[q] = a.vlo[q]; V.hi[q] = a.vhi[q]; }
   const Box3 G = V.grow(a.ghost);
-  const size_t NG = (size_t)G.size(), NF = (size_t)faceBox(G).size(), N1 = (size_t)V.grow(1).size(),
-               N2 = (size_t)V.grow(2).size(), nb = (size_t)a.nbox;
+  const size_t NG = (size_t)G.size(), NF = (size_t)faceBox(G).size(), N1 = (size_t)V.grow(1).size(), nb = (size_t)a.nbox;
   size_t off = 0;
   auto take = [&](double*& dst, size_t n) {
     if (sp) dst = sp + off;
-    off += (n + 31) / 32 * 32;  // 256-byte boundaries (TMA wants 16)
+    off += (n + 31) / 32 * 32;  // 256-byte boundaries
   };
   take(a.WA, nb * 8 * NG);
   take(a.WP, nb * 8 * NG);
   take(a.th, nb * NG);
   take(a.thr, nb * NG);
-  take(a.face, nb * kO4FaceArrays * NF);
-  take(a.face2, nb * kO4FaceArrays * NF);
+  for (int d = 0; d < 3; ++d) take(a.face[d], nb * kO4FaceArrays * NF);
   take(a.mj, nb * N1);
-  take(a.kp, nb * 16 * N2);
+  take(a.ka, nb * 7 * N1);
   return off;
 }
 
@@ -1758,177 +1101,28 @@ size_t o4ScratchDoubles(int nbox, const int vlo[3], const int vhi[3], int ghost)
 }
 
 // A batch: per box and direction the Ctx of a one-box O4Args, in device
-// memory (the kernels' argument) and mirrored on the host (launch sizes).
+// memory (the kernels' argument).
 struct O4Batch {
   int nbox = 0;
   Ctx* dev = nullptr;
-  std::vector<Ctx> host;
   bool roe = false, powell = false;
-  // work lists: per region kind and direction, chunks of kO4Chunk points of
-  // every box's region, all in one device array
+  // work lists: per region, chunks of every box's region (of every direction
+  // for the face regions), all in one device array
   WorkChunk* chunks = nullptr;
-  long chunkOff[RG_COUNT][3] = {};
-  int chunkCount[RG_COUNT][3] = {};
+  long chunkOff[RG_COUNT] = {};
+  int chunkCount[RG_COUNT] = {};
   int var[kO4TunedKernels] = {0, 0, 0};  // register-cap variant of the tuned kernels
-  // tiles of the fused face chain, per direction, in one device array;
-  // chainTI: radial width of an angular direction's tile (32, 16 or 8 by
-  // the narrowest box); chainTI0 that of direction 0 (16 or 8: its tiles
-  // are 8 rows of j deep, which halves the share of recomputed ring rows)
-  ChainTile* chainTiles = nullptr;
-  long chainOff[3] = {};
-  int chainCount[3] = {};
-  int chainTI = 32, chainTI0 = 16;
-  // TMA tensor maps of the angular chains' face slabs, per box and direction
-  // 1, 2: one copying 8 arrays, one copying 2 (device array; null without TMA)
-  CUtensorMap* maps = nullptr;
-  bool chainTma = false;
-  // The Powell face chain of a direction (face flux, radial product,
-  // divergence into -J div B) runs on a side stream beside the main face
-  // chain: fork after the reconstruction, join before the next direction.
-  // The cell-product coefficients and their averages (DivBPowell2's
-  // inputs, from the point primitives) go first on the same side stream.
+  // DivBPowell2's coefficients (from the point primitives) and the Powell
+  // face fluxes and divergence (from the reconstruction's flags and normal
+  // field) run on a side stream, joined before the cell pass.
   cudaStream_t side = nullptr;
-  cudaEvent_t pointEv = nullptr, forkEv[3] = {}, joinEv[3] = {};
-  // The Roe point dissipation (reads the face states, writes only the
-  // dissipation) runs on a second side stream beside the face-average,
-  // mapped-flux and radial-product kernels, which do not read it; the final
-  // flux waits for it.
-  cudaStream_t roeSide = nullptr;
-  cudaEvent_t roeFork[3] = {}, roeJoin[3] = {};
+  cudaEvent_t pointEv = nullptr, reconEv = nullptr, joinEv = nullptr;
 };
 
 // Minimum resident CTAs per SM (the register cap) of each variant of the
-// tuned kernels: reconstruction, Roe point dissipation, fused face chain.
-// Variant 0 is the default.  A chain CTA has one thread per face of a tile
-// row (132-144 threads); its shared memory (51-66 KB at 32-wide tiles)
-// admits at most 4 (direction 0) or 3 (with TMA) CTAs per SM.
-constexpr int kO4MinBlocks[kO4TunedKernels][kO4Variants] = {{6, 4, 8}, {4, 3, 5}, {3, 4, 2}};
-
-// Tiles of the fused face chain of direction d over the batch's boxes: TI
-// radial x 128/TI across (d = 0: j; d != 0: the other angular index),
-// walking d (d != 0) or k (d = 0) in segments of S cells, S the largest of
-// 64, 32, 16, 8 that still gives about 16 CTAs per SM.
-void chainTiles(const std::vector<Ctx>& host, int nbox, int d, int TI, std::vector<ChainTile>& out) {
-  const int TT = 128 / TI;
-  const int across = d == 0 ? 1 : (d == 1 ? 2 : 1), walk = d == 0 ? 2 : d;
-  long base = 0, longest = 1;
-  for (int b = 0; b < nbox; ++b) {
-    const Box3& V = host[(size_t)b * 3 + d].V;
-    base += (long)((V.n(0) + TI - 1) / TI) * ((V.n(across) + TT - 1) / TT);
-    longest = std::max<long>(longest, V.n(walk));
-  }
-  int S = 64;
-  while (S > 8 && base * ((longest + S - 1) / S) < 148L * 16) S /= 2;
-  for (int b = 0; b < nbox; ++b) {
-    const Box3& V = host[(size_t)b * 3 + d].V;
-    for (int c0 = V.lo[walk]; c0 <= V.hi[walk]; c0 += S)
-      for (int a0 = V.lo[across]; a0 <= V.hi[across]; a0 += TT)
-        for (int i0 = V.lo[0]; i0 <= V.hi[0]; i0 += TI)
-          out.push_back(ChainTile{b, i0, a0, c0, std::min(c0 + S - 1, V.hi[walk])});
-  }
-}
-
-// cuTensorMapEncodeTiled through the runtime's driver entry point (no link
-// against the driver library), or null where it is unavailable.
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn encodeTiled() {
-  static EncodeTiledFn fn = []() -> EncodeTiledFn {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      return nullptr;
-    return reinterpret_cast<EncodeTiledFn>(p);
-  }();
-  return fn;
-}
-
-// The tensor maps of the angular face chains of every box of a batch:
-// 4-D (radial, j, k, array) views of each box's face buffer for direction
-// d = 1, 2, boxes of (TI + 4) radial x (TT + 4) angular x 1 normal x 8 or 2
-// arrays.  False where a map cannot be made (then the chains read through
-// L1 instead).
-bool chainMaps(const std::vector<Ctx>& host, int nbox, int TI, int TI0, std::vector<CUtensorMap>& out) {
-  const EncodeTiledFn enc = encodeTiled();
-  if (!enc) return false;
-  const int TT = 128 / TI, TT0 = 128 / TI0;
-  out.resize((size_t)nbox * kChainMaps);
-  for (int b = 0; b < nbox; ++b) {
-    // direction 0: slabs of TI0 + 2 radial faces (an even count from an even
-    // offset) x TT0 + 2 rows of j x one k
-    {
-      const Ctx& c = host[(size_t)b * 3];
-      const cuuint64_t n0 = c.fr.n[0], n1 = c.fr.n[1], n2 = c.fr.n[2];
-      if ((reinterpret_cast<uintptr_t>(c.a.face) & 15) || (n0 & 1) || ((c.V.lo[0] - c.fr.lo[0]) & 1)) return false;
-      const cuuint64_t dims[4] = {n0, n1, n2, (cuuint64_t)kO4FaceArrays};
-      const cuuint64_t strides[3] = {n0 * 8, n0 * n1 * 8, n0 * n1 * n2 * 8};
-      for (int w = 0; w < 2; ++w) {
-        const cuuint32_t box[4] = {(cuuint32_t)(TI0 + 2), (cuuint32_t)(TT0 + 2), 1u, w == 0 ? 9u : 8u};
-        const cuuint32_t es[4] = {1, 1, 1, 1};
-        if (enc(&out[(size_t)b * kChainMaps + 4 + w], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, c.a.face, dims, strides,
-                box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-          return false;
-      }
-    }
-    for (int d = 1; d <= 2; ++d) {
-      const Ctx& c = host[(size_t)b * 3 + d];
-      const cuuint64_t n0 = c.fr.n[0], n1 = c.fr.n[1], n2 = c.fr.n[2];
-      // 16-byte aligned base and rows, and an even radial tile origin
-      // (tiles start at the valid box's low radial index, i0 - 2 - fr.lo)
-      if ((reinterpret_cast<uintptr_t>(c.a.face) & 15) || (n0 & 1) || ((c.V.lo[0] - 2 - c.fr.lo[0]) & 1)) return false;
-      const cuuint64_t dims[4] = {n0, n1, n2, (cuuint64_t)kO4FaceArrays};
-      const cuuint64_t strides[3] = {n0 * 8, n0 * n1 * 8, n0 * n1 * n2 * 8};
-      for (int w = 0; w < 2; ++w) {
-        const cuuint32_t box[4] = {(cuuint32_t)(TI + 4), d == 1 ? 1u : (cuuint32_t)(TT + 4),
-                                   d == 1 ? (cuuint32_t)(TT + 4) : 1u, w == 0 ? 8u : 2u};
-        const cuuint32_t es[4] = {1, 1, 1, 1};
-        if (enc(&out[(size_t)b * kChainMaps + (d - 1) * 2 + w], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, c.a.face, dims,
-                strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-          return false;
-      }
-    }
-  }
-  return true;
-}
-
-// Dynamic shared memory of the angular chain kernels (with and without TMA).
-template <int TI, bool TMA>
-cudaError_t chainSmemT() {
-  const int bytes = ChainShape<TI>::doubles(TMA) * (int)sizeof(double);
-  cudaError_t e = cudaSuccess;
-#define HC_CHAIN_ATTR(D, MB)                                                                                \
-  if (e == cudaSuccess)                                                                                    \
-    e = cudaFuncSetAttribute(o4FaceChainKernel<D, TI, MB, TMA>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  HC_CHAIN_ATTR(1, 2) HC_CHAIN_ATTR(1, 3) HC_CHAIN_ATTR(1, 4) HC_CHAIN_ATTR(2, 2) HC_CHAIN_ATTR(2, 3) HC_CHAIN_ATTR(2, 4)
-#undef HC_CHAIN_ATTR
-  return e;
-}
-
-template <int TI>
-cudaError_t chain0TmaSmem() {
-  const int bytes = Chain0Shape<TI>::doubles() * (int)sizeof(double);
-  cudaError_t e = cudaFuncSetAttribute(o4FaceChain0TmaKernel<TI, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(o4FaceChain0TmaKernel<TI, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(o4FaceChain0TmaKernel<TI, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  return e;
-}
-
-template <int TI>
-cudaError_t chain0Smem() {
-  const int bytes = chain0Doubles<TI>() * (int)sizeof(double);
-  cudaError_t e = cudaFuncSetAttribute(o4FaceChain0Kernel<TI, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(o4FaceChain0Kernel<TI, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(o4FaceChain0Kernel<TI, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  return e;
-}
+// tuned kernels: reconstruction, Riemann problem, final flux.  Variant 0 is
+// the default.
+constexpr int kO4MinBlocks[kO4TunedKernels][kO4Variants] = {{6, 8, 7}, {4, 3, 5}, {3, 4, 5}};
 
 void o4BatchSetVariants(O4Batch* B, const int v[kO4TunedKernels]) {
   for (int q = 0; q < kO4TunedKernels; ++q) B->var[q] = v[q] >= 0 && v[q] < kO4Variants ? v[q] : 0;
@@ -1952,115 +1146,55 @@ O4Batch* o4BatchCreate(const O4Args* boxes, int nbox, cudaError_t* err) {
     }
   O4Batch* B = new O4Batch;
   B->nbox = nbox;
-  B->host.resize((size_t)nbox * 3);
+  std::vector<Ctx> host((size_t)nbox * 3);
   for (int b = 0; b < nbox; ++b) {
     O4Args one = boxes[b];
     one.nbox = 1;
-    for (int d = 0; d < 3; ++d) B->host[(size_t)b * 3 + d] = makeCtx(one, d);
+    for (int d = 0; d < 3; ++d) host[(size_t)b * 3 + d] = makeCtx(one, d);
   }
   B->roe = boxes[0].G.roe;
   B->powell = boxes[0].G.powell;
   std::vector<WorkChunk> work;
-  for (int id = 0; id < RG_COUNT; ++id)
-    for (int d = 0; d < 3; ++d) {
-      B->chunkOff[id][d] = (long)work.size();
-      long total = 0, largest = 0;
-      bool equal = true;
-      for (int b = 0; b < nbox; ++b) {
-        const long n = regionOf(B->host[(size_t)b * 3 + d], id).size();
-        if (n >= 0x7fffffffL) {  // forRegion splits indices in 32 bits
-          *err = cudaErrorInvalidValue;
-          o4BatchDestroy(B);
-          return nullptr;
-        }
-        total += n;
-        equal = equal && (b == 0 || n == largest);
-        largest = n > largest ? n : largest;
-      }
-      if (equal) {
-        // boxes of one size: each box's CTAs stride over it together
-        // (about 148 x 32 CTAs in all)
-        const long need = (largest + 127) / 128;
-        const long perBox = std::max(1L, std::min(need, 148L * 32 / nbox));
-        for (int b = 0; b < nbox; ++b)
-          for (long x = 0; x < perBox; ++x) work.push_back(WorkChunk{b, (int)(perBox * 128), x * 128, largest});
-      } else {
-        // uneven boxes: contiguous chunks of equal work
-        const long chunk = chunkPoints(total);
-        for (int b = 0; b < nbox; ++b) {
-          const long n = regionOf(B->host[(size_t)b * 3 + d], id).size();
-          for (long t = 0; t < n; t += chunk) work.push_back(WorkChunk{b, 128, t, t + chunk < n ? t + chunk : n});
-        }
-      }
-      const long count = (long)work.size() - B->chunkOff[id][d];
-      if (count > 0x7fffffffL) {
+  for (int id = 0; id < RG_COUNT; ++id) {
+    B->chunkOff[id] = (long)work.size();
+    const long pass = passPoints(id);
+    const int nd = faceRegion(id) ? 3 : 1;
+    long total = 0;
+    for (size_t q = 0; q < (size_t)nbox * 3; ++q) {
+      if ((int)(q % 3) >= nd) continue;
+      const long n = regionOf(host[q], id).size();
+      if (n >= 0x7fffffffL) {  // forRegion splits indices in 32 bits
         *err = cudaErrorInvalidValue;
         o4BatchDestroy(B);
         return nullptr;
       }
-      B->chunkCount[id][d] = (int)count;
+      total += n;
     }
-  {
-    int narrow = 1 << 30;
-    for (int b = 0; b < nbox; ++b) narrow = std::min(narrow, B->host[(size_t)b * 3].V.n(0));
-    B->chainTI = narrow >= 24 ? 32 : narrow >= 12 ? 16 : 8;
-    B->chainTI0 = narrow >= 12 ? 16 : 8;
-  }
-  std::vector<ChainTile> tiles;
-  for (int d = 0; d < 3; ++d) {
-    B->chainOff[d] = (long)tiles.size();
-    chainTiles(B->host, nbox, d, d == 0 ? B->chainTI0 : B->chainTI, tiles);
-    const long count = (long)tiles.size() - B->chainOff[d];
+    const long chunk = chunkPoints(total, pass);
+    for (int d = 0; d < nd; ++d)
+      for (int b = 0; b < nbox; ++b) {
+        const long n = regionOf(host[(size_t)b * 3 + d], id).size();
+        for (long t = 0; t < n; t += chunk) work.push_back(WorkChunk{b, d, t, t + chunk < n ? t + chunk : n});
+      }
+    const long count = (long)work.size() - B->chunkOff[id];
     if (count > 0x7fffffffL) {
       *err = cudaErrorInvalidValue;
       o4BatchDestroy(B);
       return nullptr;
     }
-    B->chainCount[d] = (int)count;
+    B->chunkCount[id] = (int)count;
   }
-  *err = B->chainTI0 == 16 ? chain0Smem<16>() : chain0Smem<8>();
-  if (*err == cudaSuccess)
-    *err = B->chainTI == 32   ? chainSmemT<32, false>()
-           : B->chainTI == 16 ? chainSmemT<16, false>()
-                              : chainSmemT<8, false>();
-  {
-    std::vector<CUtensorMap> maps;
-    if (*err == cudaSuccess && chainMaps(B->host, nbox, B->chainTI, B->chainTI0, maps)) {
-      cudaError_t e = B->chainTI == 32   ? chainSmemT<32, true>()
-                      : B->chainTI == 16 ? chainSmemT<16, true>()
-                                         : chainSmemT<8, true>();
-      if (e == cudaSuccess) e = B->chainTI0 == 16 ? chain0TmaSmem<16>() : chain0TmaSmem<8>();
-      if (e == cudaSuccess) e = cudaMalloc(&B->maps, sizeof(CUtensorMap) * maps.size());
-      if (e == cudaSuccess)
-        e = cudaMemcpy(B->maps, maps.data(), sizeof(CUtensorMap) * maps.size(), cudaMemcpyHostToDevice);
-      B->chainTma = e == cudaSuccess;
-      if (e != cudaSuccess) cudaGetLastError();  // no TMA: the chains read through L1
-    }
-  }
-  if (*err == cudaSuccess) *err = cudaMalloc(&B->chainTiles, sizeof(ChainTile) * std::max<size_t>(1, tiles.size()));
-  if (*err == cudaSuccess && !tiles.empty())
-    *err = cudaMemcpy(B->chainTiles, tiles.data(), sizeof(ChainTile) * tiles.size(), cudaMemcpyHostToDevice);
-  if (*err == cudaSuccess) *err = cudaMalloc(&B->dev, sizeof(Ctx) * B->host.size());
-  if (*err == cudaSuccess) *err = cudaMemcpy(B->dev, B->host.data(), sizeof(Ctx) * B->host.size(), cudaMemcpyHostToDevice);
+  *err = cudaMalloc(&B->dev, sizeof(Ctx) * host.size());
+  if (*err == cudaSuccess) *err = cudaMemcpy(B->dev, host.data(), sizeof(Ctx) * host.size(), cudaMemcpyHostToDevice);
   if (*err == cudaSuccess && !work.empty()) {
     *err = cudaMalloc(&B->chunks, sizeof(WorkChunk) * work.size());
     if (*err == cudaSuccess)
       *err = cudaMemcpy(B->chunks, work.data(), sizeof(WorkChunk) * work.size(), cudaMemcpyHostToDevice);
   }
-  if (*err == cudaSuccess && B->roe) {
-    *err = cudaStreamCreateWithFlags(&B->roeSide, cudaStreamNonBlocking);
-    for (int d = 0; d < 3 && *err == cudaSuccess; ++d) {
-      *err = cudaEventCreateWithFlags(&B->roeFork[d], cudaEventDisableTiming);
-      if (*err == cudaSuccess) *err = cudaEventCreateWithFlags(&B->roeJoin[d], cudaEventDisableTiming);
-    }
-  }
   if (*err == cudaSuccess && B->powell) {
     *err = cudaStreamCreateWithFlags(&B->side, cudaStreamNonBlocking);
-    if (*err == cudaSuccess) *err = cudaEventCreateWithFlags(&B->pointEv, cudaEventDisableTiming);
-    for (int d = 0; d < 3 && *err == cudaSuccess; ++d) {
-      *err = cudaEventCreateWithFlags(&B->forkEv[d], cudaEventDisableTiming);
-      if (*err == cudaSuccess) *err = cudaEventCreateWithFlags(&B->joinEv[d], cudaEventDisableTiming);
-    }
+    for (cudaEvent_t* ev : {&B->pointEv, &B->reconEv, &B->joinEv})
+      if (*err == cudaSuccess) *err = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
   }
   if (*err != cudaSuccess) {
     o4BatchDestroy(B);
@@ -2073,17 +1207,9 @@ void o4BatchDestroy(O4Batch* B) {
   if (!B) return;
   if (B->dev) cudaFree(B->dev);
   if (B->chunks) cudaFree(B->chunks);
-  if (B->chainTiles) cudaFree(B->chainTiles);
-  if (B->maps) cudaFree(B->maps);
-  if (B->pointEv) cudaEventDestroy(B->pointEv);
-  for (int d = 0; d < 3; ++d) {
-    if (B->roeFork[d]) cudaEventDestroy(B->roeFork[d]);
-    if (B->roeJoin[d]) cudaEventDestroy(B->roeJoin[d]);
-    if (B->forkEv[d]) cudaEventDestroy(B->forkEv[d]);
-    if (B->joinEv[d]) cudaEventDestroy(B->joinEv[d]);
-  }
+  for (cudaEvent_t ev : {B->pointEv, B->reconEv, B->joinEv})
+    if (ev) cudaEventDestroy(ev);
   if (B->side) cudaStreamDestroy(B->side);
-  if (B->roeSide) cudaStreamDestroy(B->roeSide);
   delete B;
 }
 
@@ -2096,160 +1222,72 @@ void o4SplitArgs(const O4Args& a, std::vector<O4Args>& out) {
     o.block0 = a.block0 + b;
     o.U = a.U + (long)b * a.uStride;
     o.rhs = a.rhs + (long)b * a.rhsStride;
-    for (int d = 0; d < 3; ++d)
+    for (int d = 0; d < 3; ++d) {
       if (a.flux[d]) o.flux[d] = a.flux[d] + (long)b * 8 * c.V.extrude(d).size();
+      o.face[d] = a.face[d] + (long)b * kO4FaceArrays * c.fr.N;
+    }
     o.WA = a.WA + (long)b * 8 * c.gr.N;
     o.WP = a.WP + (long)b * 8 * c.gr.N;
     o.th = a.th + (long)b * c.gr.N;
     o.thr = a.thr + (long)b * c.gr.N;
-    o.face = a.face + (long)b * kO4FaceArrays * c.fr.N;
-    o.face2 = a.face2 + (long)b * kO4FaceArrays * c.fr.N;
     o.mj = a.mj + (long)b * c.v1r.N;
-    o.kp = a.kp + (long)b * 16 * c.v2r.N;
+    o.ka = a.ka + (long)b * 7 * c.v1r.N;
   }
 }
-
-namespace {
-}  // namespace
 
 cudaError_t launchO4BatchGravity(const O4Batch* B, cudaStream_t s) {
   const RegArgs none{};
-  if (B->chunkCount[RG_V][0] == 0) return cudaSuccess;
-  o4GravityKernel<<<B->chunkCount[RG_V][0], 128, 0, s>>>(B->dev, none, B->chunks + B->chunkOff[RG_V][0]);
+  if (B->chunkCount[RG_V] == 0) return cudaSuccess;
+  o4GravityKernel<<<B->chunkCount[RG_V], 128, 0, s>>>(B->dev, none, B->chunks + B->chunkOff[RG_V]);
   return cudaGetLastError();
-}
-
-// The fused face chain of direction d over the batch's tiles.
-template <int TI, int MB>
-cudaError_t launchChainT(const O4Batch* B, const RegArgs& rg, int d, cudaStream_t s) {
-  const int n = B->chainCount[d];
-  const ChainTile* t = B->chainTiles + B->chainOff[d];
-  if (n == 0) return cudaSuccess;
-  const size_t smemTma = ChainShape<TI>::doubles(true) * sizeof(double);
-  const size_t smemL1 = ChainShape<TI>::doubles(false) * sizeof(double);
-  if (d == 0 && B->chainTma)
-    o4FaceChain0TmaKernel<TI, MB><<<n, Chain0Shape<TI>::NTH, Chain0Shape<TI>::doubles() * sizeof(double), s>>>(
-        B->dev, rg, t, B->maps);
-  else if (d == 0)
-    o4FaceChain0Kernel<TI, MB><<<n, chain0Threads<TI>(), chain0Doubles<TI>() * sizeof(double), s>>>(B->dev, rg, t);
-  else if (d == 1 && B->chainTma)
-    o4FaceChainKernel<1, TI, MB, true><<<n, ChainShape<TI>::NTH, smemTma, s>>>(B->dev, rg, t, B->maps);
-  else if (d == 1)
-    o4FaceChainKernel<1, TI, MB, false><<<n, ChainShape<TI>::NTH, smemL1, s>>>(B->dev, rg, t, nullptr);
-  else if (B->chainTma)
-    o4FaceChainKernel<2, TI, MB, true><<<n, ChainShape<TI>::NTH, smemTma, s>>>(B->dev, rg, t, B->maps);
-  else
-    o4FaceChainKernel<2, TI, MB, false><<<n, ChainShape<TI>::NTH, smemL1, s>>>(B->dev, rg, t, nullptr);
-  return cudaGetLastError();
-}
-
-template <int TI>
-cudaError_t launchChainV(const O4Batch* B, const RegArgs& rg, int d, cudaStream_t s) {
-  switch (kO4MinBlocks[2][B->var[2]]) {
-    case 2: return launchChainT<TI, 2>(B, rg, d, s);
-    case 4: return launchChainT<TI, 4>(B, rg, d, s);
-    default: return launchChainT<TI, 3>(B, rg, d, s);
-  }
-}
-
-cudaError_t launchChain(const O4Batch* B, const RegArgs& rg, int d, cudaStream_t s) {
-  if (d == 0) return B->chainTI0 == 16 ? launchChainV<16>(B, rg, d, s) : launchChainV<8>(B, rg, d, s);
-  if (B->chainTI == 32) return launchChainV<32>(B, rg, d, s);
-  if (B->chainTI == 16) return launchChainV<16>(B, rg, d, s);
-  return launchChainV<8>(B, rg, d, s);
 }
 
 cudaError_t launchO4Batch(const O4Batch* B, const RegArgs* reg, cudaStream_t s) {
   const RegArgs none{};
   const RegArgs rg = reg ? *reg : none;
-  const Ctx* t = B->dev;
-  cudaError_t e;
-  cudaStream_t st = s;  // the stream the macros below launch on
-#define HC_LAUNCH(kernel, d, region)                                                           \
-  if (B->chunkCount[region][d]) {                                                              \
-    kernel<<<B->chunkCount[region][d], 128, 0, st>>>(t, rg, B->chunks + B->chunkOff[region][d]); \
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;                                     \
-  }
-#define HC_LAUNCH_D(kernel, region)                                                      \
-  if (d == 0) { HC_LAUNCH(kernel<0>, 0, region) }                                       \
-  else if (d == 1) { HC_LAUNCH(kernel<1>, 1, region) }                                  \
-  else { HC_LAUNCH(kernel<2>, 2, region) }
-#define HC_LAUNCH_DM(kernel, q, region)                                                  \
-  if (B->var[q] == 1) { HC_LAUNCH_DV(kernel, kO4MinBlocks[q][1], region) }                \
-  else if (B->var[q] == 2) { HC_LAUNCH_DV(kernel, kO4MinBlocks[q][2], region) }           \
-  else { HC_LAUNCH_DV(kernel, kO4MinBlocks[q][0], region) }
-#define HC_LAUNCH_T(d, region, ...)                                                                \
-  if (B->chunkCount[region][d]) {                                                                  \
-    __VA_ARGS__<<<B->chunkCount[region][d], 128, 0, st>>>(t, rg, B->chunks + B->chunkOff[region][d]); \
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;                                         \
-  }
-#define HC_LAUNCH_DV(kernel, mb, region)                                                 \
-  if (d == 0) { HC_LAUNCH_T(0, region, kernel<0, mb>) }                                 \
-  else if (d == 1) { HC_LAUNCH_T(1, region, kernel<1, mb>) }                            \
-  else { HC_LAUNCH_T(2, region, kernel<2, mb>) }
-  HC_LAUNCH(o4PrimAvgKernel, 0, RG_G)
-  HC_LAUNCH(o4ThetaRawKernel, 0, RG_GR)
-  HC_LAUNCH(o4PointKernel, 0, RG_G)
+  cudaError_t e = cudaSuccess;
+  using Kernel = void (*)(const Ctx*, const RegArgs, const WorkChunk*);
+  auto launch = [&](Kernel kernel, RegionId region, cudaStream_t st, unsigned groups = 1) {
+    if (e != cudaSuccess || B->chunkCount[region] == 0) return;
+    kernel<<<dim3((unsigned)B->chunkCount[region], groups), 128, 0, st>>>(B->dev, rg, B->chunks + B->chunkOff[region]);
+    e = cudaGetLastError();
+  };
+  // the side stream's next kernels run after everything queued on s so far
+  auto fork = [&](cudaEvent_t ev) {
+    if (e == cudaSuccess) e = cudaEventRecord(ev, s);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(B->side, ev, 0);
+  };
+  static constexpr Kernel recon[kO4Variants] = {o4FaceReconKernel<kO4MinBlocks[0][0]>,
+                                                o4FaceReconKernel<kO4MinBlocks[0][1]>,
+                                                o4FaceReconKernel<kO4MinBlocks[0][2]>};
+  static constexpr Kernel riemann[2][kO4Variants] = {
+      {o4FaceRiemannKernel<false, kO4MinBlocks[1][0]>, o4FaceRiemannKernel<false, kO4MinBlocks[1][1]>,
+       o4FaceRiemannKernel<false, kO4MinBlocks[1][2]>},
+      {o4FaceRiemannKernel<true, kO4MinBlocks[1][0]>, o4FaceRiemannKernel<true, kO4MinBlocks[1][1]>,
+       o4FaceRiemannKernel<true, kO4MinBlocks[1][2]>}};
+  static constexpr Kernel final[kO4Variants] = {o4FaceFinalKernel<kO4MinBlocks[2][0]>,
+                                                o4FaceFinalKernel<kO4MinBlocks[2][1]>,
+                                                o4FaceFinalKernel<kO4MinBlocks[2][2]>};
+  launch(o4PrimAvgKernel, RG_G, s);
+  launch(o4ThetaRawKernel, RG_GR, s);
+  launch(o4PointKernel, RG_G, s);
   if (B->powell) {
-    // DivBPowell2's coefficients need only the point primitives: fork them
-    // (the side stream runs them before the first direction's Powell chain)
-    if ((e = cudaEventRecord(B->pointEv, s)) != cudaSuccess) return e;
-    if ((e = cudaStreamWaitEvent(B->side, B->pointEv, 0)) != cudaSuccess) return e;
-    st = B->side;
-    HC_LAUNCH(o4PowellCoefKernel, 0, RG_V2)
-    HC_LAUNCH(o4PowellAvgKernel, 0, RG_V1)
-    st = s;
+    fork(B->pointEv);
+    launch(o4PowellAvgKernel, RG_V1, B->side);
   }
-  // Direction d's face arrays are face buffer d & 1 (direction 1 has its
-  // own), so the passes overlap: the Roe point dissipation of d (second side
-  // stream) runs beside the face chain of d - 1 and the reconstruction of
-  // d + 1 on the main stream; the Powell face chain of d (first side stream)
-  // beside them.  The reconstruction of d + 2 reuses d's buffer and waits
-  // for d's Powell chain; d's face chain waits for d's Roe dissipation;
-  // the chains add into rhs in direction order on the main stream.
-  for (int d = 0; d < 3; ++d) {
-    if (d >= 2 && B->powell && (e = cudaStreamWaitEvent(s, B->joinEv[d - 2], 0)) != cudaSuccess) return e;
-    HC_LAUNCH_DM(o4FaceReconKernel, 0, RG_F)
-    // direction 0's face averages for its TMA chain (beside the Roe point
-    // dissipation, which reads neither their inputs' outputs nor them)
-    if (d == 0 && B->chainTma) { HC_LAUNCH(o4FaceAvg0Kernel, 0, RG_PB) }
-    if (B->powell) {
-      // the Powell chain reads the reconstruction's flags and normal B and
-      // writes only its own face arrays and -J div B: fork it
-      if ((e = cudaEventRecord(B->forkEv[d], s)) != cudaSuccess) return e;
-      if ((e = cudaStreamWaitEvent(B->side, B->forkEv[d], 0)) != cudaSuccess) return e;
-      st = B->side;
-      HC_LAUNCH_D(o4PowellFluxKernel, RG_PF)
-      HC_LAUNCH_D(o4PowellProdKernel, RG_PP)
-      HC_LAUNCH_D(o4PowellDivKernel, RG_V1)
-      st = s;
-      if ((e = cudaEventRecord(B->joinEv[d], B->side)) != cudaSuccess) return e;
-    }
-    if (B->roe) {
-      if ((e = cudaEventRecord(B->roeFork[d], s)) != cudaSuccess) return e;
-      if ((e = cudaStreamWaitEvent(B->roeSide, B->roeFork[d], 0)) != cudaSuccess) return e;
-      st = B->roeSide;
-      HC_LAUNCH_DM(o4RoePointKernel, 1, RG_PB)
-      st = s;
-      if ((e = cudaEventRecord(B->roeJoin[d], B->roeSide)) != cudaSuccess) return e;
-    }
-    if (d >= 1) {
-      if (B->roe && (e = cudaStreamWaitEvent(s, B->roeJoin[d - 1], 0)) != cudaSuccess) return e;
-      if ((e = launchChain(B, rg, d - 1, s)) != cudaSuccess) return e;
-    }
+  launch(recon[B->var[0]], RG_F, s);
+  launch(riemann[B->roe ? 1 : 0][B->var[1]], RG_F, s);
+  if (B->powell) {
+    fork(B->reconEv);
+    launch(o4PowellFluxKernel, RG_PF, B->side);
+    launch(o4PowellDivKernel, RG_V1, B->side);
+    if (e == cudaSuccess) e = cudaEventRecord(B->joinEv, B->side);
   }
-  if (B->roe && (e = cudaStreamWaitEvent(s, B->roeJoin[2], 0)) != cudaSuccess) return e;
-  if ((e = launchChain(B, rg, 2, s)) != cudaSuccess) return e;
-  for (int d = 0; d < 3 && B->powell; ++d)
-    if ((e = cudaStreamWaitEvent(s, B->joinEv[d], 0)) != cudaSuccess) return e;
-  // after the last join: -J div B complete, coefficients averaged
-  if (B->powell) { HC_LAUNCH(o4PowellApplyKernel, 0, RG_V) }
-#undef HC_LAUNCH_DV
-#undef HC_LAUNCH_T
-#undef HC_LAUNCH_DM
-#undef HC_LAUNCH_D
-#undef HC_LAUNCH
-  return cudaSuccess;
+  launch(o4FaceAvgKernel, RG_PB, s);
+  launch(final[B->var[2]], RG_V0, s);
+  if (B->powell && e == cudaSuccess) e = cudaStreamWaitEvent(s, B->joinEv, 0);
+  launch(o4CellKernel, RG_V, s);
+  return e;
 }
 
 }  // namespace hc

@@ -555,7 +555,7 @@ int hc_amr_native(hc_ctx* ctx, const hc_amr_plan* plan, int first, int count, do
  * the host).  Order 2: the stage kernel runs one CTA per cell tile; the
  * tiles differ in shape and in the register cap (resident CTAs per SM), and
  * the fastest depends on the limiter / solver pair and the level size.
- * Order 4: the reconstruction, Roe point and final-flux kernels each come
+ * Order 4: the reconstruction, Riemann and final-flux kernels each come
  * in register-cap variants.  Order-2 results do not depend on the tile.  The
  * order-4 variants agree to round-off only: the code generator may contract
  * a multiply and an add into one fused operation differently under each
@@ -574,8 +574,8 @@ int hc_stage_tiles(int* shapes, int capacity);
  * (host, nullable, 2 ints) gets {RK stage tile, operator tile}; ms (host,
  * nullable, 2 x count doubles) the median launch times, RK stage first.
  * Order 4: time the level operator (after the stage preparation of ju) for
- * each register-cap variant of the reconstruction, Roe point dissipation
- * and final-flux kernels in turn, keeping the best of each; tiles (3 ints)
+ * each register-cap variant of the reconstruction, Riemann and
+ * final-flux kernels in turn, keeping the best of each; tiles (3 ints)
  * gets the variants, ms (3 x hc_o4_variants() doubles) the operator times.
  * Blocks the host until the timing is done: call it outside stream capture.
  * The choice is also kept process-wide for contexts of the same device,
@@ -585,7 +585,7 @@ int hc_ctx_autotune(hc_ctx* ctx, const double* ju, int* tiles, double* ms, void*
 
 /* Number of register-cap variants per tuned fourth-order kernel; with
  * min_blocks non-null, min_blocks[3 q + v] = minimum resident CTAs per SM of
- * variant v of kernel q (0 reconstruction, 1 Roe point, 2 fused face chain). */
+ * variant v of kernel q (0 reconstruction, 1 Riemann problem, 2 final flux). */
 int hc_o4_variants(int* min_blocks, int capacity);
 
 /* Use the given variants (3 ints, -1 keeps the current one). */
