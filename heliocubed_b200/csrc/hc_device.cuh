@@ -28,63 +28,6 @@ HC_DEV unsigned takeMod(unsigned& t, unsigned n) {
 HC_DEV double dmin(double a, double b) { return b < a ? b : a; }  // std::min
 HC_DEV double dmax(double a, double b) { return a < b ? b : a; }  // std::max
 
-// src/BoxOp_SecondOrder.H:7-37, one component.  LIM: 0 unlimited,
-// 1 minmod (limiter 1 or 2), 3 monotonized central.
-template <int LIM>
-HC_DEV void plmComponent(double mm, double m, double c, double p, double& lo, double& hi) {
-  const double a = m - mm, b = c - m, d = p - c;
-  double sl = 0.5 * (a + b), sr = 0.5 * (b + d);
-  if (LIM != 0) {
-    sl = a * b <= 0 ? 0.0 : (a > 0 ? dmin(a, b) : dmax(a, b));
-    sr = b * d <= 0 ? 0.0 : (b > 0 ? dmin(b, d) : dmax(b, d));
-    if (LIM == 3) {
-      if (a * b > 0) sl = (a > 0 ? 1.0 : -1.0) * dmin(0.5 * fabs(a + b), 2.0 * dmin(fabs(a), fabs(b)));
-      if (b * d > 0) sr = (b > 0 ? 1.0 : -1.0) * dmin(0.5 * fabs(b + d), 2.0 * dmin(fabs(b), fabs(d)));
-    }
-  }
-  lo = m + 0.5 * sl;
-  hi = c - 0.5 * sr;
-}
-
-// Left state of a face from cells (i-2, i-1, i) only (the "lo" half of the
-// reference's pair), with its complete-state fallback.
-template <int LIM>
-HC_DEV void plmLeft(const double* mm, const double* m, const double* c, double lo[8]) {
-#pragma unroll
-  for (int k = 0; k < NC; ++k) {
-    const double a = m[k] - mm[k], b = c[k] - m[k];
-    double sl = 0.5 * (a + b);
-    if (LIM != 0) {
-      sl = a * b <= 0 ? 0.0 : (a > 0 ? dmin(a, b) : dmax(a, b));
-      if (LIM == 3 && a * b > 0) sl = (a > 0 ? 1.0 : -1.0) * dmin(0.5 * fabs(a + b), 2.0 * dmin(fabs(a), fabs(b)));
-    }
-    lo[k] = m[k] + 0.5 * sl;
-  }
-  if (!(lo[0] >= kRHO00 && lo[4] >= 0)) {
-#pragma unroll
-    for (int k = 0; k < NC; ++k) lo[k] = m[k];
-  }
-}
-
-// Right state of a face from cells (i-1, i, i+1) only.
-template <int LIM>
-HC_DEV void plmRight(const double* m, const double* c, const double* p, double hi[8]) {
-#pragma unroll
-  for (int k = 0; k < NC; ++k) {
-    const double b = c[k] - m[k], d = p[k] - c[k];
-    double sr = 0.5 * (b + d);
-    if (LIM != 0) {
-      sr = b * d <= 0 ? 0.0 : (b > 0 ? dmin(b, d) : dmax(b, d));
-      if (LIM == 3 && b * d > 0) sr = (b > 0 ? 1.0 : -1.0) * dmin(0.5 * fabs(b + d), 2.0 * dmin(fabs(b), fabs(d)));
-    }
-    hi[k] = c[k] - 0.5 * sr;
-  }
-  if (!(hi[0] >= kRHO00 && hi[4] >= 0)) {
-#pragma unroll
-    for (int k = 0; k < NC; ++k) hi[k] = c[k];
-  }
-}
-
 // A double whose sums and products round exactly as written: the compiler
 // may contract a plain a * b + c into one fused operation or not, and does
 // so differently from kernel to kernel and with the register cap, while
@@ -135,6 +78,53 @@ HC_DEV double rsqrtN(double x) {
 HC_DEV double sqrtN(double x) {
   const double y = rsqrtN(x), s = __dmul_rn(x, y);
   return x > 1e-290 ? fma(0.5 * y, fma(-s, s, x), s) : 0.0;
+}
+
+// Half the limited slope of a cell with differences a, b to its neighbours
+// (src/BoxOp_SecondOrder.H:7-37).  LIM: 0 unlimited, 1 minmod (limiter 1 or
+// 2), 3 monotonized central: the smaller of |a + b| / 4 and min(|a|, |b|)
+// with the differences' sign, 0 where they differ in sign.  The candidates
+// keep their signs through the selection, so no sign is taken off and put
+// back; a NaN difference gives NaN.
+template <int LIM>
+HC_DEV Rn halfSlope(Rn a, Rn b) {
+  const Rn q = 0.25 * (a + b);
+  if (LIM == 0) return q;
+  const double small = fabs(b.v) < fabs(a.v) ? b.v : a.v;
+  const double t = LIM == 1 ? 0.5 * small : (fabs(small) < fabs(q.v) ? small : q.v);
+  const double sign = a * b;
+  return sign > 0.0 ? t : (sign <= 0.0 ? 0.0 : sign);
+}
+
+// Left and right states of a face from its four cells, one component.
+template <int LIM>
+HC_DEV void plmComponent(double mm, double m, double c, double p, double& lo, double& hi) {
+  const Rn a = Rn(m) - mm, b = Rn(c) - m, d = Rn(p) - c;
+  lo = m + halfSlope<LIM>(a, b);
+  hi = c - halfSlope<LIM>(b, d);
+}
+
+// Left state of a face from cells (i-2, i-1, i) only (the "lo" half of the
+// reference's pair), with its complete-state fallback.
+template <int LIM>
+HC_DEV void plmLeft(const double* mm, const double* m, const double* c, double lo[8]) {
+#pragma unroll
+  for (int k = 0; k < NC; ++k) lo[k] = m[k] + halfSlope<LIM>(Rn(m[k]) - mm[k], Rn(c[k]) - m[k]);
+  if (!(lo[0] >= kRHO00 && lo[4] >= 0)) {
+#pragma unroll
+    for (int k = 0; k < NC; ++k) lo[k] = m[k];
+  }
+}
+
+// Right state of a face from cells (i-1, i, i+1) only.
+template <int LIM>
+HC_DEV void plmRight(const double* m, const double* c, const double* p, double hi[8]) {
+#pragma unroll
+  for (int k = 0; k < NC; ++k) hi[k] = c[k] - halfSlope<LIM>(Rn(c[k]) - m[k], Rn(p[k]) - c[k]);
+  if (!(hi[0] >= kRHO00 && hi[4] >= 0)) {
+#pragma unroll
+    for (int k = 0; k < NC; ++k) hi[k] = c[k];
+  }
 }
 
 // src/MHD_Roe8Wave.H:604-629.  invGm1 = 1/(gamma-1) replaces the division
@@ -365,21 +355,20 @@ HC_DEV void secondOrderFaceFlux(double out[8], const double* l, const double* r,
 
 // src/MHD_StateConversion.H:11-32 (no constant-background magnetic test).
 HC_DEV void cartesianPrimitiveFromConserved(double out[8], const double in[8], double inverseJ, double gamma) {
-  double u[8];
+  Rn u[8];
 #pragma unroll
-  for (int c = 0; c < 8; ++c) u[c] = in[c] * inverseJ;
-  const double rho = u[0] < kMP / 100 ? kMP / 100 : u[0];
-  double kinetic = 0, magnetic = 0;
+  for (int c = 0; c < 8; ++c) u[c] = Rn(in[c]) * inverseJ;
+  const Rn rho = u[0] < kMP / 100 ? kMP / 100 : u[0].v;
+  const Rn inv = rcpN(rho);
   out[0] = rho;
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    out[1 + d] = u[1 + d] / rho;
+    out[1 + d] = u[1 + d] * inv;
     out[5 + d] = u[5 + d];
-    kinetic += 0.5 * rho * out[1 + d] * out[1 + d];
-    magnetic += u[5 + d] * u[5 + d] / (8 * kPi);
   }
-  const double pressure = (gamma - 1.0) * (u[4] - kinetic - magnetic);
-  out[4] = pressure < 0.0 ? 0.0 : pressure;
+  const Rn m2 = dot3(u[1], out[1], u[2], out[2], u[3], out[3]), b2 = dot3(u[5], u[5], u[6], u[6], u[7], u[7]);
+  const Rn pressure = (gamma - 1.0) * (mad(-0.5, m2, u[4]) - (0.125 / kPi) * b2);
+  out[4] = pressure < 0.0 ? 0.0 : pressure.v;
 }
 
 // Inner analytic wind, native conserved variables at Cartesian point X and

@@ -22,6 +22,14 @@ namespace {
 // (Rusanov, Roe).  The autotuner (hc_ctx_autotune) times them per limiter /
 // solver pair on the caller's level; every tile computes every face and cell
 // with the same arithmetic, so results do not depend on the choice.
+//
+// The kernel is bound by instruction issue and by the latency of the stencil
+// loads.  Per stage of 64 x 32^2 x 6 (MC + Rusanov, Roe): 226 and 610 us with
+// limiters that took signs off and put them back, divisions, the Roe solver
+// out of line and a loop over all threads per direction; 112 and 168 us with
+// signed half slopes, reciprocals, the faces dealt to warps and 126 / 168
+// registers (the default tile; one CTA less per SM 120 and 212, one more
+// 118 and 185 with 130 to 300 bytes spilled).
 template <int X, int Y, int Z, int MB_RUS, int MB_ROE>
 struct Tile {
   static constexpr int TX = X, TY = Y, TZ = Z, NT = X * Y * Z;
@@ -29,11 +37,11 @@ struct Tile {
   static constexpr int NF = NF0 + NF1 + NF2;
   static constexpr int minBlocks(bool roe) { return roe ? MB_ROE : MB_RUS; }
 };
-using Tile0 = Tile<16, 4, 2, 3, 2>;
+using Tile0 = Tile<16, 4, 2, 4, 3>;
 using Tile1 = Tile<32, 2, 2, 3, 2>;
 using Tile2 = Tile<8, 8, 2, 3, 2>;
 using Tile3 = Tile<16, 2, 4, 3, 2>;
-using Tile4 = Tile<16, 4, 2, 4, 3>;
+using Tile4 = Tile<16, 4, 2, 3, 2>;
 using Tile5 = Tile<32, 4, 1, 3, 2>;
 static_assert(Tile0::NT == 128 && Tile1::NT == 128 && Tile2::NT == 128 && Tile3::NT == 128 && Tile4::NT == 128 &&
                   Tile5::NT == 128,
@@ -143,10 +151,11 @@ __device__ __forceinline__ void o2Face(const StageArgs& a, const double* __restr
   const long c0 = cellOffset(i, j, k, a.wlo, a.wn);
   const long step = dir == 0 ? 1L : dir == 1 ? (long)a.wn[0] : (long)a.wn[0] * a.wn[1];
   double l[8], r[8];
+  {
+    const double* s = w + c0;
 #pragma unroll
-  for (int q = 0; q < NC; ++q) {
-    const double* s = w + q * sN + c0;
-    plmComponent<LIM>(__ldg(s - 2 * step), __ldg(s - step), __ldg(s), __ldg(s + step), l[q], r[q]);
+    for (int q = 0; q < NC; ++q, s += sN)
+      plmComponent<LIM>(__ldg(s - 2 * step), __ldg(s - step), __ldg(s), __ldg(s + step), l[q], r[q]);
   }
   // Complete-state fallbacks (src/BoxOp_SecondOrder.H:32-36).
   if (!(l[0] >= kRHO00 && l[4] >= 0)) {
@@ -200,7 +209,18 @@ __device__ __forceinline__ void o2Face(const StageArgs& a, const double* __restr
       }
     }
   }
-  const FaceGeom& g = L.face[((size_t)dir * 6 + block) * (L.na + 1) * (L.na + 1) + (size_t)k * (L.na + 1) + j];
+  FaceGeom g;  // its first fourteen doubles, in pairs
+  {
+    const int n = L.na + 1;
+    const double2* src = reinterpret_cast<const double2*>(L.face + (((dir * 6 + block) * n + k) * n + j));
+    double* dst = reinterpret_cast<double*>(&g);
+#pragma unroll
+    for (int q = 0; q < 7; ++q) {
+      const double2 v = __ldg(src + q);
+      dst[2 * q] = v.x;
+      dst[2 * q + 1] = v.y;
+    }
+  }
   if (MODE == MODE_RK && dir == 0 && i == 0 && L.ninlet) {
     // Inlet footprint on the inner face (src/BoxOp_SecondOrder.H:175-181,
     // 282-311): where an emerging cloud covers the face, the interior state
@@ -245,10 +265,7 @@ __device__ __forceinline__ void o2Face(const StageArgs& a, const double* __restr
   const double area = dir == 0 ? rd.x : rd.y;
   secondOrderFaceFlux<ROE>(out, l, r, g, area, L.gamma, L.invGm1, L.entropy);
   if (powell) {
-    double f = 0;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) f += 0.5 * (l[5 + d] + r[5 + d]) * g.n[d] * area;
-    bf = f;
+    bf = 0.5 * Rn(area) * dot3(Rn(l[5]) + r[5], g.n[0], Rn(l[6]) + r[6], g.n[1], Rn(l[7]) + r[7], g.n[2]);
   }
 }
 
@@ -268,53 +285,44 @@ __device__ __forceinline__ double cflRate(const DevLevel& L, int b, int i, int j
                                           double coneDensity = 0) {
   const CflCell& a = L.cfl[((size_t)b * L.na + k) * L.na + j];
   const double4 rd = L.radial[i + L.g];
-  const double volume = rd.w, inverseVolume = 1.0 / rd.w, width0 = rd.z * L.dxi0;
-  const double area[3] = {rd.x, rd.y, rd.y};
-  double rho = u[0] * a.inverseDet;
-  rho *= inverseVolume;
-  rho = dmax(rho, kRHO00);
-  double energy = u[4] * a.inverseDet;
-  energy *= inverseVolume;
-  double v[3], bb[3];
+  const Rn volume = rd.w, invVolume = rcpN(volume);
+  const Rn scale = invVolume * a.inverseDet;
+  const Rn rho = dmax(scale * u[0], kRHO00), invRho = rcpN(rho);
+  Rn v[3], bb[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    v[d] = a.inverseDetA[3 * d] * u[1] + a.inverseDetA[3 * d + 1] * u[2] + a.inverseDetA[3 * d + 2] * u[3];
-    bb[d] = a.inverseDetA[3 * d] * u[5] + a.inverseDetA[3 * d + 1] * u[6] + a.inverseDetA[3 * d + 2] * u[7];
-    v[d] *= inverseVolume;
-    bb[d] *= inverseVolume;
-    v[d] /= rho;
+    const double* A = a.inverseDetA + 3 * d;
+    v[d] = dot3(A[0], u[1], A[1], u[2], A[2], u[3]) * invVolume * invRho;
+    bb[d] = dot3(A[0], u[5], A[1], u[6], A[2], u[7]) * invVolume;
   }
-  double kinetic = 0, magnetic = 0;
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    const double vc = a.cell[3 * d] * v[0] + a.cell[3 * d + 1] * v[1] + a.cell[3 * d + 2] * v[2];
-    const double bc = a.cell[3 * d] * bb[0] + a.cell[3 * d + 1] * bb[1] + a.cell[3 * d + 2] * bb[2];
-    kinetic += vc * vc / 2;
-    magnetic += bc * bc / 8.0 / kPi;
-  }
-  kinetic *= rho;
-  double pressure = (energy - kinetic - magnetic) * (L.gamma - 1);
-  if (pressure < 0) pressure = 0;
-  double inverseDt = 0;
+  // |v|^2 and |B|^2 in the basis of the cell (direction 0) and of its low faces
+  const double invH = 1.0 / L.h;
+  Rn pressure = 0.0, rate = 0.0;
+  const double magneticDensity = coneDensity > 0 ? fmin(rho, coneDensity) : rho.v;
+  // src/BoxOp_SecondOrderCFL.H:196-200: a cone may impose a lighter total
+  // density under the ambient field; bound that Alfven speed
+  const Rn alfven = (0.25 / kPi) * Rn(coneDensity > 0 ? rcpN(magneticDensity) : invRho.v);
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     const double* basis = d == 0 ? a.cell : a.face[d - 1];
-    double v2 = 0, fullB2 = 0;
+    Rn v2 = 0.0, b2 = 0.0;
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
-      const double velocity = basis[3 * q] * v[0] + basis[3 * q + 1] * v[1] + basis[3 * q + 2] * v[2];
-      const double field = basis[3 * q] * bb[0] + basis[3 * q + 1] * bb[1] + basis[3 * q + 2] * bb[2];
-      v2 += velocity * velocity;
-      fullB2 += field * field;
+      const double* A = basis + 3 * q;
+      const Rn x = dot3(A[0], v[0], A[1], v[1], A[2], v[2]), y = dot3(A[0], bb[0], A[1], bb[1], A[2], bb[2]);
+      v2 = mad(x, x, v2);
+      b2 = mad(y, y, b2);
     }
-    const double width = d == 0 ? width0 : volume * a.det[d] * L.h / area[d] / a.normal[d];
-    // src/BoxOp_SecondOrderCFL.H:196-200: a cone may impose a lighter total
-    // density under the ambient field; bound that Alfven speed
-    const double magneticDensity = coneDensity > 0 ? fmin(rho, coneDensity) : rho;
-    const double wave = sqrt(L.gamma * pressure / rho + fullB2 / 4.0 / kPi / magneticDensity);
-    inverseDt += (wave + sqrt(v2)) / width;
+    if (d == 0) {
+      pressure = (mad(-0.5 * rho, v2, scale * u[4]) - (0.125 / kPi) * b2) * (L.gamma - 1);
+      if (pressure < 0.0) pressure = 0.0;
+    }
+    // 1 / width: width is the radial cell size, or volume det h / (area |n|)
+    const Rn invWidth = d == 0 ? Rn(rcpN(rd.z * L.dxi0)) : Rn(rd.y) * a.normal[d] * invVolume * invH * Rn(rcpN(a.det[d]));
+    const Rn wave = sqrtN(mad(alfven, b2, L.gamma * pressure * invRho));
+    rate = mad(wave + sqrtN(v2), invWidth, rate);
   }
-  return inverseDt;
+  return rate;
 }
 
 // Max over a warp (std::max order: a NaN candidate never replaces the max),
@@ -329,35 +337,48 @@ __device__ __forceinline__ void warpMaxAtomic(double v, unsigned long long* out)
   if ((threadIdx.x & 31) == 0 && v > 0) atomicMax(out, (unsigned long long)__double_as_longlong(v));
 }
 
-template <class TL, int DIR, int LIM, bool ROE, int MODE>
-__device__ __forceinline__ void o2FaceLoop(const StageArgs& a, const double* __restrict__ w, int block, int oi,
-                                           int oj, int ok, int v0, int v1, int v2, double* sF, int base,
-                                           bool powell) {
-  constexpr int TX = TL::TX, TY = TL::TY, TZ = TL::TZ, NT = TL::NT, NF = TL::NF;
-  constexpr int EX = TX + (DIR == 0), EY = TY + (DIR == 1), EZ = TZ + (DIR == 2);
-  constexpr int NFD = EX * EY * EZ;
-  for (int f = threadIdx.x; f < NFD; f += NT) {
-    const int fi = f % EX, fj = (f / EX) % EY, fk = f / (EX * EY);
-    const int i = oi + fi, j = oj + fj, k = ok + fk;
-    const bool valid = i <= a.hi[0] + (DIR == 0) && j <= a.hi[1] + (DIR == 1) && k <= a.hi[2] + (DIR == 2);
+// The faces of a tile as warp tasks: each direction's faces in groups of 32,
+// the groups dealt to the warps in turn, so every warp has as many (16 tasks
+// on 4 warps for the 16 x 4 x 2 tile; with a loop over all threads per
+// direction, 136, 160 and 192 faces on 128 threads gave the first warp six
+// passes and the last three before the barrier).  The direction is a run-time
+// stride: one copy of the face code.
+template <class TL, int LIM, bool ROE, int MODE>
+__device__ __forceinline__ void o2Faces(const StageArgs& a, const double* __restrict__ w, int block, int oi, int oj,
+                                        int ok, int v0, int v1, int v2, double* sF, bool powell) {
+  constexpr int TX = TL::TX, TY = TL::TY, NF = TL::NF, NF0 = TL::NF0, NF1 = TL::NF1, NF2 = TL::NF2;
+  constexpr int G0 = (NF0 + 31) / 32, G1 = (NF1 + 31) / 32, G2 = (NF2 + 31) / 32;
+#pragma unroll 1
+  for (int task = threadIdx.x / 32; task < G0 + G1 + G2; task += TL::NT / 32) {
+    const int dir = task < G0 ? 0 : task < G0 + G1 ? 1 : 2;
+    const int f = (task - (dir == 0 ? 0 : dir == 1 ? G0 : G0 + G1)) * 32 + (threadIdx.x & 31);
+    const int ex = TX + (dir == 0), ey = TY + (dir == 1);
+    if (f >= (dir == 0 ? NF0 : dir == 1 ? NF1 : NF2)) continue;
+    const int fy = dir == 0 ? f / (TX + 1) : f / TX, fk = dir == 1 ? fy / (TY + 1) : fy / TY;
+    const int i = oi + (f - fy * ex), j = oj + (fy - fk * ey), k = ok + fk;
+    const bool valid = i <= a.hi[0] + (dir == 0) && j <= a.hi[1] + (dir == 1) && k <= a.hi[2] + (dir == 2);
     double out[8];
     double bf = 0;
     if (valid) {
-      o2Face<LIM, ROE, MODE>(a, w, block, DIR, i, j, k, out, bf, powell);
-      if (MODE == MODE_BOX && a.flux[DIR]) {
-        const int f0 = v0 + (DIR == 0), f1 = v1 + (DIR == 1), f2 = v2 + (DIR == 2);
-        const long fidx = (long)(i - a.lo[0]) + (long)f0 * ((long)(j - a.lo[1]) + (long)f1 * (k - a.lo[2]));
-        const long fN = (long)f0 * f1 * f2;
+      o2Face<LIM, ROE, MODE>(a, w, block, dir, i, j, k, out, bf, powell);
+      if (MODE == MODE_BOX) {
+        double* flux = dir == 0 ? a.flux[0] : dir == 1 ? a.flux[1] : a.flux[2];
+        if (flux) {
+          const int f0 = v0 + (dir == 0), f1 = v1 + (dir == 1), f2 = v2 + (dir == 2);
+          const long fidx = (long)(i - a.lo[0]) + (long)f0 * ((long)(j - a.lo[1]) + (long)f1 * (k - a.lo[2]));
+          const long fN = (long)f0 * f1 * f2;
 #pragma unroll
-        for (int q = 0; q < NC; ++q) a.flux[DIR][q * fN + fidx] = out[q];
+          for (int q = 0; q < NC; ++q) flux[q * fN + fidx] = out[q];
+        }
       }
     } else {
 #pragma unroll
       for (int q = 0; q < NC; ++q) out[q] = 0;
     }
+    double* dst = sF + (dir == 0 ? 0 : dir == 1 ? NF0 : NF0 + NF1) + f;
 #pragma unroll
-    for (int q = 0; q < NC; ++q) sF[q * NF + base + f] = out[q];
-    sF[8 * NF + base + f] = bf;
+    for (int q = 0; q < NC; ++q) dst[q * NF] = out[q];
+    dst[8 * NF] = bf;
   }
 }
 
@@ -378,9 +399,7 @@ __global__ void __launch_bounds__(TL::NT, TL::minBlocks(ROE))
   const int oi = a.lo[0] + bx * TX, oj = a.lo[1] + by * TY, ok = a.lo[2] + bz * TZ;
   const double* __restrict__ w = a.w + (long)box * a.wBoxStride;
 
-  o2FaceLoop<TL, 0, LIM, ROE, MODE>(a, w, block, oi, oj, ok, v0, v1, v2, sF, 0, powell != 0);
-  o2FaceLoop<TL, 1, LIM, ROE, MODE>(a, w, block, oi, oj, ok, v0, v1, v2, sF, NF0, powell != 0);
-  o2FaceLoop<TL, 2, LIM, ROE, MODE>(a, w, block, oi, oj, ok, v0, v1, v2, sF, NF0 + NF1, powell != 0);
+  o2Faces<TL, LIM, ROE, MODE>(a, w, block, oi, oj, ok, v0, v1, v2, sF, powell != 0);
   __syncthreads();
 
   const int li = threadIdx.x % TX, lj = (threadIdx.x / TX) % TY, lk = threadIdx.x / (TX * TY);
@@ -422,8 +441,9 @@ __global__ void __launch_bounds__(TL::NT, TL::minBlocks(ROE))
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
 #pragma unroll
-      for (int q = 0; q < NC; ++q) kv[q] += coef[d] * (sF[q * NF + fl[d] + fs[d]] - sF[q * NF + fl[d]]);
-      if (powell) md += coef[d] * (sF[8 * NF + fl[d] + fs[d]] - sF[8 * NF + fl[d]]);
+      for (int q = 0; q < NC; ++q)
+        kv[q] = mad(coef[d], Rn(sF[q * NF + fl[d] + fs[d]]) - sF[q * NF + fl[d]], kv[q]);
+      if (powell) md = mad(coef[d], Rn(sF[8 * NF + fl[d] + fs[d]]) - sF[8 * NF + fl[d]], md);
     }
     if (powell) {
       // src/BoxOp_SecondOrder.H:351-369
@@ -431,11 +451,11 @@ __global__ void __launch_bounds__(TL::NT, TL::minBlocks(ROE))
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
         const double b = __ldg(w + (5 + d) * a.wN + cw), vel = __ldg(w + (1 + d) * a.wN + cw);
-        kv[1 + d] += md * b / (4 * kPi);
-        kv[5 + d] += md * vel;
-        vb += vel * b;
+        kv[1 + d] = mad(md * (0.25 / kPi), b, kv[1 + d]);
+        kv[5 + d] = mad(md, vel, kv[5 + d]);
+        vb = mad(vel, b, vb);
       }
-      kv[4] += md * vb / (4 * kPi);
+      kv[4] = mad(md * (0.25 / kPi), vb, kv[4]);
     }
     if (MODE == MODE_BOX) {
 #pragma unroll
@@ -458,15 +478,15 @@ __global__ void __launch_bounds__(TL::NT, TL::minBlocks(ROE))
         for (int q = 0; q < NC; ++q) {
           const double u0 = a.ju[vidx + q * N];
           const double ac = a.stage == 0 ? u0 : a.acc[vidx + q * N];
-          a.acc[vidx + q * N] = ac + fb * kv[q];
-          u[q] = u0 + fa * kv[q];
+          a.acc[vidx + q * N] = mad(fb, kv[q], ac);
+          u[q] = mad(fa, kv[q], u0);
         }
       } else {
         const double fb = dt * b4[3];
         bool bad = false;
 #pragma unroll
         for (int q = 0; q < NC; ++q) {
-          u[q] = a.acc[vidx + q * N] + fb * kv[q];
+          u[q] = mad(fb, kv[q], a.acc[vidx + q * N]);
           a.ju[vidx + q * N] = u[q];
           bad = bad || !isfinite(u[q]) || (q == 0 && !(u[q] > 0));
         }
@@ -479,7 +499,7 @@ __global__ void __launch_bounds__(TL::NT, TL::minBlocks(ROE))
       }
       // src/BoxOp_SecondOrderPreStage.H:46-54: JU/J -> Cartesian primitives.
       double wv[8];
-      const double invJ = 1.0 / (L.radial[i + L.g].w * L.grav[((size_t)block * L.na + k) * L.na + j].det);
+      const double invJ = rcpN(L.radial[i + L.g].w * L.grav[((size_t)block * L.na + k) * L.na + j].det);
       cartesianPrimitiveFromConserved(wv, u, invJ, L.gamma);
       double* wo = a.wOut + (long)box * a.wBoxStride + cw;
 #pragma unroll
@@ -505,7 +525,7 @@ __global__ void primValidKernel(const DevLevel L, const double* __restrict__ ju,
     const double* src = ju + (long)b * NC * L.Nv + r;
 #pragma unroll
     for (int c = 0; c < NC; ++c) in[c] = src[c * L.Nv];
-    const double invJ = 1.0 / (L.radial[i + L.g].w * L.grav[((size_t)b * L.na + k) * L.na + j].det);
+    const double invJ = rcpN(L.radial[i + L.g].w * L.grav[((size_t)b * L.na + k) * L.na + j].det);
     cartesianPrimitiveFromConserved(out, in, invJ, L.gamma);
     double* dst = w + (long)b * NC * L.Ng + (long)(i + L.g) + (long)L.n0 * ((long)(j + L.g) + (long)L.n1 * (k + L.g));
 #pragma unroll
