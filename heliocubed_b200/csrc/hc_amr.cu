@@ -1132,7 +1132,7 @@ __global__ void __launch_bounds__(kThreads, 2) nativeBoxKernel(const hc::O4Level
     } else {
       native(O.nr - 1, u);
       const double rl = O.radial[O.nr - 1 + O.g + 1].y, rr = O.radial[i + O.g + 1].y;
-      const double s2 = pow(rl / rr, 2.0), s1 = pow(rl / rr, 1.0);
+      const double s1 = rl / rr, s2 = s1 * s1;
 #pragma unroll
       for (int c = 0; c < 8; ++c) u[c] *= c < 6 ? s2 : s1;
     }

@@ -60,7 +60,7 @@ __device__ __forceinline__ long roff(const Reg& r, int i, int j, int k) {
 // products that of the left states, which nothing reads any more by then.
 enum FaceArr { F_FS = 0, F_PS = 7, F_FX = 0, F_QD = 8, F_L = 16, F_R = 24, F_X = 16, F_T3 = 23, F_THF = 32, F_BP = 33,
                F_SPD = 34, F_BF = 35 };
-static_assert(F_BF + 1 == kO4FaceArrays, "face arrays");
+static_assert(F_BF + 1 == kO4FaceArrays && F_T3 == F_X + 7, "face arrays");
 // F_FS array of component c in (rho, m_n, m_1, m_2, E, B_n, B_1, B_2) order (c != 5), also of F_X.
 __host__ __device__ constexpr int fluxSlot(int c) { return c < 5 ? c : c - 1; }
 
@@ -94,11 +94,22 @@ constexpr int kAvgPoints = 126;
 __host__ __device__ constexpr int passPoints(int id) { return id == RG_PB ? kAvgPoints : 128; }
 
 // One CTA's work: flat points begin .. end - 1 of one region of box `box`,
-// direction `dir`.
+// direction `dir`; with march > 0 its points are columns of that many faces.
 struct WorkChunk {
-  int box, dir;
+  int box, dir, march;
   long begin, end;
 };
+
+// The face averages and final fluxes march along an angular direction
+// transverse to the faces (k, or j for the faces of k): a thread takes
+// `march` faces and keeps the values of the row behind and of its row in
+// registers, so a row is read from L2 once and not once per neighbour.
+__host__ __device__ constexpr bool marches(int id) { return id == RG_PB || id == RG_V0; }
+__host__ __device__ constexpr int marchDim(int d) { return d == 2 ? 1 : 2; }
+__host__ __device__ inline long columns(const Box3& b, int d, int march) {
+  const int t = marchDim(d);
+  return (long)b.n(0) * b.n(3 - t) * ((b.n(t) + march - 1) / march);
+}
 // Points per CTA of a work list: its total points over about 148 x 16 CTAs,
 // rounded up to whole passes of the CTA and held within 1 to 16 passes, so
 // one launch has as many CTAs whatever the box sizes.
@@ -170,23 +181,23 @@ __device__ __forceinline__ double radialPoint(const O4Geo& g, int d, int i) {
 constexpr double kInv4Pi = 0.25 / kPi, kInv8Pi = 0.125 / kPi;
 // f_sphToPrim + energies + pressure (src/BoxOp_BertaCubedSphereImplem.H:212-340)
 __device__ __forceinline__ void sphToPrim(const double u[8], const double* A, double gamma, double w[8]) {
-  w[0] = dmax(u[0], kRHO00);
-  w[1] = u[1] / w[0];
-  w[2] = u[2] / w[0];
-  w[3] = u[3] / w[0];
-  w[4] = u[4];
-  w[5] = u[5]; w[6] = u[6]; w[7] = u[7];
-  double ke = 0., me = 0.;
+  const Rn rho = dmax(u[0], kRHO00), inv = rcpN(rho);
+  w[0] = rho;
+  Rn ke = 0.0, me = 0.0;
 #pragma unroll
-  for (int d0 = 0; d0 < 3; ++d0) {
-    const double vc = A[3 * d0] * w[1] + A[3 * d0 + 1] * w[2] + A[3 * d0 + 2] * w[3];
-    const double bc = A[3 * d0] * w[5] + A[3 * d0 + 1] * w[6] + A[3 * d0 + 2] * w[7];
-    ke += vc * vc / 2;
-    me += bc * bc * kInv8Pi;
+  for (int e = 0; e < 3; ++e) {
+    w[1 + e] = inv * u[1 + e];
+    w[5 + e] = u[5 + e];
   }
-  ke *= w[0];
-  w[4] = (w[4] - ke - me) * (gamma - 1.0);
-  if (w[4] < 0.0) w[4] = 0.0;
+#pragma unroll
+  for (int e = 0; e < 3; ++e) {
+    const Rn v = dot3(A[3 * e], w[1], A[3 * e + 1], w[2], A[3 * e + 2], w[3]);
+    const Rn b = dot3(A[3 * e], w[5], A[3 * e + 1], w[6], A[3 * e + 2], w[7]);
+    ke = mad(v, v, ke);
+    me = mad(b, b, me);
+  }
+  const Rn p = (mad(-0.5 * rho, ke, u[4]) - kInv8Pi * me) * (gamma - 1.0);
+  w[4] = p < 0.0 ? 0.0 : p.v;
 }
 
 // bertaNormalizeWenoStencil (:747-773)
@@ -363,6 +374,20 @@ __device__ __forceinline__ void pointOf(const Box3& b, int walk, unsigned t, int
   k = b.lo[2] + (int)col;
 }
 
+// Column u of region b for faces of direction d: its first point, and the
+// number of faces.
+__device__ __forceinline__ int columnOf(const Box3& b, int d, int march, unsigned u, int p[3]) {
+  const bool alongK = marchDim(d) == 2;
+  const unsigned n0 = (unsigned)b.n(0), no = (unsigned)b.n(alongK ? 1 : 2);
+  const unsigned q = u / n0, seg = q / no;
+  p[0] = b.lo[0] + (int)(u - q * n0);
+  const int other = b.lo[alongK ? 1 : 2] + (int)(q - seg * no), first = b.lo[alongK ? 2 : 1] + (int)seg * march;
+  p[1] = alongK ? other : first;
+  p[2] = alongK ? first : other;
+  const int left = b.hi[alongK ? 2 : 1] - first + 1;
+  return left < march ? left : march;
+}
+
 // Thread -> (i, j, k) over the chunk's points of region b of the chunk's box.
 template <class F>
 __device__ __forceinline__ void forRegion(const Box3& b, int walk, const WorkChunk& w, F f) {
@@ -397,37 +422,39 @@ __global__ void o4PrimAvgKernel(const Ctx* __restrict__ tab, const RegArgs rg, c
   });
 }
 
-__device__ __forceinline__ double magp(const double* W, long N, long o) {
-  const double bx = W[5 * N + o], by = W[6 * N + o], bz = W[7 * N + o];
-  return 0.5 * (bx * bx + by * by + bz * bz);
-}
-__device__ __forceinline__ double eta1(double qm, double q0, double qp) {
-  const double num = fabs(qp - 2.0 * q0 + qm);
-  const double den = fabs(qp) + 2.0 * fabs(q0) + fabs(qm) + 1.0e-40;
-  return num / den;
-}
-
-// 2. raw Jameson flag on G.grow(-1) (:347-402).
-__global__ void o4ThetaRawKernel(const Ctx* __restrict__ tab, const RegArgs rg, const WorkChunk* __restrict__ wk) {
+// 2. raw Jameson flag on G.grow(-1) (:347-402): per direction the largest of
+// three curvatures |q+ - 2 q + q-| / (|q+| + 2 |q| + |q-| + 1e-40) of the
+// density, the pressure and the magnetic pressure.  The scales are far from
+// the ends of the range of doubles except where a field vanishes; there the
+// sum is 1e-40, whose reciprocal is exact enough.
+__global__ void __launch_bounds__(128) o4ThetaRawKernel(const Ctx* __restrict__ tab, const RegArgs rg, const WorkChunk* __restrict__ wk) {
   const WorkChunk wc = wk[blockIdx.x];
   const Ctx& c = tab[wc.box * 3 + 0];
   const O4Args& a = c.a;
+  const long N = c.gr.N;
+  const int st[3] = {1, c.gr.n[0], c.gr.n[0] * c.gr.n[1]};
+  auto magp = [&](const double* W) -> Rn {
+    const double bx = __ldg(W + 5 * N), by = __ldg(W + 6 * N), bz = __ldg(W + 7 * N);
+    return 0.5 * dot3(bx, bx, by, by, bz, bz);
+  };
+  auto eta = [](Rn m, Rn q, Rn p) -> Rn {
+    const Rn num = fabs(mad(-2.0, q, p + m).v);
+    return num * rcpN(mad(2.0, fabs(q.v), Rn(fabs(p.v)) + fabs(m.v)) + 1.0e-40);
+  };
   forRegion(c.GR, WALK_JK, wc, [&](int i, int j, int k) {
-    const double* W = a.WA;
-    const long N = c.gr.N, o = roff(c.gr, i, j, k);
-    double et[3];
+    const long o = roff(c.gr, i, j, k);
+    const double* W = a.WA + o;
+    const Rn r0 = __ldg(W), p0 = __ldg(W + 4 * N), m0 = magp(W);
+    Rn sum = 0.0;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      int m[3] = {i, j, k}, p[3] = {i, j, k};
-      m[d] -= 1; p[d] += 1;
-      const long om = roff(c.gr, m[0], m[1], m[2]), op = roff(c.gr, p[0], p[1], p[2]);
-      const double er = eta1(W[om], W[o], W[op]);
-      const double ep = eta1(W[4 * N + om], W[4 * N + o], W[4 * N + op]);
-      const double em = eta1(magp(W, N, om), magp(W, N, o), magp(W, N, op));
-      et[d] = dmax(er, dmax(ep, em));
+      const double *lo = W - st[d], *hi = W + st[d];
+      const double er = eta(__ldg(lo), r0, __ldg(hi)), ep = eta(__ldg(lo + 4 * N), p0, __ldg(hi + 4 * N)),
+                   em = eta(magp(lo), m0, magp(hi));
+      const Rn et = dmax(er, dmax(ep, em));
+      sum = mad(et, et, sum);
     }
-    const double eta = sqrt(et[0] * et[0] + et[1] * et[1] + et[2] * et[2]);
-    a.thr[o] = eta < a.G.eta_d ? 1.0 : 0.0;
+    a.thr[o] = sqrt(sum.v) < a.G.eta_d ? 1.0 : 0.0;
   });
 }
 
@@ -495,9 +522,9 @@ __device__ __forceinline__ int place(int q, int d) {
 // One thread per face, one launch for the three directions.  The kernel
 // holds two components at a time: with the Riemann solver in the same kernel
 // it took 128 registers, and 16 warps an SM are too few for the latency of
-// the FP64 chains (64 x 32^2 x 6, three directions: 325 us against NN + NN).
-// Pairs of components in a loop: all eight unrolled overflow the
-// instruction cache.
+// the FP64 chains (64 x 32^2 x 6, three directions: 325 us against 163 + 130).
+// Pairs of components in a loop: all eight unrolled overflow the instruction
+// cache (225 us), one at a time costs the registers' rotation (229 us).
 template <int MB>
 __global__ void __launch_bounds__(128, MB) o4FaceReconKernel(const Ctx* __restrict__ tab, const RegArgs rg, const WorkChunk* __restrict__ wk) {
   const WorkChunk wc = wk[blockIdx.x];
@@ -728,60 +755,72 @@ __global__ void __launch_bounds__(128, MB) o4FaceRiemannKernel(const Ctx* __rest
 // the metric factors of the mapping do not vary radially, so the two
 // commute, and the mapping then takes flux and dissipation together.
 //
-// One thread per face.  The radial neighbours' averages are the
+// One thread per column of faces.  The radial neighbours' averages are the
 // neighbouring threads' (shared memory; the first and last thread of the
-// CTA only serve as neighbours).  HBM-bound: nine arrays read with four
-// neighbours each through L1, eight written.
-__global__ void __launch_bounds__(128, 8) o4FaceAvgKernel(const Ctx* __restrict__ tab, const RegArgs rg, const WorkChunk* __restrict__ wk) {
-  __shared__ double sh[8][128];
+// CTA only serve as neighbours).  Bound by the latency of L2: 64^3, three
+// directions, 182 us marching against 257 with a thread per face, which read
+// every transverse row again for each neighbour (L1 held none of them).
+__global__ void __launch_bounds__(128, 6) o4FaceAvgKernel(const Ctx* __restrict__ tab, const RegArgs rg, const WorkChunk* __restrict__ wk) {
+  __shared__ double sh[2][8][128];
   const WorkChunk wc = wk[blockIdx.x];
   const int d = wc.dir, tid = threadIdx.x;
   const Ctx& c = tab[wc.box * 3 + d];
   const O4Geo& G = c.a.G;
   const Box3 PB = regionOf(c, RG_PB);
   const long NF = c.fr.N;
-  const int2 tr = transverse(c.fr, d);
-  const int n = PB.n(0) * PB.n(1) * PB.n(2);
-  for (long at = wc.begin; at < wc.end; at += kAvgPoints) {
-    const int t = (int)at + tid - 1;
-    const bool in = t >= 0 && t < n;
+  // strides of the marching and of the other transverse direction
+  const int st = stride(c.fr, marchDim(d)), so = d == 0 ? stride(c.fr, 1) : 1;
+  const long u = wc.begin + tid - 1;
+  const bool in = u >= 0 && u < columns(PB, d, wc.march);
+  int p[3] = {0, 0, 0};
+  const int steps = in ? columnOf(PB, d, wc.march, (unsigned)u, p) : 0;
+  const int i = p[0];
+  // outputs: the CTA's inner threads, below the chunk's end, radially on final faces
+  const bool mine = in && tid >= 1 && tid <= kAvgPoints && u < wc.end && i >= c.V0.lo[0] && i <= c.V0.hi[0];
+  double* base = in ? faceArr(c, 0) + roff(c.fr, p[0], p[1], p[2]) : nullptr;
+  const Rn s = adjDr(G, d, i), ds = (Rn(adjDr(G, d, i + 1)) - adjDr(G, d, i - 1)) * (1.0 / 48.0);
+  // the pressure sum follows the seven flux sums
+  double fm[8], f0[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    fm[e] = in ? __ldg(base + (F_FS + e) * NF - st) : 0.0;
+    f0[e] = in ? __ldg(base + (F_FS + e) * NF) : 0.0;
+  }
+#pragma unroll 1
+  for (int step = 0; step < wc.march; ++step) {
     Rn fa[8];
-    int i = 0;
-    double* base = nullptr;
-    if (in) {
-      int j, k;
-      pointOf(PB, d == 0 ? WALK_JK : d == 1 ? WALK_K : WALK_J, (unsigned)t, i, j, k);
-      base = faceArr(c, 0) + roff(c.fr, i, j, k);
-      const double w = base[F_THF * NF] > 0.5 ? 1.0 / 24.0 : 0.0;
-      // the pressure sum follows the seven flux sums
+    if (step < steps) {
+      const bool sm = __ldg(base + F_THF * NF) > 0.5;
+      double fp[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) fp[e] = __ldg(base + (F_FS + e) * NF + st);
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         const double* F = base + (F_FS + e) * NF;
-        const Rn pt = __ldg(F);
-        const Rn lap = mad(-4.0, pt, (Rn(__ldg(F - tr.x)) + __ldg(F + tr.x)) + (Rn(__ldg(F - tr.y)) + __ldg(F + tr.y)));
-        fa[e] = w != 0.0 ? mad(lap, w, pt) : pt;
+        const Rn pt = f0[e], march = Rn(fm[e]) + fp[e], other = Rn(__ldg(F - so)) + __ldg(F + so);
+        const Rn lap = mad(-4.0, pt, other + march);
+        fa[e] = sm ? mad(lap, 1.0 / 24.0, pt) : pt;
+        fm[e] = f0[e];
+        f0[e] = fp[e];
       }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) fa[e] = 0.0;
     }
     if (d != 0) {
+      double (*row)[128] = sh[step & 1];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) sh[e][tid] = fa[e];
+      for (int e = 0; e < 8; ++e) row[e][tid] = fa[e];
       __syncthreads();
-    }
-    // outputs: the CTA's inner threads, below the chunk's end, radially on final faces
-    if (in && tid >= 1 && tid <= kAvgPoints && t < wc.end && i >= c.V0.lo[0] && i <= c.V0.hi[0]) {
-      const Rn s = adjDr(G, d, i);
-      if (d != 0) {
-        const Rn ds = (Rn(adjDr(G, d, i + 1)) - adjDr(G, d, i - 1)) * (1.0 / 48.0);
+      if (mine && step < steps) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) fa[e] = mad(Rn(sh[e][tid + 1]) - sh[e][tid - 1], ds, s * fa[e]);
-      } else {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) fa[e] = s * fa[e];
+        for (int e = 0; e < 8; ++e) base[(F_X + e) * NF] = mad(Rn(row[e][tid + 1]) - row[e][tid - 1], ds, s * fa[e]);
       }
+    } else if (mine && step < steps) {
 #pragma unroll
-      for (int e = 0; e < 8; ++e) base[(F_X + e) * NF] = fa[e];
+      for (int e = 0; e < 8; ++e) base[(F_X + e) * NF] = s * fa[e];
     }
-    if (d != 0) __syncthreads();
+    base += st;
   }
 }
 
@@ -794,109 +833,136 @@ __global__ void __launch_bounds__(128, 8) o4FaceAvgKernel(const Ctx* __restrict_
 // 1 and 2 have one transverse product and direction 0 two.  The record
 // holds the halved M, det and normal and their angular differences / 48.
 //
-// One thread per face, no walk and no barrier: about 90 loads (five taps of
-// 15 arrays, the record) through L1.  The walk over face slabs staged by TMA
-// that this replaces ran at 10-20 % of the warp slots between its barriers
-// (66-80 KB of shared memory and 128 registers a CTA).
-template <int D0, class Load>
-__device__ __forceinline__ void finalFlux(const double* __restrict__ M, Load load, const double* __restrict__ T3, long ta, long tb, Rn fx[8]) {
-  // components in two vector groups and the two scalars
-  {
-    Rn z, ya, yb;
-    load(0, z, ya, yb);
-    fx[0] = mad(M[9], z, Rn(M[22]) * ya);
-    if (D0) fx[0] = mad(M[35], yb, fx[0]);
-    load(4, z, ya, yb);
-    fx[4] = mad(M[9], z, Rn(M[22]) * ya);
-    if (D0) fx[4] = mad(M[35], yb, fx[4]);
+// One thread per column of faces, no barrier.  Bound by the latency of L2:
+// 64^3, three directions, 398 us marching against 475 with a thread per face
+// (about 75 taps; three component groups in separate CTAs, which raised the
+// warps from 12 to 32 an SM, were slower, 2.2 times the instructions, and so
+// was taking the other direction's taps through shared memory, 467 us).  The walk over face slabs staged by TMA that this and
+// the averages replace ran at 10-20 % of the warp slots between its barriers
+// (833 us).
+template <bool D0>
+__device__ __forceinline__ void finalColumn(const Ctx& c, const RegArgs& rg, const Box3& V0, int d, int march, unsigned u) {
+  const O4Args& a = c.a;
+  const bool roe = roeNow(a.G);
+  const long NF = c.fr.N;
+  int p[3];
+  const int steps = columnOf(V0, d, march, u, p), t = marchDim(d);
+  const int st = stride(c.fr, t), so = D0 ? stride(c.fr, 1) : 1;
+  double* base = faceArr(c, 0) + roff(c.fr, p[0], p[1], p[2]);
+  const long row = t == 2 ? a.G.na + 2 * a.G.ext + 1 : 1;  // record step along the march
+  const double* M = faceRec(a.G, a.block0, d, p[1], p[2]);
+  // seam register and caller's flux
+  const Reg r0 = regOf(V0);
+  double* const reg = a.seamReg ? a.seamReg : rg.reg;
+  const long nrna = (long)a.G.na * a.G.nr;
+  // row behind and row of the march: area products X (7) and T3, dissipation Q
+  double xm[8], x0[8], qm[8], q0[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const double *X = base + (F_X + e) * NF, *Q = base + (F_QD + e) * NF;
+    xm[e] = __ldg(X - st);
+    x0[e] = __ldg(X);
+    qm[e] = __ldg(Q - st);
+    q0[e] = __ldg(Q);
   }
+#pragma unroll 1
+  for (int step = 0; step < steps; ++step) {
+    const bool sm = __ldg(base + F_THF * NF) > 0.5;
+    const double sigma = roe ? 1.0 : __ldg(base + F_SPD * NF);
+    double xp[8], qp[8];
 #pragma unroll
-  for (int grp = 0; grp < 2; ++grp) {
-    const int b = grp == 0 ? 1 : 5;
-    Rn out[3];
-#pragma unroll
-    for (int e = 0; e < 3; ++e) {
-      Rn z, ya, yb;
-      load(b + e, z, ya, yb);
-#pragma unroll
-      for (int row = 0; row < 3; ++row) {
-        const Rn first = e == 0 ? Rn(M[3 * row]) * z : mad(M[3 * row + e], z, out[row]);
-        out[row] = mad(M[13 + 3 * row + e], ya, first);
-        if (D0) out[row] = mad(M[26 + 3 * row + e], yb, out[row]);
+    for (int e = 0; e < 8; ++e) {
+      xp[e] = __ldg(base + (F_X + e) * NF + st);
+      qp[e] = __ldg(base + (F_QD + e) * NF + st);
+    }
+    // Z and the transverse differences of Y of place q: along the march (m)
+    // and, for direction 0, along j (o)
+    auto load = [&](int q, Rn& z, Rn& ym, Rn& yo) {
+      const double* Q = base + (F_QD + q) * NF;
+      const Rn pt = q0[q], lo = __ldg(Q - so), hi = __ldg(Q + so);
+      const Rn lap = mad(-4.0, pt, (lo + hi) + (Rn(qm[q]) + qp[q]));
+      z = -(sigma * (sm ? mad(lap, 1.0 / 24.0, pt) : pt));
+      ym = 0.0;
+      yo = 0.0;
+      if (q != 5) {  // the normal field has no flux
+        const int e = fluxSlot(q);
+        z = z + x0[e];
+        ym = Rn(xp[e]) - xm[e];
+        if (D0) yo = Rn(__ldg(base + (F_X + e) * NF + so)) - __ldg(base + (F_X + e) * NF - so);
       }
+      if (roe) {
+        ym = ym - (Rn(qp[q]) - qm[q]);
+        if (D0) yo = yo - (hi - lo);
+      }
+    };
+    // record places: the differences along j come first for direction 0
+    constexpr int dm = D0 ? 26 : 13, dj = 13;
+    Rn fx[8];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      Rn z, ym, yo;
+      load(4 * e, z, ym, yo);
+      fx[4 * e] = mad(__ldg(M + 9), z, Rn(__ldg(M + dm + 9)) * ym);
+      if (D0) fx[4 * e] = mad(__ldg(M + dj + 9), yo, fx[4 * e]);
     }
 #pragma unroll
-    for (int row = 0; row < 3; ++row) fx[b + row] = out[row];
-  }
-  const Rn p = __ldg(T3), pa = Rn(__ldg(T3 + ta)) - __ldg(T3 - ta);
-  const Rn pb = D0 ? Rn(__ldg(T3 + tb)) - __ldg(T3 - tb) : Rn(0.0);
+    for (int b = 1; b < 8; b += 4)
 #pragma unroll
-  for (int row = 0; row < 3; ++row) {
-    fx[1 + row] = fx[1 + row] + mad(M[10 + row], p, Rn(M[23 + row]) * pa);
-    if (D0) fx[1 + row] = mad(M[36 + row], pb, fx[1 + row]);
+      for (int e = 0; e < 3; ++e) {
+        Rn z, ym, yo;
+        load(b + e, z, ym, yo);
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+          const Rn first = e == 0 ? Rn(__ldg(M + 3 * r)) * z : mad(__ldg(M + 3 * r + e), z, fx[b + r]);
+          fx[b + r] = mad(__ldg(M + dm + 3 * r + e), ym, first);
+          if (D0) fx[b + r] = mad(__ldg(M + dj + 3 * r + e), yo, fx[b + r]);
+        }
+      }
+    // pressure force
+    const Rn pm = Rn(xp[7]) - xm[7];
+    const Rn po = D0 ? Rn(__ldg(base + F_T3 * NF + so)) - __ldg(base + F_T3 * NF - so) : Rn(0.0);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      fx[1 + r] = fx[1 + r] + mad(__ldg(M + 10 + r), x0[7], Rn(__ldg(M + dm + 10 + r)) * pm);
+      if (D0) fx[1 + r] = mad(__ldg(M + dj + 10 + r), po, fx[1 + r]);
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      base[(F_FX + q) * NF] = fx[q];
+      xm[q] = x0[q];
+      x0[q] = xp[q];
+      qm[q] = q0[q];
+      q0[q] = qp[q];
+    }
+    if (a.flux[d]) {
+      double* out = a.flux[d] + roff(r0, p[0], p[1], p[2]);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) out[q * r0.N] = fx[q];
+    }
+    if (!D0 && reg) {
+      const int f = d == 1 ? p[1] : p[2];
+      if (f == 0 || f == a.G.na) {
+        const double w = a.seamReg ? rg.w * (a.seamCfl / *a.seamInvMax) : rg.wDev ? rg.w * (rg.cfl / *rg.wDev) : rg.w;
+        double* S = reg + (((long)a.block0 * 2 + (d - 1)) * 2 + (f == 0 ? 0 : 1)) * 8 * nrna +
+                    (long)(d == 1 ? p[2] : p[1]) * a.G.nr + p[0];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) S[q * nrna] = mad(w, fx[q], S[q * nrna]);
+      }
+    }
+    base += st;
+    M += row * (D0 ? kO4FaceRec0 : kO4FaceRec12);
+    if (t == 2) ++p[2]; else ++p[1];
   }
 }
 
 template <int MB>
 __global__ void __launch_bounds__(128, MB) o4FaceFinalKernel(const Ctx* __restrict__ tab, const RegArgs rg, const WorkChunk* __restrict__ wk) {
   const WorkChunk wc = wk[blockIdx.x];
-  const int d = wc.dir;
-  const Ctx& c = tab[wc.box * 3 + d];
-  const O4Args& a = c.a;
-  const bool roe = roeNow(a.G);
-  const long NF = c.fr.N;
-  const int2 tr = transverse(c.fr, d);
-  forRegion(c.V0, d == 0 ? WALK_JK : d == 1 ? WALK_K : WALK_J, wc, [&](int i, int j, int k) {
-    double* const base = faceArr(c, 0) + roff(c.fr, i, j, k);
-    const double* M = faceRec(a.G, a.block0, d, j, k);
-    const bool sm = base[F_THF * NF] > 0.5;
-    const double sigma = roe ? 1.0 : base[F_SPD * NF];
-    // first angular transverse direction: j for d = 0, the only one otherwise
-    const int ta = d == 0 ? tr.x : tr.y, tb = tr.y;
-    auto load = [&](int q, Rn& z, Rn& ya, Rn& yb) {
-      const double* Q = base + (F_QD + q) * NF;
-      const Rn pt = __ldg(Q), a1 = __ldg(Q - tr.x), b1 = __ldg(Q + tr.x), a2 = __ldg(Q - tr.y), b2 = __ldg(Q + tr.y);
-      const Rn avg = sm ? mad(mad(-4.0, pt, (a1 + b1) + (a2 + b2)), 1.0 / 24.0, pt) : pt;
-      const Rn q1 = b1 - a1, q2 = b2 - a2;
-      z = -(sigma * avg);
-      ya = 0.0;
-      yb = 0.0;
-      if (q != 5) {  // the normal field has no flux
-        const double* X = base + (F_X + fluxSlot(q)) * NF;
-        z = z + __ldg(X);
-        ya = Rn(__ldg(X + ta)) - __ldg(X - ta);
-        if (d == 0) yb = Rn(__ldg(X + tb)) - __ldg(X - tb);
-      }
-      if (roe) {
-        ya = ya - (d == 0 ? q1 : q2);
-        if (d == 0) yb = yb - q2;
-      }
-    };
-    Rn fx[8];
-    if (d == 0) finalFlux<1>(M, load, base + F_T3 * NF, ta, tb, fx);
-    else finalFlux<0>(M, load, base + F_T3 * NF, ta, tb, fx);
-#pragma unroll
-    for (int q = 0; q < 8; ++q) base[(F_FX + q) * NF] = fx[q];
-    // the caller's flux and the seam register
-    if (a.flux[d]) {
-      const Reg r0 = regOf(c.V0);
-      double* out = a.flux[d] + roff(r0, i, j, k);
-#pragma unroll
-      for (int q = 0; q < 8; ++q) out[q * r0.N] = fx[q];
-    }
-    double* const reg = a.seamReg ? a.seamReg : rg.reg;
-    if (reg && d > 0) {
-      const int f = d == 1 ? j : k;
-      if (f == 0 || f == a.G.na) {
-        const long nrna = (long)a.G.na * a.G.nr;
-        const int side = f == 0 ? 0 : 1, s = d == 1 ? k : j;
-        const double w = a.seamReg ? rg.w * (a.seamCfl / *a.seamInvMax) : rg.wDev ? rg.w * (rg.cfl / *rg.wDev) : rg.w;
-        double* S = reg + (((long)a.block0 * 2 + (d - 1)) * 2 + side) * 8 * nrna + (long)s * a.G.nr + i;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) S[q * nrna] = mad(w, fx[q], S[q * nrna]);
-      }
-    }
-  });
+  const Ctx& c = tab[wc.box * 3 + wc.dir];
+  const unsigned u = (unsigned)wc.begin + threadIdx.x;
+  if ((long)u >= wc.end) return;
+  if (wc.dir == 0) finalColumn<true>(c, rg, c.V0, 0, wc.march, u);
+  else finalColumn<false>(c, rg, c.V0, wc.dir, wc.march, u);
 }
 
 // 9, 12b. Flux divergence of the three directions and the Powell source
@@ -1170,12 +1236,23 @@ O4Batch* o4BatchCreate(const O4Args* boxes, int nbox, cudaError_t* err) {
       }
       total += n;
     }
-    const long chunk = chunkPoints(total, pass);
-    for (int d = 0; d < nd; ++d)
-      for (int b = 0; b < nbox; ++b) {
-        const long n = regionOf(host[(size_t)b * 3 + d], id).size();
-        for (long t = 0; t < n; t += chunk) work.push_back(WorkChunk{b, d, t, t + chunk < n ? t + chunk : n});
-      }
+    if (marches(id)) {
+      // columns as long as leaves every SM about 1024 threads, at most 16
+      // faces: a column's first row costs two more
+      const int march = (int)std::max(1L, std::min(16L, total / (148L * 1024)));
+      for (int d = 0; d < nd; ++d)
+        for (int b = 0; b < nbox; ++b) {
+          const long n = columns(regionOf(host[(size_t)b * 3 + d], id), d, march);
+          for (long u = 0; u < n; u += pass) work.push_back(WorkChunk{b, d, march, u, std::min(u + pass, n)});
+        }
+    } else {
+      const long chunk = chunkPoints(total, pass);
+      for (int d = 0; d < nd; ++d)
+        for (int b = 0; b < nbox; ++b) {
+          const long n = regionOf(host[(size_t)b * 3 + d], id).size();
+          for (long t = 0; t < n; t += chunk) work.push_back(WorkChunk{b, d, 0, t, std::min(t + chunk, n)});
+        }
+    }
     const long count = (long)work.size() - B->chunkOff[id];
     if (count > 0x7fffffffL) {
       *err = cudaErrorInvalidValue;

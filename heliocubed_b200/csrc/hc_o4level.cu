@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(128, 5) o4CartesianKernel(const O4StageIO io) 
     const int na = O.na;
     // Quotients use reciprocals of <det A> and dVolr (one rounding from the
     // reference's divisions).
-    const double invDet = 1.0 / detAt(O, b, j, k);
+    const double invDet = rcpN(detAt(O, b, j, k));
     const double dd1 = 0.5 * (detAt(O, b, j + 1, k) - detAt(O, b, j - 1, k));
     const double dd2 = 0.5 * (detAt(O, b, j, k + 1) - detAt(O, b, j, k - 1));
     // CubedSphereShell::deriv3case at (j, k): undivided centred difference
@@ -84,14 +84,14 @@ __global__ void __launch_bounds__(128, 5) o4CartesianKernel(const O4StageIO io) 
     double invJ[3], invK[3];
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
-      invJ[q] = 1.0 / detAt(O, b, ja + q, k);
-      invK[q] = 1.0 / detAt(O, b, j, ka + q);
+      invJ[q] = rcpN(detAt(O, b, ja + q, k));
+      invK[q] = rcpN(detAt(O, b, j, ka + q));
     }
     // the radial window of deriv3case at i
     const int ia = i == 0 ? 0 : (i == O.nr - 1 ? O.nr - 3 : i - 1);
     double invV[3];
 #pragma unroll
-    for (int q = 0; q < 3; ++q) invV[q] = 1.0 / volAt(O, ia + q);
+    for (int q = 0; q < 3; ++q) invV[q] = rcpN(volAt(O, ia + q));
     const double dv = 0.5 * (volAt(O, i + 1) - volAt(O, i - 1));
     const int slot = i - ia;
     // JU addressed from the box's base with fixed strides (component, j, k)
@@ -187,7 +187,7 @@ __global__ void o4SeamKernel(const O4StageIO io) {
     double thermal = u[4];
     if (u[0] > 0) {
 #pragma unroll
-      for (int d = 0; d < 3; ++d) thermal -= 0.5 * u[1 + d] * u[1 + d] / u[0] + u[5 + d] * u[5 + d] / (8 * kPi);
+      for (int d = 0; d < 3; ++d) thermal -= 0.5 * u[1 + d] * u[1 + d] / u[0] + u[5 + d] * u[5 + d] * (0.125 / kPi);
     }
     if (!(valid && u[0] >= kRHO00 && thermal >= 0 && isfinite(thermal))) {
       const O4Point P = O.pts[(long)b * O.npts + pt[0]];
@@ -296,7 +296,7 @@ __global__ void o4NativeKernel(const O4StageIO io) {
     } else {
       nativeCell(O, io.cart, b, O.nr - 1, j, k, u);
       const double rl = O.radial[O.nr - 1 + O.g + 1].y, rr = O.radial[i + O.g + 1].y;
-      const double s2 = pow(rl / rr, 2.0), s1 = pow(rl / rr, 1.0);
+      const double s1 = rl / rr, s2 = s1 * s1;
 #pragma unroll
       for (int c = 0; c < 8; ++c) u[c] *= c < 6 ? s2 : s1;
     }
