@@ -48,7 +48,13 @@ struct Chunk {
   int item, pad;
   long long begin, end;
 };
-constexpr long long kChunk = 16384;  // elements per CTA: 64 per thread
+// Elements per CTA: 4 per thread.  A list's items are boxes of some 500 to
+// 30,000 elements, so longer chunks (16,384) gave the small boxes of a level
+// one CTA each, 31 dependent rounds in it and most SMs idle.  32 x 32^2 shell
+// with 192 boxes of 8^3, per launch: commit 148 -> 84 us (with its loads ahead
+// of its tests), mapped 88 -> 79, native 72 -> 58, copies 30 -> 26, the
+// tableau's combinations 44 -> 13.
+constexpr long long kChunk = 1024;
 
 __global__ void __launch_bounds__(kThreads) rkCombineKernel(const hc_rk_box* __restrict__ boxes,
                                                             const Chunk* __restrict__ chunks, const RkFactors F) {
@@ -274,31 +280,36 @@ __global__ void __launch_bounds__(kThreads) cfPassKernel(const CfItem* __restric
       const double* row = src + (long long)B.coarse_n[0] * (b + (long long)B.coarse_n[1] * e2);
       for (int fi = tx; fi < fn0; fi += 32) {
         const double* w = sw[0][sc[0][fi]];
-        const int q0 = sq[0][fi];
-        double v = 0.0;
-        for (int k0 = -2; k0 <= 2; ++k0) {
-          if (w[k0 + 2] == 0.0) continue;
-          const int a = q0 + k0 - B.coarse_lo[0];
-          if (!rowIn || a < 0 || a >= B.coarse_n[0]) {
-            v = CUDART_NAN;
-            break;
-          }
-          v = __dadd_rn(v, __dmul_rn(w[k0 + 2], row[a]));
+        const int a0 = sq[0][fi] - 2 - B.coarse_lo[0];
+        // the five points' loads before their sums; a used point outside the
+        // coarse box makes the sum NaN
+        double x[5];
+        bool out = false;
+#pragma unroll
+        for (int m = 0; m < 5; ++m) {
+          const bool in = rowIn && a0 + m >= 0 && a0 + m < B.coarse_n[0];
+          x[m] = in ? row[a0 + m] : 0.0;
+          out = out || (!in && w[m] != 0.0);
         }
-        v0[r * fn0 + fi] = v;
+        double v = 0.0;
+#pragma unroll
+        for (int m = 0; m < 5; ++m)
+          if (w[m] != 0.0) v = __dadd_rn(v, __dmul_rn(w[m], x[m]));
+        v0[r * fn0 + fi] = out ? CUDART_NAN : v;
       }
     }
     __syncthreads();
     double* slot = ring + ((ck - c0[2]) % 5) * plane;
     for (int fj = ty; fj < fn1; fj += TY) {
-      const double* w = sw[1][sc[1][fj]];
-      const int base = sq[1][fj] - c0[1];
+      double w[5];
+#pragma unroll
+      for (int m = 0; m < 5; ++m) w[m] = sw[1][sc[1][fj]][m];
+      const double* first = v0 + (sq[1][fj] - c0[1] - 2) * fn0;
       for (int fi = tx; fi < fn0; fi += 32) {
         double v = 0.0;
-        for (int k1 = -2; k1 <= 2; ++k1) {
-          if (w[k1 + 2] == 0.0) continue;
-          v = __dadd_rn(v, __dmul_rn(w[k1 + 2], v0[(base + k1) * fn0 + fi]));
-        }
+#pragma unroll
+        for (int m = 0; m < 5; ++m)
+          if (w[m] != 0.0) v = __dadd_rn(v, __dmul_rn(w[m], first[m * fn0 + fi]));
         slot[fj * fn0 + fi] = v;
       }
     }
@@ -307,14 +318,19 @@ __global__ void __launch_bounds__(kThreads) cfPassKernel(const CfItem* __restric
     const int qk = ck - 2;
     const int plo = max(qk * B.ratio[2], B.fine_lo[2]), phi = min(qk * B.ratio[2] + B.ratio[2] - 1, B.fine_lo[2] + fn2 - 1);
     for (int p2 = plo; p2 <= phi; ++p2) {
-      const double* w = sw[2][p2 - qk * B.ratio[2]];
+      double w[5];
+      const double* from[5];
+#pragma unroll
+      for (int m = 0; m < 5; ++m) {
+        w[m] = sw[2][p2 - qk * B.ratio[2]][m];
+        from[m] = ring + ((qk + m - 2 - c0[2] + 5) % 5) * plane;
+      }
       double* o = out + (long long)plane * (p2 - B.fine_lo[2]);
       for (int e = tid; e < plane; e += kThreads) {
         double v = 0.0;
-        for (int k2 = -2; k2 <= 2; ++k2) {
-          if (w[k2 + 2] == 0.0) continue;
-          v = __dadd_rn(v, __dmul_rn(w[k2 + 2], ring[((qk + k2 - c0[2]) % 5) * plane + e]));
-        }
+#pragma unroll
+        for (int m = 0; m < 5; ++m)
+          if (w[m] != 0.0) v = __dadd_rn(v, __dmul_rn(w[m], from[m][e]));
         o[e] = v;
       }
     }
@@ -337,10 +353,17 @@ __global__ void __launch_bounds__(kThreads) cfCommitKernel(const CfItem* __restr
     bool inside = true;
     for (int d = 0; d < 3; ++d) inside = inside && p[d] >= B.valid_lo[d] && p[d] <= B.valid_hi[d];
     if (inside) continue;
+    // all components are loaded before the first test (at most kCfMaxComp)
+    double v[kCfMaxComp];
     bool finite = true;
-    for (int c = 0; c < B.ncomp; ++c) finite = finite && isfinite(res[(long long)c * fineN + t]);
+#pragma unroll
+    for (int c = 0; c < kCfMaxComp; ++c) v[c] = c < B.ncomp ? res[(long long)c * fineN + t] : 0.0;
+#pragma unroll
+    for (int c = 0; c < kCfMaxComp; ++c) finite = finite && isfinite(v[c]);
     if (!finite) continue;
-    for (int c = 0; c < B.ncomp; ++c) B.fine[(long long)c * fineN + t] = res[(long long)c * fineN + t];
+#pragma unroll
+    for (int c = 0; c < kCfMaxComp; ++c)
+      if (c < B.ncomp) B.fine[(long long)c * fineN + t] = v[c];
   }
 }
 
@@ -373,7 +396,11 @@ __global__ void __launch_bounds__(kThreads) cfMappedKernel(const hc_cf_fine_box*
     for (int d = 0; d < 3; ++d) p[d] += B.mapped_lo[d];
     if (inValid(B, p)) {
       const long long so = boxOff(B.state_lo, B.state_n, p[0], p[1], p[2]);
-      for (int c = 0; c < 8; ++c) B.mapped[c * mN + t] = B.state[c * sN + so];
+      double v[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) v[c] = B.state[c * sN + so];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) B.mapped[c * mN + t] = v[c];
       continue;
     }
     const double J = B.jac[boxOff(B.jac_lo, B.jac_n, p[0], p[1], p[2])];
@@ -388,13 +415,17 @@ __global__ void __launch_bounds__(kThreads) cfMappedKernel(const hc_cf_fine_box*
       dn[d] = boxOff(B.donor_lo, B.donor_n, b[0], b[1], b[2]);
     }
     const long long o = boxOff(B.donor_lo, B.donor_n, p[0], p[1], p[2]);
+    double value[8];
+#pragma unroll
     for (int c = 0; c < 8; ++c) {
       const double* U = B.donor + c * dN;
-      double value = __dmul_rn(J, U[o]);
+      value[c] = __dmul_rn(J, U[o]);
+#pragma unroll
       for (int d = 0; d < 3; ++d)
-        value = __dadd_rn(value, __ddiv_rn(__dmul_rn(dJ[d], __dsub_rn(U[up[d]], U[dn[d]])), 48.0));
-      B.mapped[c * mN + t] = value;
+        value[c] = __dadd_rn(value[c], __ddiv_rn(__dmul_rn(dJ[d], __dsub_rn(U[up[d]], U[dn[d]])), 48.0));
     }
+#pragma unroll
+    for (int c = 0; c < 8; ++c) B.mapped[c * mN + t] = value[c];
   }
 }
 
@@ -463,7 +494,15 @@ __global__ void __launch_bounds__(kThreads) copyKernel(const hc_copy_box* __rest
                       B.sign[2] * x[B.perm[2]] + B.shift[2]};
     const long long so = boxOff(B.src_lo, B.src_n, x[0], x[1], x[2]);
     const long long dO = boxOff(B.dst_lo, B.dst_n, y[0], y[1], y[2]);
-    for (int c = 0; c < B.ncomp; ++c) B.dst[c * dN + dO] = B.src[c * sN + so];
+    // eight components' loads before their stores (the arrays may be one)
+    for (int c = 0; c < B.ncomp; c += 8) {
+      double v[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = c + e < B.ncomp ? B.src[(c + e) * sN + so] : 0.0;
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        if (c + e < B.ncomp) B.dst[(c + e) * dN + dO] = v[e];
+    }
   }
 }
 
