@@ -42,12 +42,19 @@ const double PI = 3.14159265358979323846;
 
 struct Vec3 { double x[3]; };
 
-// Basis A = (Xhat, dXhat/dxi1, dXhat/dxi2) at panel coordinates (x1, x2).
-void basisAt(int b, double x1, double x2, double A[3][3], double X[3]) {
-  const double ta = std::tan(-PI / 4 + PI / 2 * x1), tb = std::tan(-PI / 4 + PI / 2 * x2);
+// One panel coordinate's share of the basis: tan of its angle and the
+// derivative of that.
+struct Axis {
+  double t, d;
+  Axis() = default;
+  explicit Axis(double x) : t(std::tan(-PI / 4 + PI / 2 * x)), d(PI / 2 * (1 + t * t)) {}
+};
+
+// Basis A = (Xhat, dXhat/dxi1, dXhat/dxi2) at panel coordinates (a, c).
+void basisAt(int b, const Axis& a, const Axis& c, double A[3][3], double X[3]) {
+  const double ta = a.t, tb = c.t, da = a.d, db = c.d;
   const double rho2 = 1 + ta * ta + tb * tb, rho = std::sqrt(rho2), r3 = rho * rho2;
   const double q[3] = {1 / rho, ta / rho, tb / rho};
-  const double da = PI / 2 * (1 + ta * ta), db = PI / 2 * (1 + tb * tb);
   const double q1[3] = {-ta / r3 * da, (1 / rho - ta * ta / r3) * da, -ta * tb / r3 * da};
   const double q2[3] = {-tb / r3 * db, -ta * tb / r3 * db, (1 / rho - tb * tb / r3) * db};
   for (int k = 0; k < 3; ++k) {
@@ -58,6 +65,7 @@ void basisAt(int b, double x1, double x2, double A[3][3], double X[3]) {
     if (X) X[k] = A[k][0];
   }
 }
+void basisAt(int b, double x1, double x2, double A[3][3], double X[3]) { basisAt(b, Axis(x1), Axis(x2), A, X); }
 
 void cross(const double u[3], const double v[3], double w[3]) {
   w[0] = u[1] * v[2] - u[2] * v[1];
@@ -87,6 +95,25 @@ struct Gauss {
       w[i] = 1 / ((1 - z * z) * pp * pp);
     }
   }
+};
+
+// The coordinates that the metric quadratures visit, for cells lo .. hi of
+// width h: low edge, centre and quadrature points.  A panel has some n^2 x 64
+// points per average and only n x 8 coordinates, so the tangents, most of
+// a context's set-up time when taken at every point, are taken once.
+struct Axes {
+  int lo;
+  std::vector<Axis> edges, mids, points;
+  Axes(int lo_, int hi, double h, const Gauss& G) : lo(lo_) {
+    for (int j = lo; j <= hi; ++j) {
+      edges.emplace_back(j * h);
+      mids.emplace_back((j + 0.5) * h);
+      for (int p = 0; p < 8; ++p) points.emplace_back((j + G.x[p]) * h);
+    }
+  }
+  const Axis& edge(int j) const { return edges[j - lo]; }
+  const Axis& mid(int j) const { return mids[j - lo]; }
+  const Axis& at(int j, int p) const { return points[(size_t)(j - lo) * 8 + p]; }
 };
 
 // Cofactor row d of A (normal of a constant-xi_d face), times det when
@@ -307,6 +334,7 @@ int buildLevel(hc_ctx* c) {
   const int nr = P.nr, na = P.na, g = kGhost;
   const double h = 1.0 / na;
   Gauss G;
+  const Axes T(0, na, h, G);
   DevLevel& L = c->L;
   L.nr = nr; L.na = na; L.g = g;
   L.n0 = nr + 2 * g; L.n1 = na + 2 * g;
@@ -355,15 +383,15 @@ int buildLevel(hc_ctx* c) {
             for (int p = 0; p < 8; ++p)
               for (int q = 0; q < 8; ++q) {
                 double A[3][3], m[3];
-                basisAt(b, (j + G.x[p]) * h, (k + G.x[q]) * h, A, nullptr);
+                basisAt(b, T.at(j, p), T.at(k, q), A, nullptr);
                 cofactorRow(A, 0, m);
                 for (int r = 0; r < 3; ++r) n[r] += G.w[p] * G.w[q] * m[r];
               }
           } else {
             for (int p = 0; p < 8; ++p) {
               double A[3][3], m[3];
-              if (d == 1) basisAt(b, j * h, (k + G.x[p]) * h, A, nullptr);
-              else basisAt(b, (j + G.x[p]) * h, k * h, A, nullptr);
+              if (d == 1) basisAt(b, T.edge(j), T.at(k, p), A, nullptr);
+              else basisAt(b, T.at(j, p), T.edge(k), A, nullptr);
               cofactorRow(A, d, m);
               for (int r = 0; r < 3; ++r) n[r] += G.w[p] * m[r];
             }
@@ -378,14 +406,14 @@ int buildLevel(hc_ctx* c) {
         for (int p = 0; p < 8; ++p)
           for (int q = 0; q < 8; ++q) {
             double A[3][3];
-            basisAt(b, (j + G.x[p]) * h, (k + G.x[q]) * h, A, nullptr);
+            basisAt(b, T.at(j, p), T.at(k, q), A, nullptr);
             const double dt = det3(A), wt = G.w[p] * G.w[q];
             det += wt * dt;
             for (int r = 0; r < 3; ++r)
               for (int s = 0; s < 3; ++s) dA[r][s] += wt * dt * A[r][s];
           }
         double Ac[3][3], X[3], Ai[3][3];
-        basisAt(b, (j + 0.5) * h, (k + 0.5) * h, Ac, X);
+        basisAt(b, T.mid(j), T.mid(k), Ac, X);
         inv3(Ac, Ai);
         GravCell& gc = grav[ci];
         for (int r = 0; r < 3; ++r) { gc.x[r] = X[r]; gc.a0[r] = dA[r][0]; }
@@ -417,14 +445,14 @@ int buildLevel(hc_ctx* c) {
           double fd = 0;
           for (int p = 0; p < 8; ++p) {
             double A[3][3];
-            if (d == 1) basisAt(b, j * h, (k + G.x[p]) * h, A, nullptr);
-            else basisAt(b, (j + G.x[p]) * h, k * h, A, nullptr);
+            if (d == 1) basisAt(b, T.edge(j), T.at(k, p), A, nullptr);
+            else basisAt(b, T.at(j, p), T.edge(k), A, nullptr);
             fd += G.w[p] * det3(A);
           }
           cc.det[d] = fd;
           double F[3][3];
-          if (d == 1) basisAt(b, j * h, (k + 0.5) * h, F, nullptr);
-          else basisAt(b, (j + 0.5) * h, k * h, F, nullptr);
+          if (d == 1) basisAt(b, T.edge(j), T.mid(k), F, nullptr);
+          else basisAt(b, T.mid(j), T.edge(k), F, nullptr);
           for (int r = 0; r < 3; ++r)
             for (int s = 0; s < 3; ++s) cc.face[d - 1][3 * r + s] = F[r][s];
         }
@@ -576,13 +604,14 @@ int buildO4Geometry(hc_ctx* c) {
   const int n = na + 2 * ext + 1;
   const double h = 1.0 / na;
   Gauss G;
+  const Axes T(-ext, na + ext, h, G);
   constexpr int kRec = 22;  // <det A A> (9), <det A>, normal (3), point basis (9)
   std::vector<double> face((size_t)6 * 3 * n * n * kRec), cell((size_t)6 * n * n * 9);
   for (int b = 0; b < 6; ++b)
     for (int k = -ext; k <= na + ext; ++k)
       for (int j = -ext; j <= na + ext; ++j) {
         double A[3][3];
-        basisAt(b, (j + 0.5) * h, (k + 0.5) * h, A, nullptr);
+        basisAt(b, T.mid(j), T.mid(k), A, nullptr);
         double* cb = &cell[(((size_t)b * n + (k + ext)) * n + (j + ext)) * 9];
         for (int r = 0; r < 3; ++r)
           for (int q = 0; q < 3; ++q) cb[3 * r + q] = A[r][q];
@@ -593,7 +622,7 @@ int buildO4Geometry(hc_ctx* c) {
             for (int p = 0; p < 8; ++p)
               for (int q = 0; q < 8; ++q) {
                 double Aq[3][3], m[3];
-                basisAt(b, (j + G.x[p]) * h, (k + G.x[q]) * h, Aq, nullptr);
+                basisAt(b, T.at(j, p), T.at(k, q), Aq, nullptr);
                 const double wt = G.w[p] * G.w[q], dt = det3(Aq);
                 det += wt * dt;
                 cofactorRow(Aq, 0, m);
@@ -605,8 +634,8 @@ int buildO4Geometry(hc_ctx* c) {
           } else {
             for (int p = 0; p < 8; ++p) {
               double Aq[3][3], m[3];
-              if (d == 1) basisAt(b, j * h, (k + G.x[p]) * h, Aq, nullptr);
-              else basisAt(b, (j + G.x[p]) * h, k * h, Aq, nullptr);
+              if (d == 1) basisAt(b, T.edge(j), T.at(k, p), Aq, nullptr);
+              else basisAt(b, T.at(j, p), T.edge(k), Aq, nullptr);
               const double dt = det3(Aq);
               det += G.w[p] * dt;
               cofactorRow(Aq, d, m);
@@ -622,9 +651,9 @@ int buildO4Geometry(hc_ctx* c) {
           e[9] = det;
           for (int r = 0; r < 3; ++r) e[10 + r] = nn[r];
           double F[3][3];
-          if (d == 0) basisAt(b, (j + 0.5) * h, (k + 0.5) * h, F, nullptr);
-          else if (d == 1) basisAt(b, j * h, (k + 0.5) * h, F, nullptr);
-          else basisAt(b, (j + 0.5) * h, k * h, F, nullptr);
+          if (d == 0) basisAt(b, T.mid(j), T.mid(k), F, nullptr);
+          else if (d == 1) basisAt(b, T.edge(j), T.mid(k), F, nullptr);
+          else basisAt(b, T.mid(j), T.edge(k), F, nullptr);
           for (int r = 0; r < 3; ++r)
             for (int q = 0; q < 3; ++q) e[13 + 3 * r + q] = F[r][q];
         }
@@ -738,6 +767,7 @@ int buildO4Level(hc_ctx* c) {
   const int nA = na + 2 * ga, nG = na + 2 * g;
   const double h = 1.0 / na;
   Gauss G;
+  const Axes T(-ga - 1, na + ga, h, G);
   O4Level& O = c->o4l;
   O.nr = nr; O.na = na; O.g = g; O.ga = ga; O.nA = nA; O.nG = nG;
   O.Nv = (long)nr * na * na;
@@ -776,7 +806,7 @@ int buildO4Level(hc_ctx* c) {
         for (int p = 0; p < 8; ++p)
           for (int q = 0; q < 8; ++q) {
             double Aq[3][3];
-            basisAt(b, (j + G.x[p]) * h, (k + G.x[q]) * h, Aq, nullptr);
+            basisAt(b, T.at(j, p), T.at(k, q), Aq, nullptr);
             for (int r = 0; r < 3; ++r)
               for (int s2 = 0; s2 < 3; ++s2) A[r][s2] += G.w[p] * G.w[q] * Aq[r][s2];
           }
@@ -799,7 +829,7 @@ int buildO4Level(hc_ctx* c) {
         for (int p = 0; p < 8; ++p)
           for (int q = 0; q < 8; ++q) {
             double Aq[3][3];
-            basisAt(b, (j + G.x[p]) * h, (k + G.x[q]) * h, Aq, nullptr);
+            basisAt(b, T.at(j, p), T.at(k, q), Aq, nullptr);
             det += G.w[p] * G.w[q] * det3(Aq);
           }
         detx[((size_t)b * (na + 2) + (k + 1)) * (na + 2) + (j + 1)] = det;
@@ -807,13 +837,13 @@ int buildO4Level(hc_ctx* c) {
     for (int k = -g; k < na + g; ++k)
       for (int j = -g; j < na + g; ++j) {
         double A[3][3], X[3];
-        basisAt(b, (j + 0.5) * h, (k + 0.5) * h, A, X);
+        basisAt(b, T.mid(j), T.mid(k), A, X);
         for (int q = 0; q < 3; ++q) xhat[(((size_t)b * nG + (k + g)) * nG + (j + g)) * 3 + q] = X[q];
       }
     for (int q = 0; q < O.npts; ++q) {
       const int j = ptJK[q].x, k = ptJK[q].y;
       double A[3][3], X[3], y1, y2;
-      basisAt(b, (j + 0.5) * h, (k + 0.5) * h, A, X);
+      basisAt(b, T.mid(j), T.mid(k), A, X);
       O4Point pt{};
       pt.p = locateTie(X);
       panelCoords(pt.p, X, y1, y2);
@@ -1073,17 +1103,21 @@ int o4Stage(hc_ctx* c, double* ju, int stage, double dtv, const double* invMax, 
   O4StageIO io{O, stage == 0 ? ju : c->o4next, c->o4cart, c->o4us, c->o4pv,
                StageTime{tbase, tdev, c4[stage], invMax, dtv}};
   rc = checkLaunch(launchO4Prepare(io, s), "O4 prepare");
-  if (rc == HC_OK) rc = checkLaunch(cudaMemsetAsync(c->o4k, 0, sizeof(double) * 6 * 8 * O.Nv, s), "O4 k");
+  // the operator writes every k unless gravity comes before it or it covers
+  // a window only
+  const bool fresh = !c->P.sun_gravity && c->winHi == 0;
+  if (rc == HC_OK && !fresh) rc = checkLaunch(cudaMemsetAsync(c->o4k, 0, sizeof(double) * 6 * 8 * O.Nv, s), "O4 k");
   if (rc != HC_OK) return rc;
   if (c->P.sun_gravity) {
     rc = checkLaunch(launchO4BatchGravity(c->o4levelBatch, s), "O4 gravity");
     if (rc != HC_OK) return rc;
   }
-  const RegArgs rg{c->o4reg, invMax ? b4[stage] : dtv * b4[stage], invMax, c->P.cfl};
+  const RkUpdate update{stage, ju, c->acc, c->o4next, invMax, c->P.cfl, dtv};
+  RegArgs rg{c->o4reg, invMax ? b4[stage] : dtv * b4[stage], invMax, c->P.cfl, fresh};
+  if (c->winHi == 0) rg.rk = update;
   o4BatchSetVariants(c->o4levelBatch, c->o4var);
   rc = checkLaunch(launchO4Batch(c->o4levelBatch, &rg, s), "O4 operator");
-  if (rc == HC_OK)
-    rc = checkLaunch(launchO4Update(O, stage, c->o4k, ju, c->acc, c->o4next, invMax, c->P.cfl, dtv, s), "O4 update");
+  if (rc == HC_OK && c->winHi != 0) rc = checkLaunch(launchO4Update(O, update, c->o4k, s), "O4 update");
   if (rc == HC_OK && stage == 3) rc = checkLaunch(launchO4Reflux(O, c->L, c->o4reg, ju, s), "O4 reflux");
   return rc;
 }
@@ -1426,7 +1460,7 @@ int hc_level_rhs_fluxes(hc_ctx* c, const double* w, double* k, double* const* fl
   if (rc != HC_OK) return rc;
   // this evaluation's seam fluxes (weight 1) into the register, then each
   // seam face's rhs takes the mean of both panels' fluxes
-  const RegArgs rg{c->o4reg, 1.0, nullptr, c->P.cfl};
+  const RegArgs rg{c->o4reg, 1.0, nullptr, c->P.cfl, 0};
   o4BatchSetVariants(B, c->o4var);
   rc = checkLaunch(launchO4Batch(B, &rg, s), "O4 operator");
   if (rc == HC_OK) rc = checkLaunch(launchO4Reflux(O, c->L, c->o4reg, k, s), "O4 seam reconciliation");
@@ -1442,11 +1476,14 @@ int hc_level_rhs(hc_ctx* c, const double* w, double* k, void* stream) {
     O4Batch* B = (w == c->o4us && k == c->o4k && c->winHi == 0) ? c->o4levelBatch
                                                                  : cachedBatch(c, levelO4Args(c, w, k), &rc);
     if (!B) return rc;
-    rc = checkLaunch(cudaMemsetAsync(k, 0, sizeof(double) * 6 * NC * c->o4l.Nv, s), "O4 k");
-    if (rc == HC_OK && c->P.sun_gravity) rc = checkLaunch(launchO4BatchGravity(B, s), "O4 gravity");
-    if (rc != HC_OK) return rc;
+    if (c->P.sun_gravity) {
+      rc = checkLaunch(cudaMemsetAsync(k, 0, sizeof(double) * 6 * NC * c->o4l.Nv, s), "O4 k");
+      if (rc == HC_OK) rc = checkLaunch(launchO4BatchGravity(B, s), "O4 gravity");
+      if (rc != HC_OK) return rc;
+    }
+    const RegArgs rg{nullptr, 0.0, nullptr, 0.0, !c->P.sun_gravity};
     o4BatchSetVariants(B, c->o4var);
-    return checkLaunch(launchO4Batch(B, nullptr, s), "O4 operator");
+    return checkLaunch(launchO4Batch(B, &rg, s), "O4 operator");
   }
   StageArgs a = levelArgs(c, w);
   a.rhs = k;
@@ -1666,21 +1703,20 @@ int ensembleStep(hc_ensemble* E, double* const* ju, double* const* time, double*
       const O4StageIO io{c->o4l, stage == 0 ? ju[q] : c->o4next, c->o4cart, c->o4us, c->o4pv,
                          StageTime{0.0, time ? time[q] : nullptr, c4[stage], invMaxOf(c), 0.0}};
       rc = checkLaunch(launchO4Prepare(io, lane(q)), "O4 prepare");
-      if (rc == HC_OK)
+      if (rc == HC_OK && E->gravity)
         rc = checkLaunch(cudaMemsetAsync(c->o4k, 0, sizeof(double) * 6 * 8 * c->o4l.Nv, lane(q)), "O4 k");
     }
     if (rc == HC_OK) rc = ensembleJoin(E, s);
     if (rc == HC_OK && E->gravity) rc = checkLaunch(launchO4BatchGravity(E->batch, s), "O4 gravity");
     if (rc != HC_OK) break;
-    const RegArgs rg{nullptr, b4[stage], nullptr, 0.0};  // each box carries its level's register
+    const RegArgs rg{nullptr, b4[stage], nullptr, 0.0, !E->gravity};  // each box carries its level's register
     o4BatchSetVariants(E->batch, E->members[0]->o4var);
     rc = checkLaunch(launchO4Batch(E->batch, &rg, s), "O4 operator");
     if (rc == HC_OK) rc = ensembleFork(E, s);
     for (int q = 0; q < m && rc == HC_OK; ++q) {
       hc_ctx* c = E->members[q];
-      rc = checkLaunch(
-          launchO4Update(c->o4l, stage, c->o4k, ju[q], c->acc, c->o4next, invMaxOf(c), c->P.cfl, 0.0, lane(q)),
-          "O4 update");
+      const RkUpdate update{stage, ju[q], c->acc, c->o4next, invMaxOf(c), c->P.cfl, 0.0};
+      rc = checkLaunch(launchO4Update(c->o4l, update, c->o4k, lane(q)), "O4 update");
     }
   }
   for (int q = 0; q < m && rc == HC_OK; ++q) {

@@ -455,4 +455,27 @@ HC_DEV void o4NativeCore(const double* c0, long sj, long sk, long sc, const doub
   }
 }
 
+// Classical RK4 after a stage (the tableau of src/MHD_AMRRungeKutta.H:10-12)
+// of the eight components at offset `at`, n apart.
+template <class U>
+HC_DEV void rkUpdate(const U& u, double dt, long at, long n, const Rn kv[8]) {
+  const Rn fb = dt * (u.stage == 0 || u.stage == 3 ? 1.0 / 6 : 1.0 / 3), fa = dt * (u.stage == 2 ? 1.0 : 0.5);
+  double v[8], w[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    v[q] = u.stage == 3 ? 0.0 : u.ju[at + q * n];
+    w[q] = u.stage == 0 ? v[q] : u.acc[at + q * n];
+  }
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const double sum = mad(fb, kv[q], w[q]);
+    if (u.stage == 3) {
+      u.ju[at + q * n] = sum;
+    } else {
+      u.acc[at + q * n] = sum;
+      u.next[at + q * n] = mad(fa, kv[q], v[q]);
+    }
+  }
+}
+
 }  // namespace hc

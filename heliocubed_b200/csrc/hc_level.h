@@ -251,10 +251,10 @@ struct O4Args {
   Reg rr;
 };
 // Flux sums (7, the normal field's vanishes) and pressure sum, whose place the
-// final fluxes (8) take; point dissipation (8); left and right states (16),
-// the left ones' place taken by the area products of the averages (7 + 1);
-// flag, centred normal field, speed bound, Powell flux.
-constexpr int kO4FaceArrays = 36;
+// final fluxes (8) take; left states (8), whose place the area products of
+// the averages (7 + 1) take; right states (8), whose place the point
+// dissipation (8) takes; flag, centred normal field, speed bound, Powell flux.
+constexpr int kO4FaceArrays = 28;
 
 size_t o4ScratchDoubles(int nbox, const int vlo[3], const int vhi[3], int ghost);
 // Carve the operator scratch of a.nbox boxes with the valid box a.vlo..vhi
@@ -265,11 +265,22 @@ size_t o4CarveScratch(O4Args& a, double* sp);
 // Seam flux register of the level step (reg null: off): the final face flux
 // of panel-boundary faces of directions 1, 2 of whole-panel boxes is added
 // times w (times cfl / *wDev when wDev is set) into reg [6][2][2][8][na][nr].
+// fresh: rhs is written, not accumulated (the caller need not clear it).
+// rk.stage >= 0: the boxes are a whole level's panels and the RK4 update of
+// that stage takes the place of the rhs store.
+struct RkUpdate {
+  int stage = -1;
+  double *ju = nullptr, *acc = nullptr, *next = nullptr;  // [6][8][Nv]
+  const double* invDtMax = nullptr;                       // device: dt = cfl / *invDtMax (null: dtv)
+  double cfl = 0, dtv = 0;
+};
 struct RegArgs {
-  double* reg;
-  double w;
-  const double* wDev;
-  double cfl;
+  double* reg = nullptr;
+  double w = 0;
+  const double* wDev = nullptr;
+  double cfl = 0;
+  int fresh = 0;
+  RkUpdate rk{};
 };
 
 // A batch of boxes of any sizes for the operator kernels: per box and
@@ -336,8 +347,7 @@ struct O4StageIO {
 cudaError_t launchO4Prepare(const O4StageIO& io, cudaStream_t s);
 // acc/stage/ju update after stage s (classical RK4, b = 1/6, 1/3, 1/3, 1/6;
 // next stage = ju + a_{s+1} dt k with a = 1/2, 1/2, 1).
-cudaError_t launchO4Update(const O4Level& O, int stage, const double* k, double* ju, double* acc, double* next,
-                           const double* invDtMax, double cfl, double dtv, cudaStream_t s);
+cudaError_t launchO4Update(const O4Level& O, const RkUpdate& u, const double* k, cudaStream_t s);
 // Seam flux reconciliation from the time-integrated register
 // [6][2][2][8][na][nr] (edge axis 1..2, side 0..1, component, along-edge, radial).
 cudaError_t launchO4Reflux(const O4Level& O, const DevLevel& L, const double* reg, double* ju, cudaStream_t s);

@@ -12,7 +12,8 @@
 //   o4FaceFinalKernel: mapped final flux of every face
 //   o4CellKernel: flux divergence and Powell source into rhs
 // and on a side stream o4PowellAvgKernel, o4PowellFluxKernel, o4PowellDivKernel.
-// Every intermediate covers the box the reference computes it on.
+// Every intermediate covers what a later kernel reads of the box the reference
+// computes it on.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -55,11 +56,13 @@ __device__ __forceinline__ long roff(const Reg& r, int i, int j, int k) {
 // Offsets of the face arrays inside a direction's face scratch (units of
 // F.N).  Vector components of the flux sums, dissipations and averages are
 // kept along (normal, next, next but one) native direction; the flux sum of
-// the normal field vanishes and has no array.  The final fluxes (Cartesian
-// components) take the place of the flux sums and pressures, and the area
-// products that of the left states, which nothing reads any more by then.
-enum FaceArr { F_FS = 0, F_PS = 7, F_FX = 0, F_QD = 8, F_L = 16, F_R = 24, F_X = 16, F_T3 = 23, F_THF = 32, F_BP = 33,
-               F_SPD = 34, F_BF = 35 };
+// the normal field vanishes and has no array.  Arrays share places with what
+// nothing reads any more: the final fluxes (Cartesian components) that of the
+// flux sums and pressures, the area products that of the left states, and
+// the dissipation that of the right states (a face's states are in its
+// thread's hands before the thread writes the face's dissipation).
+enum FaceArr { F_FS = 0, F_PS = 7, F_FX = 0, F_L = 8, F_X = 8, F_T3 = 15, F_R = 16, F_QD = 16, F_THF = 24, F_BP = 25,
+               F_SPD = 26, F_BF = 27 };
 static_assert(F_BF + 1 == kO4FaceArrays && F_T3 == F_X + 7, "face arrays");
 // F_FS array of component c in (rho, m_n, m_1, m_2, E, B_n, B_1, B_2) order (c != 5), also of F_X.
 __host__ __device__ constexpr int fluxSlot(int c) { return c < 5 ? c : c - 1; }
@@ -67,7 +70,7 @@ __host__ __device__ constexpr int fluxSlot(int c) { return c < 5 ? c : c - 1; }
 struct Ctx {
   O4Args a;
   int d;
-  Box3 V, G, GR, GD, F, F1, V0, V1;
+  Box3 V, G, GR, GD, F, V0, V1;
   Reg gr, fr, v1r, vr;
 };
 
@@ -85,8 +88,20 @@ __host__ __device__ inline Box3 regionOf(const Ctx& c, int id) {
     case RG_F: return c.F;
     case RG_PB: return c.V0.growTrans(c.d, 1);
     case RG_V0: return c.V0;
-    default: return c.V1.extrude(c.d).growTrans(c.d, 1);
+    default: {  // Powell fluxes: the faces of V1, and their radial neighbours for the area product
+      Box3 b = c.V1.extrude(c.d);
+      if (c.d != 0) { b.lo[0] -= 1; b.hi[0] += 1; }
+      return b;
+    }
   }
+}
+// Whether at most one coordinate of a cell lies outside the valid box grown
+// by g: the corners of the ghosted box, which no face stencil reaches (the
+// stencils are long along one direction only), are not computed.
+__device__ __forceinline__ bool crossShaped(const Box3& V, int g, int i, int j, int k) {
+  const bool a = i < V.lo[0] - g || i > V.hi[0] + g, b = j < V.lo[1] - g || j > V.hi[1] + g,
+             c = k < V.lo[2] - g || k > V.hi[2] + g;
+  return !((a && b) || (a && c) || (b && c));
 }
 // Points a CTA takes per pass: the face averages give up one thread at each
 // end, whose averages only serve their neighbours.
@@ -135,10 +150,11 @@ Ctx makeCtx(const O4Args& a, int d) {
   c.G = c.V.grow(a.ghost);
   c.GR = c.G.grow(-1);
   c.GD = c.G.grow(-2);
-  c.F = c.G.extrude(d).grow(-3);
-  c.F1 = c.F.growTrans(d, -1);
   c.V0 = c.V.extrude(d);
   c.V1 = c.V.grow(1);
+  // faces whose states something reads: one beyond the valid box along the
+  // normal (the Powell fluxes of V1), two across (the averages' neighbours)
+  c.F = c.V1.extrude(d).growTrans(d, 1);
   c.gr = regOf(c.G);
   // face scratch is laid out on the largest face box over the directions
   c.fr = regOf(faceBox(c.G));
@@ -388,6 +404,8 @@ __device__ __forceinline__ int columnOf(const Box3& b, int d, int march, unsigne
   return left < march ? left : march;
 }
 
+__device__ __forceinline__ void prefetch(const double* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
 // Thread -> (i, j, k) over the chunk's points of region b of the chunk's box.
 template <class F>
 __device__ __forceinline__ void forRegion(const Box3& b, int walk, const WorkChunk& w, F f) {
@@ -411,6 +429,7 @@ __global__ void o4PrimAvgKernel(const Ctx* __restrict__ tab, const RegArgs rg, c
   const Ctx& c = tab[wc.box * 3 + 0];
   const O4Args& a = c.a;
   forRegion(c.G, WALK_JK, wc, [&](int i, int j, int k) {
+    if (!crossShaped(c.V, 4, i, j, k)) return;  // what the flags below read
     double u[8], w[8];
     const double* U = a.U + roff(a.ur, i, j, k);
 #pragma unroll
@@ -442,6 +461,7 @@ __global__ void __launch_bounds__(128) o4ThetaRawKernel(const Ctx* __restrict__ 
     return num * rcpN(mad(2.0, fabs(q.v), Rn(fabs(p.v)) + fabs(m.v)) + 1.0e-40);
   };
   forRegion(c.GR, WALK_JK, wc, [&](int i, int j, int k) {
+    if (!crossShaped(c.V, 3, i, j, k)) return;  // what the dilation reads
     const long o = roff(c.gr, i, j, k);
     const double* W = a.WA + o;
     const Rn r0 = __ldg(W), p0 = __ldg(W + 4 * N), m0 = magp(W);
@@ -464,7 +484,8 @@ __global__ void o4PointKernel(const Ctx* __restrict__ tab, const RegArgs rg, con
   const WorkChunk wc = wk[blockIdx.x];
   const Ctx& c = tab[wc.box * 3 + 0];
   const O4Args& a = c.a;
-  forRegion(c.G, WALK_JK, wc, [&](int i, int j, int k) {
+  forRegion(c.GR, WALK_JK, wc, [&](int i, int j, int k) {
+    if (!crossShaped(c.V, 2, i, j, k)) return;  // what the reconstruction reads
     const long N = c.gr.N, o = roff(c.gr, i, j, k);
     const double* R = a.thr;
     double t = 0.0;
@@ -479,12 +500,16 @@ __global__ void o4PointKernel(const Ctx* __restrict__ tab, const RegArgs rg, con
       t = dmin(t, R[roff(c.gr, i, j, k - 1)]);
       t = dmin(t, R[roff(c.gr, i, j, k + 1)]);
     }
-    const bool inner = i >= c.GR.lo[0] && i <= c.GR.hi[0] && j >= c.GR.lo[1] && j <= c.GR.hi[1] &&
-                       k >= c.GR.lo[2] && k <= c.GR.hi[2];
     View U{a.U, a.ur};
     double u[8], w[8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) u[q] = (inner && t > 0.5) ? U(q, i, j, k) - lapCell(U, q, i, j, k) * (1.0 / 24.0) : U(q, i, j, k);
+    for (int q = 0; q < 8; ++q) u[q] = U(q, i, j, k);
+    // the neighbours are loaded whatever the flag, with the flags' own loads
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const double point = fma(lapCell(U, q, i, j, k), -1.0 / 24.0, u[q]);
+      u[q] = t > 0.5 ? point : u[q];
+    }
     sphToPrim(u, cellBasis(a.G, a.block0, j, k), a.G.gamma, w);
     double* W = a.WP + o;
 #pragma unroll
@@ -613,8 +638,8 @@ __global__ void __launch_bounds__(128, MB) o4FaceRiemannKernel(const Ctx* __rest
       copyAsync(&sh[slot][8 + q][threadIdx.x], src + (F_R - F_L + place(q, d)) * NF);
     }
     const double* R = roeRec(a.G, blk, d, j, k);
-    asm volatile("prefetch.global.L1 [%0];" ::"l"(R));
-    asm volatile("prefetch.global.L1 [%0];" ::"l"(R + 16));
+    prefetch(R);
+    prefetch(R + 16);
   };
   const unsigned end = (unsigned)wc.end;
   int slot = 0;
@@ -650,6 +675,9 @@ __global__ void __launch_bounds__(128, MB) o4FaceRiemannKernel(const Ctx* __rest
         base[F_THF * NF] = 0.0;
       }
     }
+    base[F_BP * NF] = 0.5 * (Rn(l[5]) + r[5]);
+    const int along = d == 0 ? i : d == 1 ? j : k;
+    if (along < c.V.lo[d] || along > c.V.hi[d] + 1) continue;  // a face of the Powell flux only
     const double* R = roeRec(a.G, blk, d, j, k);
     double f[10];
 #pragma unroll
@@ -693,7 +721,6 @@ __global__ void __launch_bounds__(128, MB) o4FaceRiemannKernel(const Ctx* __rest
 #pragma unroll
     for (int q = 0; q < 7; ++q) base[(F_FS + q) * NF] = fs[q];
     base[F_PS * NF] = ps;
-    base[F_BP * NF] = 0.5 * (Rn(l[5]) + r[5]);
     const Box3 PB = regionOf(c, RG_PB);
     if (i < PB.lo[0] || i > PB.hi[0] || j < PB.lo[1] || j > PB.hi[1] || k < PB.lo[2] || k > PB.hi[2]) continue;
     if (roe) {
@@ -834,7 +861,7 @@ __global__ void __launch_bounds__(128, 6) o4FaceAvgKernel(const Ctx* __restrict_
 // holds the halved M, det and normal and their angular differences / 48.
 //
 // One thread per column of faces, no barrier.  Bound by the latency of L2:
-// 64^3, three directions, 398 us marching against 475 with a thread per face
+// 64^3, three directions, 351 us marching against 475 with a thread per face
 // (about 75 taps; three component groups in separate CTAs, which raised the
 // warps from 12 to 32 an SM, were slower, 2.2 times the instructions, and so
 // was taking the other direction's taps through shared memory, 467 us).  The walk over face slabs staged by TMA that this and
@@ -874,6 +901,15 @@ __device__ __forceinline__ void finalColumn(const Ctx& c, const RegArgs& rg, con
     for (int e = 0; e < 8; ++e) {
       xp[e] = __ldg(base + (F_X + e) * NF + st);
       qp[e] = __ldg(base + (F_QD + e) * NF + st);
+    }
+    // the next step's rows on their way to L1 (395 -> 351 us; the averages,
+    // at twice the warps, got slower with it)
+    if (step + 1 < steps) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        prefetch(base + (F_X + e) * NF + 2 * st);
+        prefetch(base + (F_QD + e) * NF + 2 * st);
+      }
     }
     // Z and the transverse differences of Y of place q: along the march (m)
     // and, for direction 0, along j (o)
@@ -966,18 +1002,22 @@ __global__ void __launch_bounds__(128, MB) o4FaceFinalKernel(const Ctx* __restri
 }
 
 // 9, 12b. Flux divergence of the three directions and the Powell source
-// (DivBPowell2's cell products) into rhs, one pass over the cells.
+// (DivBPowell2's cell products) into rhs, one pass over the cells.  HBM-bound
+// (64^3: 900 MB, 208 us); a launch that starts from rhs 0 (rg.fresh) neither
+// clears nor reads it, and in the RK4 step of a whole level the stage update
+// (rg.rk) follows in registers, so the stage rhs is not stored at all.
 __global__ void __launch_bounds__(128) o4CellKernel(const Ctx* __restrict__ tab, const RegArgs rg, const WorkChunk* __restrict__ wk) {
   const WorkChunk wc = wk[blockIdx.x];
   const Ctx& c = tab[wc.box * 3 + 0];
   const O4Args& a = c.a;
   const long NF = c.fr.N;
+  const double dt = rg.rk.stage < 0 ? 0.0 : rg.rk.invDtMax ? rg.rk.cfl / *rg.rk.invDtMax : rg.rk.dtv;
   forRegion(c.V, WALK_JK, wc, [&](int i, int j, int k) {
     double* R = a.rhs + roff(c.vr, i, j, k);
     const long fo = roff(c.fr, i, j, k);
     Rn kv[8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) kv[q] = R[q * c.vr.N];
+    for (int q = 0; q < 8; ++q) kv[q] = rg.fresh ? 0.0 : R[q * c.vr.N];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       const Rn coef = -a.scale / a.G.dx[d];
@@ -1002,8 +1042,13 @@ __global__ void __launch_bounds__(128) o4CellKernel(const Ctx* __restrict__ tab,
         kv[q] = kv[q] + value;
       }
     }
+    if (rg.rk.stage < 0) {
 #pragma unroll
-    for (int q = 0; q < 8; ++q) R[q * c.vr.N] = kv[q];
+      for (int q = 0; q < 8; ++q) R[q * c.vr.N] = kv[q];
+    } else {
+      const long N = c.vr.N, at = (long)a.block0 * 8 * N + roff(c.vr, i, j, k);
+      rkUpdate(rg.rk, dt, at, N, kv);
+    }
   });
 }
 
@@ -1313,14 +1358,14 @@ void o4SplitArgs(const O4Args& a, std::vector<O4Args>& out) {
 }
 
 cudaError_t launchO4BatchGravity(const O4Batch* B, cudaStream_t s) {
-  const RegArgs none{};
+  const RegArgs none;
   if (B->chunkCount[RG_V] == 0) return cudaSuccess;
   o4GravityKernel<<<B->chunkCount[RG_V], 128, 0, s>>>(B->dev, none, B->chunks + B->chunkOff[RG_V]);
   return cudaGetLastError();
 }
 
 cudaError_t launchO4Batch(const O4Batch* B, const RegArgs* reg, cudaStream_t s) {
-  const RegArgs none{};
+  const RegArgs none;
   const RegArgs rg = reg ? *reg : none;
   cudaError_t e = cudaSuccess;
   using Kernel = void (*)(const Ctx*, const RegArgs, const WorkChunk*);
@@ -1347,7 +1392,7 @@ cudaError_t launchO4Batch(const O4Batch* B, const RegArgs* reg, cudaStream_t s) 
                                                 o4FaceFinalKernel<kO4MinBlocks[2][2]>};
   launch(o4PrimAvgKernel, RG_G, s);
   launch(o4ThetaRawKernel, RG_GR, s);
-  launch(o4PointKernel, RG_G, s);
+  launch(o4PointKernel, RG_GR, s);
   if (B->powell) {
     fork(B->pointEv);
     launch(o4PowellAvgKernel, RG_V1, B->side);

@@ -306,27 +306,18 @@ __global__ void o4NativeKernel(const O4StageIO io) {
   }
 }
 
-// RK4 update after stage s (the tableau of src/MHD_AMRRungeKutta.H:10-12).
-__global__ void o4UpdateKernel(const O4Level O, int stage, const double* __restrict__ k, double* __restrict__ ju,
-                               double* __restrict__ acc, double* __restrict__ next, const double* invDtMax, double cfl,
-                               double dtv) {
-  const double b4[4] = {1.0 / 6, 1.0 / 3, 1.0 / 3, 1.0 / 6};
-  const double a4[4] = {0.5, 0.5, 1.0, 0.0};
-  const double dt = invDtMax ? cfl / *invDtMax : dtv;
-  const double fb = dt * b4[stage], fa = dt * a4[stage];
-  const long n = 6L * 8 * O.Nv;
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
-    const double kv = k[t];
-    if (stage == 0) {
-      const double u = ju[t];
-      acc[t] = u + fb * kv;
-      next[t] = u + fa * kv;
-    } else if (stage < 3) {
-      acc[t] += fb * kv;
-      next[t] = ju[t] + fa * kv;
-    } else {
-      ju[t] = acc[t] + fb * kv;
-    }
+// RK4 update after a stage from a stored rhs (ensembles, and levels whose
+// operator covers a radial window).
+__global__ void o4UpdateKernel(const O4Level O, const RkUpdate u, const double* __restrict__ k) {
+  const double dt = u.invDtMax ? u.cfl / *u.invDtMax : u.dtv;
+  const unsigned n = (unsigned)(6L * O.Nv), nv = (unsigned)O.Nv;
+  HC_LEVEL_LOOP(t, n) {
+    const unsigned b = t / nv;
+    const long at = (long)b * 8 * O.Nv + (t - b * nv);
+    Rn kv[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) kv[q] = __ldg(k + at + q * O.Nv);
+    rkUpdate(u, dt, at, O.Nv, kv);
   }
 }
 
@@ -383,9 +374,8 @@ cudaError_t launchO4Prepare(const O4StageIO& io, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launchO4Update(const O4Level& O, int stage, const double* k, double* ju, double* acc, double* next,
-                           const double* invDtMax, double cfl, double dtv, cudaStream_t s) {
-  o4UpdateKernel<<<blocksFor(6L * 8 * O.Nv), kThreads, 0, s>>>(O, stage, k, ju, acc, next, invDtMax, cfl, dtv);
+cudaError_t launchO4Update(const O4Level& O, const RkUpdate& u, const double* k, cudaStream_t s) {
+  o4UpdateKernel<<<blocksFor(6L * O.Nv), kThreads, 0, s>>>(O, u, k);
   return cudaGetLastError();
 }
 
