@@ -80,7 +80,7 @@ def launches_per_step(args) -> int:
     if args.order == 2:
         return 11  # prim + cfl + 4 x (ghosts, stage) + time (prologue in every 1-step call)
     operator = operator_launches(args)
-    per_stage = 4 + int(args.gravity) + operator + 1               # prepare, gravity, operator, update
+    per_stage = 4 + int(args.gravity) + operator                   # prepare, gravity, operator with the update
     return 1 + 4 * per_stage + 2 + 1                               # cfl, stages, reflux, time
 
 
@@ -701,7 +701,7 @@ def serve_launches(reqs, cohort_steps: int | None = None) -> int:
         a = argparse.Namespace(order=r.order, riemann=2 if r.order == 4 else 1, gravity=0)
         per_step = launches_per_step(a)
         if cohort_steps is not None and r.order == 4:
-            per_step -= 4 * operator_launches(a)
+            per_step -= 4 * (operator_launches(a) - 1)  # the update is a kernel of its own here
         total += 3 + per_step * r.steps
     if cohort_steps:
         total += 4 * operator_launches(argparse.Namespace(riemann=2)) * cohort_steps
@@ -1157,7 +1157,7 @@ def main() -> int:
     ap.add_argument("--no-graph", dest="graph", action="store_false",
                     help="launch the step eagerly instead of replaying a captured CUDA graph")
     ap.add_argument("--o4-variants", default=None, metavar="R,P,F",
-                    help="order 4: use these register-cap variants of the reconstruction, Roe point and final-flux "
+                    help="order 4: use these register-cap variants of the reconstruction, Riemann and final-flux "
                          "kernels instead of timing them (for profiler runs)")
     ap.add_argument("--cpu-max-steps", type=int, default=60)
     ap.add_argument("--ref-budget", type=float, default=20.0)
