@@ -48,13 +48,16 @@ struct Chunk {
   int item, pad;
   long long begin, end;
 };
-// Elements per CTA: 4 per thread.  A list's items are boxes of some 500 to
-// 30,000 elements, so longer chunks (16,384) gave the small boxes of a level
+// Elements per CTA: a list's total over kListCtas, as a power of two from
+// kMinChunk (4 per thread) to kMaxChunk (64).  A list's items are boxes of some
+// 500 to 30,000 elements; 16,384 for every list gave the small boxes of a level
 // one CTA each, 31 dependent rounds in it and most SMs idle.  32 x 32^2 shell
-// with 192 boxes of 8^3, per launch: commit 148 -> 84 us (with its loads ahead
-// of its tests), mapped 88 -> 79, native 72 -> 58, copies 30 -> 26, the
-// tableau's combinations 44 -> 13.
-constexpr long long kChunk = 1024;
+// with 192 boxes of 8^3, per launch, 16,384 against 1,024: commit 148 -> 84 us
+// (with its loads ahead of its tests), mapped 88 -> 79, native 72 -> 58, copies
+// 30 -> 26, the tableau's combinations 44 -> 13.  Long lists keep long chunks:
+// 1962 boxes of 8.9 M cells, five combinations 1.66 ms at 1,024, 1.60 at 16,384;
+// commit of 576 boxes of 18^3 246 us at 1,024, 220 at 4,096.
+constexpr long long kMinChunk = 1024, kMaxChunk = 16384, kListCtas = 1184;
 
 __global__ void __launch_bounds__(kThreads) rkCombineKernel(const hc_rk_box* __restrict__ boxes,
                                                             const Chunk* __restrict__ chunks, const RkFactors F) {
@@ -514,7 +517,25 @@ int cudaFailed(cudaError_t e, const char* what) {
 }
 
 void addChunks(std::vector<Chunk>& out, int item, long long elems) {
-  for (long long b = 0; b < elems; b += kChunk) out.push_back(Chunk{item, 0, b, b + kChunk < elems ? b + kChunk : elems});
+  out.push_back(Chunk{item, 0, 0, elems});
+}
+
+// Splits a list's whole items; start holds each item's first chunk and follows.
+void splitChunks(std::vector<Chunk>& list, std::vector<int>* start) {
+  long long total = 0;
+  for (const Chunk& c : list) total += c.end;
+  long long step = kMinChunk;
+  while (step < kMaxChunk && step * kListCtas < total) step *= 2;
+  std::vector<Chunk> out;
+  std::vector<int> first;
+  for (const Chunk& c : list) {
+    first.push_back((int)out.size());
+    for (long long b = 0; b < c.end; b += step) out.push_back(Chunk{c.item, 0, b, b + step < c.end ? b + step : c.end});
+  }
+  first.push_back((int)out.size());
+  if (start)
+    for (int& q : *start) q = first[q];
+  list.swap(out);
 }
 
 int argFail(const char* msg) { return hc::setLastError(HC_ERR_ARG, msg); }
@@ -622,6 +643,8 @@ extern "C" int hc_amr_plan_create(hc_ctx* ctx, const hc_rk_box* boxes, int nbox,
     addChunks(rc, r, 8LL * (R.hi[0] - R.lo[0] + 1) * (R.hi[1] - R.lo[1] + 1) * (R.hi[2] - R.lo[2] + 1));
   }
   P->restrictChunkStart.push_back((int)rc.size());
+  splitChunks(bc, nullptr);
+  splitChunks(rc, &P->restrictChunkStart);
   P->nBoxChunks = (int)bc.size();
   cudaError_t e = cudaSuccess;
   if (!bc.empty()) {
@@ -691,6 +714,7 @@ extern "C" int hc_amr_plan_set_reflux(hc_amr_plan* P, const hc_reflux_box* patch
     addChunks(rc, r, 8LL * (R.hi[0] - R.lo[0] + 1) * (R.hi[1] - R.lo[1] + 1) * (R.hi[2] - R.lo[2] + 1));
   }
   start.push_back((int)rc.size());
+  splitChunks(rc, &start);
   hc_reflux_box* dev = nullptr;
   Chunk* devChunks = nullptr;
   cudaError_t e = cudaSuccess;
@@ -897,6 +921,7 @@ extern "C" int hc_amr_plan_set_cf_interp(hc_amr_plan* P, const hc_cf_box* boxes,
     addChunks(cc, b, (long long)boxes[b].fine_n[0] * boxes[b].fine_n[1] * boxes[b].fine_n[2]);
   }
   start.push_back((int)cc.size());
+  splitChunks(cc, &start);
   CfItem* dev = nullptr;
   Chunk* devChunks = nullptr;
   cudaError_t e = cudaSuccess;
@@ -1057,6 +1082,8 @@ extern "C" int hc_amr_plan_set_cf_fine(hc_amr_plan* P, const hc_cf_fine_box* box
   }
   ms.push_back((int)mc.size());
   qs.push_back((int)qc.size());
+  splitChunks(mc, &ms);
+  splitChunks(qc, &qs);
   hc_cf_fine_box* dev = nullptr;
   Chunk *devM = nullptr, *devQ = nullptr;
   cudaError_t e = cudaSuccess;
@@ -1221,6 +1248,7 @@ extern "C" int hc_amr_plan_set_native(hc_amr_plan* P, const hc_native_box* boxes
     addChunks(ch, b, (long long)boxes[b].usph_n[0] * boxes[b].usph_n[1] * boxes[b].usph_n[2]);
   }
   st.push_back((int)ch.size());
+  splitChunks(ch, &st);
   hc_native_box* dev = nullptr;
   Chunk* devC = nullptr;
   cudaError_t e = cudaSuccess;
@@ -1329,6 +1357,7 @@ extern "C" int hc_amr_plan_set_copies(hc_amr_plan* P, const hc_copy_box* copies,
     addChunks(cc, q, (long long)(C.hi[0] - C.lo[0] + 1) * (C.hi[1] - C.lo[1] + 1) * (C.hi[2] - C.lo[2] + 1));
   }
   start.push_back((int)cc.size());
+  splitChunks(cc, &start);
   hc_copy_box* dev = nullptr;
   Chunk* devChunks = nullptr;
   cudaError_t e = cudaSuccess;
