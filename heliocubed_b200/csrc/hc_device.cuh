@@ -8,6 +8,7 @@
 
 #include <cuda_runtime.h>
 #include <math.h>
+#include <math_constants.h>
 
 #include "hc_common.h"
 
@@ -73,11 +74,14 @@ HC_DEV double rsqrtN(double x) {
   const double e = fma(__dmul_rn(-x, y), y, 1.0);
   return fma(__dmul_rn(y, e), fma(0.375, e, 0.5), y);
 }
-// sqrt(x) with one Newton correction of x rsqrt(x) (good to the last bit),
-// 0 for x below 1e-290 (far below any squared speed).
+// sqrt(x) with one Newton correction of x rsqrt(x) (good to the last bit).
+// 0 for x below 1e-290 (far below any squared speed), negative ones
+// included; infinity and NaN are returned as they are, so an infinite speed
+// stays infinite.
 HC_DEV double sqrtN(double x) {
   const double y = rsqrtN(x), s = __dmul_rn(x, y);
-  return x > 1e-290 ? fma(0.5 * y, fma(-s, s, x), s) : 0.0;
+  const double root = fma(0.5 * y, fma(-s, s, x), s);
+  return x <= 1e-290 ? 0.0 : (x < CUDART_INF ? root : x);
 }
 
 // Half the limited slope of a cell with differences a, b to its neighbours
@@ -140,7 +144,7 @@ HC_DEV void rusanovDissipation(double out[8], const double* wl, const double* wr
     const Rn v2 = dot3(w[1], w[1], w[2], w[2], w[3], w[3]), b2 = dot3(w[5], w[5], w[6], w[6], w[7], w[7]);
     energy[side] = mad(0.5 * inv4Pi, b2, mad(0.5 * Rn(w[0]), v2, Rn(w[4]) * invGm1));
     const Rn x = mad(inv4Pi, b2, gamma * Rn(w[4])), xr = x * w[0];
-    const double fast = xr > 1e-290 ? __dmul_rn(x, rsqrtN(xr)) : sqrt(x.v / w[0]);
+    const double fast = xr > 1e-290 && xr < CUDART_INF ? __dmul_rn(x, rsqrtN(xr)) : sqrt(x.v / w[0]);
     speed = fmax(speed, Rn(fabs(w[1])) + fast);
   }
   const Rn s = speed;
@@ -209,9 +213,10 @@ __device__ __forceinline__ bool roe8Body(double out[8], const double* wl, const 
     hzz = BZ * rb;
     // The slow speed is a difference of nearly equal numbers where bb is
     // small; rounded as the reference rounds it (no fused product), so that
-    // h = szb and the slow speed is 0 where bb vanishes.
+    // h = szb and the slow speed is 0 where bb vanishes.  A NaN of overflowed
+    // squares counts as 0, as in the reference's maximum.
     const Rn szb = cc + (bb + k4 * BYZ2 * iRho);
-    const Rn h = sqrtN(szb * szb - 4.0 * cc * bb);
+    const Rn h = sqrtN(dmax(0.0, szb * szb - 4.0 * cc * bb));
     aas = 0.5 * (szb - h);
     aaf = 0.5 * (szb + h);
     if (aas <= 0.0) aas = 0.0;

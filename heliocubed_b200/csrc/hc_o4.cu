@@ -768,7 +768,7 @@ __global__ void __launch_bounds__(128, MB) o4FaceRiemannKernel(const Ctx* __rest
       const Rn rs = rsqrtN(rho), ce2 = a.G.gamma * Rn(p) * (rs * rs);
       const Rn aa = mad(kInv4Pi * b2, rs * rs, ce2);
       const Rn bb = Rn(fabs(bn.v)) * sqrtN(ce2) * rs * 0.56418958354775628694807945156077;  // 1 / sqrt(pi)
-      const Rn af = 0.5 * (Rn(sqrtN(aa + bb)) + sqrtN(aa - bb));
+      const Rn af = 0.5 * (Rn(sqrtN(dmax(0.0, aa + bb))) + sqrtN(dmax(0.0, aa - bb)));
       base[F_SPD * NF] = mad(af, sqrt(dot3(f[0], f[0], f[3], f[3], f[6], f[6]).v), fabs(0.5 * (Rn(l[1]) + r[1])));
     }
   }
