@@ -68,6 +68,8 @@ HC_DEV double rcpN(double x) {
   const double e = fma(-x, y, 1.0);
   return fma(y, fma(e, e, e), y);
 }
+// 1 / rho of a density: 0 for infinity, as the division gives.
+HC_DEV double rcpDensity(double rho) { return rho == CUDART_INF ? 0.0 : rcpN(rho); }
 HC_DEV double rsqrtN(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
@@ -364,14 +366,16 @@ HC_DEV void cartesianPrimitiveFromConserved(double out[8], const double in[8], d
 #pragma unroll
   for (int c = 0; c < 8; ++c) u[c] = Rn(in[c]) * inverseJ;
   const Rn rho = u[0] < kMP / 100 ? kMP / 100 : u[0].v;
-  const Rn inv = rcpN(rho);
+  const Rn inv = rcpDensity(rho);
   out[0] = rho;
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     out[1 + d] = u[1 + d] * inv;
     out[5 + d] = u[5 + d];
   }
-  const Rn m2 = dot3(u[1], out[1], u[2], out[2], u[3], out[3]), b2 = dot3(u[5], u[5], u[6], u[6], u[7], u[7]);
+  // rho |v|^2 as m . v, but inf * 0 (no kinetic energy at all) of an infinite density
+  const Rn m2 = inv.v == 0.0 ? CUDART_NAN : dot3(u[1], out[1], u[2], out[2], u[3], out[3]).v;
+  const Rn b2 = dot3(u[5], u[5], u[6], u[6], u[7], u[7]);
   const Rn pressure = (gamma - 1.0) * (mad(-0.5, m2, u[4]) - (0.125 / kPi) * b2);
   out[4] = pressure < 0.0 ? 0.0 : pressure.v;
 }

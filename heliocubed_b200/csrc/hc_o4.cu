@@ -197,7 +197,7 @@ __device__ __forceinline__ double radialPoint(const O4Geo& g, int d, int i) {
 constexpr double kInv4Pi = 0.25 / kPi, kInv8Pi = 0.125 / kPi;
 // f_sphToPrim + energies + pressure (src/BoxOp_BertaCubedSphereImplem.H:212-340)
 __device__ __forceinline__ void sphToPrim(const double u[8], const double* A, double gamma, double w[8]) {
-  const Rn rho = dmax(u[0], kRHO00), inv = rcpN(rho);
+  const Rn rho = dmax(u[0], kRHO00), inv = rcpDensity(rho);
   w[0] = rho;
   Rn ke = 0.0, me = 0.0;
 #pragma unroll

@@ -70,6 +70,10 @@ def test_operator_of_an_infinite_speed(oracle_lib, riemann, component, value):
 @pytest.mark.parametrize("riemann,fallback,component,value", [(1, 0, 4, np.inf), (1, 1, 4, np.inf), (2, 1, 4, np.inf),
                                                               (2, 0, 4, 1e200)])
 def test_o4_operator_of_an_infinite_speed(oracle_lib, riemann, fallback, component, value):
+    _check_o4_box(oracle_lib, riemann, fallback, component, value)
+
+
+def _check_o4_box(oracle_lib, riemann, fallback, component, value):
     sh, orc = _pair(oracle_lib, spatial_order=4, riemann_solver=riemann, berta_fallback_type=fallback)
     lo, hi = (6, 4, 3), (11, 9, 10)
     v = [h - low + 1 for low, h in zip(lo, hi)]
@@ -84,3 +88,19 @@ def test_o4_operator_of_an_infinite_speed(oracle_lib, riemann, fallback, compone
     got = torch.zeros(want.size, dtype=torch.float64, device="cuda")
     sh.box_rhs_o4(make_box(lo, hi, 5, 1), torch.from_numpy(u).cuda(), got)
     _assert_same(got.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("riemann,fallback", [(1, 0), (2, 0), (1, 1), (2, 1)])
+def test_o4_operator_of_an_infinite_density(oracle_lib, riemann, fallback):
+    """The cell is at rest: its finite momenta over the density are 0."""
+    _check_o4_box(oracle_lib, riemann, fallback, 0, np.inf)
+
+
+def test_primitives_of_an_infinite_density(oracle_lib):
+    sh, orc = _pair(oracle_lib)
+    ju = sh.init_perturbed_wind(5)
+    ju.view(6, 8, NA, NA, NR)[3, 0, 7, 5, 9] = np.inf
+    cell = (3, slice(None), 9, 7, 11)  # two ghosts
+    got, want = (w.reshape(6, 8, NA + 4, NA + 4, NR + 4)[cell]
+                 for w in (sh.prepare(ju).cpu().numpy(), orc.prepare(ju.cpu().numpy(), 0.0)))
+    assert np.array_equal(got[1:4], np.zeros(3)) and np.array_equal(np.isfinite(got), np.isfinite(want))
