@@ -91,7 +91,13 @@ HC_DEV double sqrtN(double x) {
 // 2), 3 monotonized central: the smaller of |a + b| / 4 and min(|a|, |b|)
 // with the differences' sign, 0 where they differ in sign.  The candidates
 // keep their signs through the selection, so no sign is taken off and put
-// back; a NaN difference gives NaN.
+// back.  Where the product of the differences is NaN the reference takes
+// std::min / std::max of the two: NaN for a NaN a, a for a NaN b (a NaN cell
+// does not reach past the faces next to it), and of 0 and an infinity 0, but
+// infinity for 0 and +inf.  That value (odd) is formed for every face with one
+// product and an integer selection, ahead of the choice: from comparisons, in
+// a branch, or inside the choice it made the second-order steps 4 to 37 %
+// slower.
 template <int LIM>
 HC_DEV Rn halfSlope(Rn a, Rn b) {
   const Rn q = 0.25 * (a + b);
@@ -99,7 +105,10 @@ HC_DEV Rn halfSlope(Rn a, Rn b) {
   const double small = fabs(b.v) < fabs(a.v) ? b.v : a.v;
   const double t = LIM == 1 ? 0.5 * small : (fabs(small) < fabs(q.v) ? small : q.v);
   const double sign = a * b;
-  return sign > 0.0 ? t : (sign <= 0.0 ? 0.0 : sign);
+  const double h = 0.5 * small;
+  const double odd =
+      __hiloint2double(__double2hiint(b.v) == 0x7ff00000 ? 0x7ff00000 : __double2hiint(h), __double2loint(h));
+  return sign > 0.0 ? t : (sign <= 0.0 ? 0.0 : odd);
 }
 
 // Left and right states of a face from its four cells, one component.

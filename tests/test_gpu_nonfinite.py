@@ -60,8 +60,27 @@ def _assert_same(got, want):
 @pytest.mark.parametrize("riemann,component,value", [(1, 4, np.inf), (2, 4, np.inf), (2, 4, 1e200), (1, 6, 1e200),
                                                      (2, 6, -1e200)])
 def test_operator_of_an_infinite_speed(oracle_lib, riemann, component, value):
-    sh, orc = _pair(oracle_lib, riemann_solver=riemann)
+    _check_level(oracle_lib, 3, riemann, component, value)
+
+
+@pytest.mark.parametrize("limiter,riemann", [(0, 1), (1, 1), (2, 2), (3, 1), (3, 2)])
+@pytest.mark.parametrize("component,value", [(0, np.nan), (1, np.nan), (3, -np.inf), (4, np.nan), (6, np.nan)])
+def test_limiter_of_a_bad_cell(oracle_lib, limiter, riemann, component, value):
+    _check_level(oracle_lib, limiter, riemann, component, value)
+
+
+@pytest.mark.parametrize("limiter", [1, 3])
+@pytest.mark.parametrize("value", [np.inf, -np.inf])
+def test_limiter_of_an_infinity_in_a_flat_field(oracle_lib, limiter, value):
+    """Differences 0 and infinity."""
+    _check_level(oracle_lib, limiter, 1, 6, value, flat=True)
+
+
+def _check_level(oracle_lib, limiter, riemann, component, value, flat=False):
+    sh, orc = _pair(oracle_lib, limiter=limiter, riemann_solver=riemann)
     w = orc.prepare(sh.init_perturbed_wind(5).cpu().numpy(), 0.0)
+    if flat:
+        w.reshape(6, 8, -1)[:, component] = 0.0
     w.reshape(6, 8, NA + 4, NA + 4, NR + 4)[2, component, 7, 6, 9] = value
     got = sh.rhs(torch.from_numpy(w).cuda()).cpu().numpy()
     _assert_same(got.reshape(6, 8, -1).swapaxes(0, 1), orc.rhs(w).reshape(6, 8, -1).swapaxes(0, 1))
