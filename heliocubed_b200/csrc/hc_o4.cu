@@ -252,8 +252,10 @@ __device__ __forceinline__ double normalizeStencil(double (&v)[N]) {
 // The weights do not change with the scale of the stencil (eps guards 0 / 0
 // only), so the stencil is scaled by the power of two of its largest value,
 // formed from the exponents in integer arithmetic: |v| < 2, every weight
-// lies in [1e-118, 1e9] and neither a product nor the reciprocal under- or
-// overflows.  A zero stencil gives zeros; a NaN or infinity gives NaN.
+// lies in [6e-119, 1e9], and neither the product of the sums nor its
+// reciprocal, nor the quotients formed before they are scaled back, under- or
+// overflow (values below 8e307, whose differences are finite).  A zero
+// stencil gives zeros; a NaN or infinity gives NaN.
 // The reconstruction is bound by instruction issue; sharing takes about 95
 // FP64 instructions per component and face where two separate sides with
 // divisions took 170 (64 x 32^2 x 6: 89 -> 70 us per direction).
@@ -283,9 +285,10 @@ __device__ __forceinline__ void wenozFace(const double v[6], double& L, double& 
   // mirrored; its e carry the opposite sign
   side(plus(t4, mad(3.0, d3, -d4)), plus(t3, d3 + d2), plus(t2, mad(3.0, d2, -d1)), mad(-3.0, d4, 7.0 * d3),
        mad(3.0, d2, d3), mad(5.0, d2, -d1), nr, dr);
-  const Rn q = scale8 * Rn(rcpN(dl * dr));
-  L = mad(nl * dr, q, v[2]);
-  R = mad(-(nr * dl), q, v[3]);
+  // the quotients first: the reciprocal of a constant stencil is near 1e234
+  const Rn q = rcpN(dl * dr);
+  L = mad(nl * dr * q, scale8, v[2]);
+  R = mad(-(nr * dl) * q, scale8, v[3]);
 }
 
 // f_weno3_pointwise_faceF (:881-946), one component, cells W[i-2..i+1].
