@@ -325,10 +325,12 @@ __device__ __forceinline__ double cflRate(const DevLevel& L, int b, int i, int j
   return rate;
 }
 
-// Max over a warp (std::max order: a NaN candidate never replaces the max),
+// Max over a warp (std::max order: a NaN candidate never replaces the max;
+// it leaves the exchange at once, or its lane would not pass the others on),
 // then one atomic per warp on the bit pattern (non-negative doubles order as
 // unsigned integers).
 __device__ __forceinline__ void warpMaxAtomic(double v, unsigned long long* out) {
+  v = v > 0 ? v : 0.0;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const double other = __shfl_xor_sync(0xffffffffu, v, o);

@@ -46,6 +46,27 @@ def test_cfl_rate_of_a_bad_cell(oracle_lib, component, value):
         assert same, (cell, got, want)
 
 
+def test_time_step_beside_a_nan_cell():
+    """The rate that a step leaves for the next one: the largest of the finite
+    cells, also where a warp's first lane is a NaN cell (i = 0; the fastest
+    cell is 12 cells further in the same row)."""
+    if not gpu_available():
+        pytest.skip("no CUDA device")
+    sh = hc.Shell(hc.Params(nr=32, na=NA))
+    first = sh.init_perturbed_wind(3)
+    v = first.view(6, 8, NA, NA, 32)
+    v[0, 4, 8, 8, 0] = np.nan
+    v[0, 4, 8, 8, 12] *= 1e4
+    one, two = first.clone(), first.clone()
+    t1, t2 = (torch.zeros(1, dtype=torch.float64, device="cuda") for _ in range(2))
+    sh.advance(one, 1, t1)
+    sh.advance(two, 2, t2)
+    rate = sh.inv_dt_max(one).item()
+    assert one.view(6, 8, NA, NA, 32)[0, :, 8, 8, 0].isnan().any() and 0 < rate < np.inf
+    dt = sh.params.cfl / rate
+    assert abs((t2 - t1).item() - dt) <= 1e-10 * dt
+
+
 def _assert_same(got, want):
     """Finite values in the same places, and there equal to 1e-12 of the
     component's largest."""
