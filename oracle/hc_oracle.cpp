@@ -1132,20 +1132,22 @@ void levelRk4(const Level& L, double* ju, double dt, double t) {
   }
 }
 
-// src/BoxOp_SecondOrderCFL.H:99-210 (no mapped scale, no cone density).
-double levelInvDt(const Level& L, const double* ju, double coneDensity = 0) {
+// src/BoxOp_SecondOrderCFL.H:99-210 (no mapped scale, no cone density), in the
+// arithmetic of R (double, or long double from the same tables).
+template <class R>
+R levelInvDtIn(const Level& L, const double* ju, R coneDensity) {
   const hc_params& P = L.P;
   LevelArrays I(L);
   const int nr = L.nr, na = L.na;
-  const double gamma = P.gamma, h = L.h;
-  double gmax = 0;
-  (void)h;
+  const R gamma = P.gamma, h = R(1) / na, pi = R(3.14159265358979323846264338327950288L);
+  R gmax = 0;
 #pragma omp parallel for collapse(2) reduction(max : gmax) schedule(static)
   for (int b = 0; b < 6; ++b)
     for (int k = 0; k < na; ++k)
       for (int j = 0; j < na; ++j) {
         size_t cidx = L.cellIdx(b, j, k);
-        double inverseDet = 1.0 / L.det[cidx], dA[3][3], inverseDetA[3][3], cell[3][3], face[2][3][3];
+        const R inverseDet = R(1) / L.det[cidx];
+        double dA[3][3], inverseDetA[3][3], cell[3][3], face[2][3][3];
         double fdet[3], normal[3];
         for (int r = 0; r < 3; ++r) for (int s = 0; s < 3; ++s) { dA[r][s] = L.detAA[cidx * 9 + r * 3 + s]; cell[r][s] = L.cellBasis[cidx * 9 + r * 3 + s]; }
         inverse3(dA, inverseDetA);
@@ -1156,51 +1158,55 @@ double levelInvDt(const Level& L, const double* ju, double coneDensity = 0) {
         }
         for (int i = 0; i < nr; ++i) {
           const Radial& r = L.rad(i);
-          const double inverseVolume = 1.0 / r.vol, width0 = r.Dr0 * (1.0 / shellCells(L.P));
+          const R inverseVolume = R(1) / r.vol, width0 = r.Dr0 * (R(1) / shellCells(L.P));
           const double area[3] = {r.area0, r.areaT, r.areaT};
           double u[8];
           for (int c = 0; c < NC; ++c) u[c] = ju[I.v(b, c, i, j, k)];
-          double rho = u[0] * inverseDet;
+          R rho = u[0] * inverseDet;
           rho *= inverseVolume;
-          rho = std::max(rho, RHO00);
-          double energy = u[4] * inverseDet;
+          rho = std::max(rho, R(RHO00));
+          R energy = u[4] * inverseDet;
           energy *= inverseVolume;
-          double v[3] = {}, bb[3] = {};
+          R v[3] = {}, bb[3] = {};
           for (int d = 0; d < 3; ++d) {
             for (int q = 0; q < 3; ++q) { v[d] += inverseDetA[d][q] * u[1 + q]; bb[d] += inverseDetA[d][q] * u[5 + q]; }
             v[d] *= inverseVolume; bb[d] *= inverseVolume;
             v[d] /= rho;
           }
-          double vc[3] = {}, bc[3] = {}, kinetic = 0, magnetic = 0, b2 = 0;
+          R vc[3] = {}, bc[3] = {}, kinetic = 0, magnetic = 0, b2 = 0;
           for (int d = 0; d < 3; ++d) {
             for (int q = 0; q < 3; ++q) { vc[d] += cell[d][q] * v[q]; bc[d] += cell[d][q] * bb[q]; }
             kinetic += vc[d] * vc[d] / 2;
-            magnetic += bc[d] * bc[d] / 8.0 / M_PI;
+            magnetic += bc[d] * bc[d] / 8.0 / pi;
             b2 += bc[d] * bc[d];
           }
           kinetic *= rho;
-          double pressure = (energy - kinetic - magnetic) * (gamma - 1);
+          R pressure = (energy - kinetic - magnetic) * (gamma - 1);
           if (pressure < 0) pressure = 0;
-          double inverseDt = 0;
+          R inverseDt = 0;
           for (int d = 0; d < 3; ++d) {
             const double (*basis)[3] = d == 0 ? cell : face[d - 1];
-            double v2 = 0, fullB2 = 0;
+            R v2 = 0, fullB2 = 0;
             for (int q = 0; q < 3; ++q) {
-              double velocity = 0, field = 0;
+              R velocity = 0, field = 0;
               for (int s = 0; s < 3; ++s) { velocity += basis[q][s] * v[s]; field += basis[q][s] * bb[s]; }
               v2 += velocity * velocity;
               fullB2 += field * field;
             }
-            const double width = d == 0 ? width0 : r.vol * fdet[d] * h / area[d] / normal[d];
+            const R width = d == 0 ? width0 : r.vol * fdet[d] * h / area[d] / normal[d];
             // src/BoxOp_SecondOrderCFL.H:196-200
-            const double magneticDensity = coneDensity > 0 ? std::min(rho, coneDensity) : rho;
-            const double wave = std::sqrt(gamma * pressure / rho + fullB2 / 4.0 / M_PI / magneticDensity);
+            const R magneticDensity = coneDensity > 0 ? std::min(rho, coneDensity) : rho;
+            const R wave = std::sqrt(gamma * pressure / rho + fullB2 / 4.0 / pi / magneticDensity);
             inverseDt += (wave + std::sqrt(v2)) / width;
           }
           gmax = std::max(gmax, inverseDt);
         }
       }
   return gmax;
+}
+
+double levelInvDt(const Level& L, const double* ju, double coneDensity = 0) {
+  return levelInvDtIn<double>(L, ju, coneDensity);
 }
 
 // src/BoxOp_EulerCubedSphereImplem.H:817-876
@@ -1486,6 +1492,11 @@ int orc_level_prepare(void* L, const double* ju, double* w, double t) { levelPre
 int orc_level_rhs(void* L, const double* w, double* k) { levelRhs(*static_cast<Level*>(L), w, k); return 0; }
 int orc_level_rk4_step(void* L, double* ju, double dt, double t) { levelRk4(*static_cast<Level*>(L), ju, dt, t); return 0; }
 double orc_level_inv_dt(void* L, const double* ju) { return levelInvDt(*static_cast<Level*>(L), ju); }
+// (rate - reference) / reference with the reference in extended precision
+double orc_level_inv_dt_error(void* L, const double* ju, double rate) {
+  const long double ref = levelInvDtIn<long double>(*static_cast<Level*>(L), ju, 0.0L);
+  return (double)((rate - ref) / ref);
+}
 int orc_level_valid(void* L, const double* ju) { return levelValid(*static_cast<Level*>(L), ju); }
 int orc_level_init(void* L, const hc_init* in, double* ju) { levelInit(*static_cast<Level*>(L), *in, ju); return 0; }
 // The CFL rate with the cone density floor of the inlet cones active at t

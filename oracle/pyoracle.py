@@ -111,6 +111,8 @@ def lib() -> C.CDLL:
         L.orc_level_rk4_step.argtypes = [C.c_void_p, _D, C.c_double, C.c_double]
         L.orc_level_inv_dt.restype = C.c_double
         L.orc_level_inv_dt.argtypes = [C.c_void_p, _D]
+        L.orc_level_inv_dt_error.restype = C.c_double
+        L.orc_level_inv_dt_error.argtypes = [C.c_void_p, _D, C.c_double]
         L.orc_level_valid.argtypes = [C.c_void_p, _D]
         L.orc_level_init.argtypes = [C.c_void_p, C.POINTER(HcInit), _D]
         L.orc_geometry.restype = C.c_long
@@ -274,6 +276,10 @@ class OracleLevel:
 
     def inv_dt(self, ju: np.ndarray) -> float:
         return self.L.orc_level_inv_dt(self.h, dptr(ju))
+
+    def inv_dt_error(self, ju: np.ndarray, rate: float) -> float:
+        """Relative error of a CFL rate against extended precision."""
+        return self.L.orc_level_inv_dt_error(self.h, dptr(ju), rate)
 
     def valid(self, ju: np.ndarray) -> bool:
         return bool(self.L.orc_level_valid(self.h, dptr(ju)))
