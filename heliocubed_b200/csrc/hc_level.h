@@ -290,7 +290,7 @@ struct RegArgs {
 struct O4Batch;
 // Register-cap variants of the operator's three face kernels
 // (reconstruction, Riemann problem, final flux), chosen by the
-// autotuner; results do not depend on them.
+// autotuner; results do not depend on them (bit for bit).
 constexpr int kO4TunedKernels = 3, kO4Variants = 3;
 void o4BatchSetVariants(O4Batch* b, const int v[kO4TunedKernels]);
 int o4VariantMinBlocks(int kernel, int variant);

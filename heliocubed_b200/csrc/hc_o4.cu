@@ -185,10 +185,10 @@ __device__ __forceinline__ double adjDr(const O4Geo& g, int d, int i) {
   const double4 r = radialRow(g, i);
   return d == 0 ? r.x : r.y;
 }
-__device__ __forceinline__ double radialPoint(const O4Geo& g, int d, int i) {
+__device__ __forceinline__ Rn radialPoint(const O4Geo& g, int d, int i) {
   if (d == 0) return adjDr(g, 0, i);
-  const double a = adjDr(g, d, i);
-  return a - (1.0 / 24.0) * (adjDr(g, d, i + 1) - 2.0 * a + adjDr(g, d, i - 1));
+  const Rn a = adjDr(g, d, i);
+  return mad(-1.0 / 24.0, mad(-2.0, a, adjDr(g, d, i + 1)) + adjDr(g, d, i - 1), a);
 }
 
 // ---- pointwise pieces -----------------------------------------------------
