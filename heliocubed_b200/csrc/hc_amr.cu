@@ -341,9 +341,13 @@ __global__ void __launch_bounds__(kThreads) cfPassKernel(const CfItem* __restric
   }
 }
 
-__global__ void __launch_bounds__(kThreads) cfCommitKernel(const CfItem* __restrict__ items,
-                                                           const Chunk* __restrict__ chunks,
-                                                           const double* __restrict__ scratch) {
+// Four CTAs an SM: with sixteen components in registers it took 196 of them,
+// one CTA an SM, and 225 us for 576 boxes of 20^3 and eight components; eight
+// and their loads ahead of the test take 62 and 100 us (one component after
+// the other 180).
+__global__ void __launch_bounds__(kThreads, 4) cfCommitKernel(const CfItem* __restrict__ items,
+                                                              const Chunk* __restrict__ chunks,
+                                                              const double* __restrict__ scratch) {
   const Chunk ch = chunks[blockIdx.x];
   const CfItem& it = items[ch.item];
   const hc_cf_box B = it.box;
@@ -356,17 +360,22 @@ __global__ void __launch_bounds__(kThreads) cfCommitKernel(const CfItem* __restr
     bool inside = true;
     for (int d = 0; d < 3; ++d) inside = inside && p[d] >= B.valid_lo[d] && p[d] <= B.valid_hi[d];
     if (inside) continue;
-    // all components are loaded before the first test (at most kCfMaxComp)
-    double v[kCfMaxComp];
+    // eight components are loaded before the first test; a ninth and more are
+    // tested first and read again for the store
+    const double* from = res + t;
+    double* to = B.fine + t;
+    double v[8];
     bool finite = true;
 #pragma unroll
-    for (int c = 0; c < kCfMaxComp; ++c) v[c] = c < B.ncomp ? res[(long long)c * fineN + t] : 0.0;
+    for (int c = 0; c < 8; ++c) v[c] = c < B.ncomp ? from[c * fineN] : 0.0;
 #pragma unroll
-    for (int c = 0; c < kCfMaxComp; ++c) finite = finite && isfinite(v[c]);
+    for (int c = 0; c < 8; ++c) finite = finite && isfinite(v[c]);
+    for (int c = 8; c < B.ncomp; ++c) finite = finite && isfinite(from[c * fineN]);
     if (!finite) continue;
 #pragma unroll
-    for (int c = 0; c < kCfMaxComp; ++c)
-      if (c < B.ncomp) B.fine[(long long)c * fineN + t] = v[c];
+    for (int c = 0; c < 8; ++c)
+      if (c < B.ncomp) to[c * fineN] = v[c];
+    for (int c = 8; c < B.ncomp; ++c) to[c * fineN] = from[c * fineN];
   }
 }
 
@@ -482,9 +491,12 @@ __global__ void __launch_bounds__(kThreads) cfQuotientKernel(const hc_cf_fine_bo
   }
 }
 
-// Region copies with a signed-permutation index map (exchanges).
-__global__ void __launch_bounds__(kThreads) copyKernel(const hc_copy_box* __restrict__ items,
-                                                       const Chunk* __restrict__ chunks) {
+// Region copies with a signed-permutation index map (exchanges).  Four CTAs an
+// SM (64 registers; 122 uncapped, and then two): the three copy lists of the
+// 576-box step take 104, 40 and 15 us, uncapped 145, 80 and 15, with each
+// component stored before the next is loaded 150, 61 and 18.
+__global__ void __launch_bounds__(kThreads, 4) copyKernel(const hc_copy_box* __restrict__ items,
+                                                          const Chunk* __restrict__ chunks) {
   const Chunk ch = chunks[blockIdx.x];
   const hc_copy_box B = items[ch.item];
   const int n0 = B.hi[0] - B.lo[0] + 1, n1 = B.hi[1] - B.lo[1] + 1;
@@ -498,13 +510,15 @@ __global__ void __launch_bounds__(kThreads) copyKernel(const hc_copy_box* __rest
     const long long so = boxOff(B.src_lo, B.src_n, x[0], x[1], x[2]);
     const long long dO = boxOff(B.dst_lo, B.dst_n, y[0], y[1], y[2]);
     // eight components' loads before their stores (the arrays may be one)
+    const double* src = B.src + so;
+    double* dst = B.dst + dO;
     for (int c = 0; c < B.ncomp; c += 8) {
       double v[8];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) v[e] = c + e < B.ncomp ? B.src[(c + e) * sN + so] : 0.0;
+      for (int e = 0; e < 8; ++e, src += sN) v[e] = c + e < B.ncomp ? *src : 0.0;
 #pragma unroll
-      for (int e = 0; e < 8; ++e)
-        if (c + e < B.ncomp) B.dst[(c + e) * dN + dO] = v[e];
+      for (int e = 0; e < 8; ++e, dst += dN)
+        if (c + e < B.ncomp) *dst = v[e];
     }
   }
 }
