@@ -48,16 +48,25 @@ struct Chunk {
   int item, pad;
   long long begin, end;
 };
-// Elements per CTA: a list's total over kListCtas, as a power of two from
-// kMinChunk (4 per thread) to kMaxChunk (64).  A list's items are boxes of some
-// 500 to 30,000 elements; 16,384 for every list gave the small boxes of a level
-// one CTA each, 31 dependent rounds in it and most SMs idle.  32 x 32^2 shell
-// with 192 boxes of 8^3, per launch, 16,384 against 1,024: commit 148 -> 84 us
-// (with its loads ahead of its tests), mapped 88 -> 79, native 72 -> 58, copies
-// 30 -> 26, the tableau's combinations 44 -> 13.  Long lists keep long chunks:
-// 1962 boxes of 8.9 M cells, five combinations 1.66 ms at 1,024, 1.60 at 16,384;
-// commit of 576 boxes of 18^3 246 us at 1,024, 220 at 4,096.
-constexpr long long kMinChunk = 1024, kMaxChunk = 16384, kListCtas = 1184;
+// Elements per CTA: a list's total over about as many CTAs as two waves of its
+// kernel take, as a power of two from kMinChunk (4 per thread) to kMaxChunk
+// (64), and each item in equal pieces below that.  The copying kernels have
+// four to eight CTAs an SM, the conversions (85 to 128 registers) two.  A
+// list's items are boxes of some 500 to 30,000 elements; 16,384 for every list
+// gave the small boxes of a level one CTA each, 31 dependent rounds in it and
+// most SMs idle.
+// us per launch of two-level steps:
+//                                     one CTA a box   592 CTAs   1,184 CTAs
+//   192 boxes of 8^3  mapped               88                        79
+//                     native               72                        58
+//                     combinations         44                        13
+//   576 boxes of 8^3  mapped              152           152         170
+//                     native              146           145         153
+//                     commit of 20^3      179           115          97
+//                     combinations         53            53          37
+// (576 boxes' native in 1,184 unequal pieces, 4,096 + 1,736 elements: 169).
+constexpr long long kMinChunk = 1024, kMaxChunk = 16384;
+constexpr long long kListCtas = 148 * 8, kConversionCtas = 148 * 4;
 
 __global__ void __launch_bounds__(kThreads) rkCombineKernel(const hc_rk_box* __restrict__ boxes,
                                                             const Chunk* __restrict__ chunks, const RkFactors F) {
@@ -530,21 +539,26 @@ int cudaFailed(cudaError_t e, const char* what) {
   return hc::setLastError(HC_ERR_CUDA, msg);
 }
 
-void addChunks(std::vector<Chunk>& out, int item, long long elems) {
+// An item as one chunk; splitChunks cuts the whole list.
+void addItem(std::vector<Chunk>& out, int item, long long elems) {
   out.push_back(Chunk{item, 0, 0, elems});
 }
 
-// Splits a list's whole items; start holds each item's first chunk and follows.
-void splitChunks(std::vector<Chunk>& list, std::vector<int>* start) {
+// Splits a list's whole items for about `ctas` CTAs; start holds each item's
+// first chunk and follows.
+void splitChunks(std::vector<Chunk>& list, std::vector<int>* start, long long ctas) {
   long long total = 0;
   for (const Chunk& c : list) total += c.end;
   long long step = kMinChunk;
-  while (step < kMaxChunk && step * kListCtas < total) step *= 2;
+  while (step < kMaxChunk && step * ctas < total) step *= 2;
   std::vector<Chunk> out;
   std::vector<int> first;
   for (const Chunk& c : list) {
     first.push_back((int)out.size());
-    for (long long b = 0; b < c.end; b += step) out.push_back(Chunk{c.item, 0, b, b + step < c.end ? b + step : c.end});
+    // equal pieces of whole rounds of a CTA (step is a multiple of one)
+    const long long pieces = (c.end + step - 1) / step;
+    const long long len = pieces ? ((c.end + pieces - 1) / pieces + kThreads - 1) / kThreads * kThreads : 0;
+    for (long long b = 0; b < c.end; b += len) out.push_back(Chunk{c.item, 0, b, b + len < c.end ? b + len : c.end});
   }
   first.push_back((int)out.size());
   if (start)
@@ -650,15 +664,15 @@ extern "C" int hc_amr_plan_create(hc_ctx* ctx, const hc_rk_box* boxes, int nbox,
     }
   }
   std::vector<Chunk> bc, rc;
-  for (int b = 0; b < nbox; ++b) addChunks(bc, b, 8 * boxes[b].ncells);
+  for (int b = 0; b < nbox; ++b) addItem(bc, b, 8 * boxes[b].ncells);
   for (int r = 0; r < nrestrict; ++r) {
     const hc_restrict_box& R = restricts[r];
     P->restrictChunkStart.push_back((int)rc.size());
-    addChunks(rc, r, 8LL * (R.hi[0] - R.lo[0] + 1) * (R.hi[1] - R.lo[1] + 1) * (R.hi[2] - R.lo[2] + 1));
+    addItem(rc, r, 8LL * (R.hi[0] - R.lo[0] + 1) * (R.hi[1] - R.lo[1] + 1) * (R.hi[2] - R.lo[2] + 1));
   }
   P->restrictChunkStart.push_back((int)rc.size());
-  splitChunks(bc, nullptr);
-  splitChunks(rc, &P->restrictChunkStart);
+  splitChunks(bc, nullptr, kListCtas);
+  splitChunks(rc, &P->restrictChunkStart, kListCtas);
   P->nBoxChunks = (int)bc.size();
   cudaError_t e = cudaSuccess;
   if (!bc.empty()) {
@@ -725,10 +739,10 @@ extern "C" int hc_amr_plan_set_reflux(hc_amr_plan* P, const hc_reflux_box* patch
   for (int r = 0; r < npatch; ++r) {
     const hc_reflux_box& R = patches[r];
     start.push_back((int)rc.size());
-    addChunks(rc, r, 8LL * (R.hi[0] - R.lo[0] + 1) * (R.hi[1] - R.lo[1] + 1) * (R.hi[2] - R.lo[2] + 1));
+    addItem(rc, r, 8LL * (R.hi[0] - R.lo[0] + 1) * (R.hi[1] - R.lo[1] + 1) * (R.hi[2] - R.lo[2] + 1));
   }
   start.push_back((int)rc.size());
-  splitChunks(rc, &start);
+  splitChunks(rc, &start, kListCtas);
   hc_reflux_box* dev = nullptr;
   Chunk* devChunks = nullptr;
   cudaError_t e = cudaSuccess;
@@ -932,10 +946,10 @@ extern "C" int hc_amr_plan_set_cf_interp(hc_amr_plan* P, const hc_cf_box* boxes,
           for (int i = 0; i < 5; ++i) it.w[d][child][i] = 0.0;
       }
     start.push_back((int)cc.size());
-    addChunks(cc, b, (long long)boxes[b].fine_n[0] * boxes[b].fine_n[1] * boxes[b].fine_n[2]);
+    addItem(cc, b, (long long)boxes[b].fine_n[0] * boxes[b].fine_n[1] * boxes[b].fine_n[2]);
   }
   start.push_back((int)cc.size());
-  splitChunks(cc, &start);
+  splitChunks(cc, &start, kListCtas);
   CfItem* dev = nullptr;
   Chunk* devChunks = nullptr;
   cudaError_t e = cudaSuccess;
@@ -1089,15 +1103,15 @@ extern "C" int hc_amr_plan_set_cf_fine(hc_amr_plan* P, const hc_cf_fine_box* box
                      "mapped box equal to valid.grow(2), state and out on valid, a block containing valid and at "
                      "least 3 cells wide");
     ms.push_back((int)mc.size());
-    addChunks(mc, b, (long long)B.mapped_n[0] * B.mapped_n[1] * B.mapped_n[2]);
+    addItem(mc, b, (long long)B.mapped_n[0] * B.mapped_n[1] * B.mapped_n[2]);
     qs.push_back((int)qc.size());
-    addChunks(qc, b, (long long)(B.valid_hi[0] - B.valid_lo[0] + 1) * (B.valid_hi[1] - B.valid_lo[1] + 1) *
+    addItem(qc, b, (long long)(B.valid_hi[0] - B.valid_lo[0] + 1) * (B.valid_hi[1] - B.valid_lo[1] + 1) *
                          (B.valid_hi[2] - B.valid_lo[2] + 1));
   }
   ms.push_back((int)mc.size());
   qs.push_back((int)qc.size());
-  splitChunks(mc, &ms);
-  splitChunks(qc, &qs);
+  splitChunks(mc, &ms, kConversionCtas);
+  splitChunks(qc, &qs, kConversionCtas);
   hc_cf_fine_box* dev = nullptr;
   Chunk *devM = nullptr, *devQ = nullptr;
   cudaError_t e = cudaSuccess;
@@ -1259,10 +1273,10 @@ extern "C" int hc_amr_plan_set_native(hc_amr_plan* P, const hc_native_box* boxes
     if (!nativeShapeOk(boxes[b]))
       return argFail("hc_amr_plan_set_native: a box needs cart and usph arrays, a block 0..5 and non-empty boxes");
     st.push_back((int)ch.size());
-    addChunks(ch, b, (long long)boxes[b].usph_n[0] * boxes[b].usph_n[1] * boxes[b].usph_n[2]);
+    addItem(ch, b, (long long)boxes[b].usph_n[0] * boxes[b].usph_n[1] * boxes[b].usph_n[2]);
   }
   st.push_back((int)ch.size());
-  splitChunks(ch, &st);
+  splitChunks(ch, &st, kConversionCtas);
   hc_native_box* dev = nullptr;
   Chunk* devC = nullptr;
   cudaError_t e = cudaSuccess;
@@ -1368,10 +1382,10 @@ extern "C" int hc_amr_plan_set_copies(hc_amr_plan* P, const hc_copy_box* copies,
                      "region in the source box and the region's image in the destination box");
     start.push_back((int)cc.size());
     const hc_copy_box& C = copies[q];
-    addChunks(cc, q, (long long)(C.hi[0] - C.lo[0] + 1) * (C.hi[1] - C.lo[1] + 1) * (C.hi[2] - C.lo[2] + 1));
+    addItem(cc, q, (long long)(C.hi[0] - C.lo[0] + 1) * (C.hi[1] - C.lo[1] + 1) * (C.hi[2] - C.lo[2] + 1));
   }
   start.push_back((int)cc.size());
-  splitChunks(cc, &start);
+  splitChunks(cc, &start, kListCtas);
   hc_copy_box* dev = nullptr;
   Chunk* devChunks = nullptr;
   cudaError_t e = cudaSuccess;
