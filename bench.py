@@ -386,7 +386,7 @@ def measure_uniform(args, world, rank, local, e2e_min_steps: int = 4) -> dict:
     else:
         from heliocubed_b200.level import o4_variants
         mb = o4_variants()
-        names = ("reconstruction", "roe_point", "face_chain")
+        names = ("reconstruction", "riemann", "final_flux")
         if args.o4_variants:
             # fixed variants (profiling: timings taken under a profiler would
             # steer the tuner to a different choice than the plain run's)

@@ -32,8 +32,10 @@ disjoint, inside one panel with the six donor ghost layers inside it (no
 fine panel-seam interpolation is needed), and at least 10 fine cells from
 both radial boundaries (every ghost's coarse interpolation stencil inside
 the coarse level).  The coarse level is prepared by the uniform level's
-Cartesian conversion.  All arrays are allocated when the step is built; the
-first step also builds the coarse level's operator batch.
+Cartesian conversion.  The fine level's arrays and plans are
+allocated when the step is built; the first step allocates the coarse level's
+stage buffers and builds its operator batch, so it takes longer than the
+others (take it outside a stream capture).
 """
 from __future__ import annotations
 

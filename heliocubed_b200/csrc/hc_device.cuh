@@ -188,8 +188,9 @@ HC_DEV void rusanovDissipation(double out[8], const double* wl, const double* wr
 //    component, thermal energy): thermal energy is the same in every frame.
 //    thermal >= 0 is tested as rho (e - b^2/8 pi) >= m^2 / 2, no division.
 //  * Square roots and reciprocals by rsqrtN / rcpN.
-// Measured on a B200: second-order Roe step at 96 x 64^2 x 6 12.65 -> 7.34 ms;
-// fourth-order Roe step at 64 x 64^2 x 6 13.96 -> 12.26 ms.
+// Measured on a B200 when it replaced the eigenvector matrices: second-order
+// Roe step at 96 x 64^2 x 6 12.65 -> 7.34 ms (3.84 now, with the stage kernel's
+// own changes); fourth-order Roe step at 64 x 64^2 x 6 13.96 -> 12.26 ms (9.9).
 template <bool CHECK>
 __device__ __forceinline__ bool roe8Body(double out[8], const double* wl, const double* wr, double gamma, double del2,
                                          double invHg) {
